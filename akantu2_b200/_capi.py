@@ -109,6 +109,9 @@ def lib():
         "akb_model_get_nodal_async": (c_int, [vp, c_int, vp, i64, ctypes.POINTER(i64)]),
         "akb_model_wait_nodal_async": (c_int, [vp, i64]),
         "akb_model_set_node_shape": (c_int, [vp, c_int, c_int]),
+        "akb_patch_plan_check": (c_int, [c_int, vp, i64, vp, i64, c_int, vp, c_int, vp]),
+        "akb_model_set_fused_step": (c_int, [vp, c_int]),
+        "akb_model_get_fused_step": (c_int, [vp, ctypes.POINTER(c_int)]),
         "akb_model_get_node_shape": (c_int, [vp, ctypes.POINTER(c_int), ctypes.POINTER(c_int)]),
         "akb_model_set_dependent_launch": (c_int, [vp, c_int]),
         "akb_model_set_increment_tracking": (c_int, [vp, c_int]),

@@ -517,11 +517,13 @@ __global__ void k_predict(int64_t N, const uint8_t *__restrict__ blocked,
 
 // plastic internals of one quadrature point: loads previous state, runs the
 // radial return, stores the new state (and the plastic energy in a step)
-// GT: storage type of the displacement gradient (the element-math type)
-template <int D, class GT>
+// GT: storage type of the displacement gradient (the element-math type);
+// COND: the new state is written only if store (not for a copy of the element
+// evaluated in a neighbouring patch)
+template <int D, class GT, bool COND = false>
 __device__ __forceinline__ void plastic_point(const MatParams &mp, const GroupArgs &ps,
                                               int64_t ne, int64_t le, int q,
-                                              const double *gd, double *s) {
+                                              const double *gd, double *s, bool store = true) {
   constexpr int DD = D * D, NS = SymComps<D>::value;
   const GT *gu_prev = static_cast<const GT *>(ps.gu_prev);
   double gp[DD], sp[DD], epp[DD], ep[DD], iso;
@@ -542,6 +544,8 @@ __device__ __forceinline__ void plastic_point(const MatParams &mp, const GroupAr
   const int64_t qi = (int64_t)q * ne + le;
   plastic_update<D>(mp.lambda, mp.mu, mp.sigma_y, mp.h, gd, gp, sp, epp, ps.iso_cur_in[qi],
                     ps.iso_prev[qi], mp.dsth, s, ep, &iso);
+  if constexpr (COND)
+    if (!store) return;
   if (ps.update_energy) {
     // MaterialPlastic::updateEnergies (material_plastic.cc:85-103)
     double wp = 0.;
@@ -1169,43 +1173,16 @@ __device__ __forceinline__ T hex8_affine_adjugate(const T (*wx)[3], T *Ja) {
 // 1/det of each element are read from geo [10][E], formed once by
 // k_hex8_affine_geometry with the same arithmetic, instead of gathering the
 // element's coordinates every step
-template <int LAW, int QU, bool AFF = false, bool GEO = false, class T = float>
-__device__ __forceinline__ void element_hex8sf(int64_t le, int64_t e_begin, int64_t e_count,
-                                               int64_t E, const int32_t *conn,
-                                               const int32_t *pos,
-                                               const double *X, const T *geo,
-                                               const double *u, const MatParams &mp,
-                                               const GroupArgs &ps, T *re) {
+// The element's work once its nodal displacements wu and (without GEO) its
+// coordinates wx, both relative to its first node in lexicographic corner
+// order, or (with GEO) its adjugate Ja and 1/det are known: the elemental
+// force in the same order, A
+template <int LAW, int QU, bool AFF, bool GEO, class T>
+__device__ __forceinline__ void hex8sf_forces(T (*wx)[3], T (*wu)[3], T *Ja, T rdet_a,
+                                              const MatParams &mpe, const GroupArgs &ps,
+                                              int64_t e_count, int64_t le, T (*A)[3]) {
   static_assert(AFF || !GEO, "the geometry table holds parallelepipeds only");
-  const int64_t e = e_begin + le;
-  const MatParams mpe = group_params(mp, ps, le);
-  // reference node a sits at lexicographic corner lex[a] = [sx>0] + 2[sy>0] + 4[sz>0]
-  constexpr int lex[8] = {0, 1, 3, 2, 4, 5, 7, 6};
-  T wx[8][3], wu[8][3];
-  double x0[3], u0[3];
-#pragma unroll
-  for (int a = 0; a < 8; ++a) {
-    const int64_t node = conn[(int64_t)a * E + e];
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-      const double uu = u[node * 3 + i];
-      if (a == 0) u0[i] = uu;
-      wu[lex[a]][i] = (T)(uu - u0[i]);
-      if constexpr (!GEO) {
-        const double x = X[node * 3 + i];
-        if (a == 0) x0[i] = x;
-        wx[lex[a]][i] = (T)(x - x0[i]);
-      }
-    }
-  }
-  T Ja[9], rdet_a = T(0);
-  if constexpr (GEO) {
-#pragma unroll
-    for (int k = 0; k < 9; ++k) Ja[k] = geo[(int64_t)k * E + e];
-    rdet_a = geo[(int64_t)9 * E + e];
-  } else {
-    wht8(wx);
-  }
+  if constexpr (!GEO) wht8(wx);
   wht8(wu);
   // Gauss coordinate 1/sqrt(3), rounded once to T
   constexpr T g1 = std::is_same<T, float>::value ? T(0.577350269189625764509f)
@@ -1218,7 +1195,6 @@ __device__ __forceinline__ void element_hex8sf(int64_t le, int64_t e_begin, int6
     }
     wu[3][c] *= g1; wu[5][c] *= g1; wu[6][c] *= g1; wu[7][c] *= g2;
   }
-  T A[8][3];
 #pragma unroll
   for (int m = 0; m < 8; ++m)
 #pragma unroll
@@ -1304,6 +1280,44 @@ __device__ __forceinline__ void element_hex8sf(int64_t le, int64_t e_begin, int6
     A[3][c] *= s1; A[5][c] *= s1; A[6][c] *= s1; A[7][c] *= s2;
   }
   iwht8(A);
+}
+
+template <int LAW, int QU, bool AFF = false, bool GEO = false, class T = float>
+__device__ __forceinline__ void element_hex8sf(int64_t le, int64_t e_begin, int64_t e_count,
+                                               int64_t E, const int32_t *conn,
+                                               const int32_t *pos,
+                                               const double *X, const T *geo,
+                                               const double *u, const MatParams &mp,
+                                               const GroupArgs &ps, T *re) {
+  const int64_t e = e_begin + le;
+  const MatParams mpe = group_params(mp, ps, le);
+  // reference node a sits at lexicographic corner lex[a] = [sx>0] + 2[sy>0] + 4[sz>0]
+  constexpr int lex[8] = {0, 1, 3, 2, 4, 5, 7, 6};
+  T wx[8][3], wu[8][3];
+  double x0[3], u0[3];
+#pragma unroll
+  for (int a = 0; a < 8; ++a) {
+    const int64_t node = conn[(int64_t)a * E + e];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const double uu = u[node * 3 + i];
+      if (a == 0) u0[i] = uu;
+      wu[lex[a]][i] = (T)(uu - u0[i]);
+      if constexpr (!GEO) {
+        const double x = X[node * 3 + i];
+        if (a == 0) x0[i] = x;
+        wx[lex[a]][i] = (T)(x - x0[i]);
+      }
+    }
+  }
+  T Ja[9], rdet_a = T(0);
+  if constexpr (GEO) {
+#pragma unroll
+    for (int k = 0; k < 9; ++k) Ja[k] = geo[(int64_t)k * E + e];
+    rdet_a = geo[(int64_t)9 * E + e];
+  }
+  T A[8][3];
+  hex8sf_forces<LAW, QU, AFF, GEO, T>(wx, wu, Ja, rdet_a, mpe, ps, e_count, le, A);
 #pragma unroll
   for (int a = 0; a < 8; ++a) store_slot<3>(re, pos[(int64_t)a * E + e], A[lex[a]]);
 }
@@ -1388,32 +1402,14 @@ __device__ __forceinline__ void elastic_stress_x2(float lambda, float mu, float 
 // elastic and neohookean laws (the plastic state is FP64 per point).  Every
 // FP32 operation is explicitly rounded (scalar __f*_rn or packed .rn), so
 // neither the points per iteration nor the register cap changes a result.
-// the element's work once its relative nodal displacements wu (lexicographic
-// corner order, FP32) are known
-// The element's per-element table entries come as views: node a is cn[a cs],
-// its slot position pv[a ps], adjugate entry k gv[k gs] (the global [row][E]
-// tables at the element, or a block's staged copies in shared memory).
-template <int LAW, int PU, bool GEO>
-__device__ __forceinline__ void element_hex8sf_x2_core(float (*wu)[3], int64_t le,
-                                                       int64_t e_count, const int32_t *cn,
-                                                       int64_t cs, const int32_t *pv,
-                                                       int64_t pvs, const double *X,
-                                                       const float *gv, int64_t gs,
-                                                       const MatParams &mp, const GroupArgs &ps,
-                                                       float *re) {
+// hex8sf_x2_forces: the element's work once its relative nodal displacements
+// wu (lexicographic corner order, FP32), its adjugate Ja and 1/det are known;
+// A receives its elemental force in the same order
+template <int LAW, int PU>
+__device__ __forceinline__ void hex8sf_x2_forces(float (*wu)[3], const float *Ja, float rdet,
+                                                 const MatParams &mpe, const GroupArgs &ps,
+                                                 int64_t e_count, int64_t le, float (*A)[3]) {
   static_assert(LAW != LAW_PLASTIC, "plastic hexahedra use the scalar kernel");
-  const MatParams mpe = group_params(mp, ps, le);
-  constexpr int lex[8] = {0, 1, 3, 2, 4, 5, 7, 6};
-  float Ja[9], rdet;
-  if constexpr (GEO) {
-#pragma unroll
-    for (int k = 0; k < 9; ++k) Ja[k] = gv[k * gs];
-    rdet = gv[9 * gs];
-  } else {
-    float wx[8][3];
-    hex8_geometry_modes(0, cs, cn, X, wx);
-    rdet = hex8_affine_adjugate(wx, Ja);
-  }
   wht8(wu);
   constexpr float g1 = 0.577350269189625764509f;
   constexpr float g2 = 1.f / 3.f;
@@ -1430,7 +1426,6 @@ __device__ __forceinline__ void element_hex8sf_x2_core(float (*wu)[3], int64_t l
     wu[6][c] = __fmul_rn(wu[6][c], rg1);
     wu[7][c] = __fmul_rn(wu[7][c], rg2);
   }
-  float A[8][3];
 #pragma unroll
   for (int m = 0; m < 8; ++m)
 #pragma unroll
@@ -1522,6 +1517,33 @@ __device__ __forceinline__ void element_hex8sf_x2_core(float (*wu)[3], int64_t l
     A[7][c] = __fmul_rn(A[7][c], s2);
   }
   iwht8(A);
+}
+
+// The element's per-element table entries come as views: node a is cn[a cs],
+// its slot position pv[a ps], adjugate entry k gv[k gs] (the global [row][E]
+// tables at the element, or a block's staged copies in shared memory).
+template <int LAW, int PU, bool GEO>
+__device__ __forceinline__ void element_hex8sf_x2_core(float (*wu)[3], int64_t le,
+                                                       int64_t e_count, const int32_t *cn,
+                                                       int64_t cs, const int32_t *pv,
+                                                       int64_t pvs, const double *X,
+                                                       const float *gv, int64_t gs,
+                                                       const MatParams &mp, const GroupArgs &ps,
+                                                       float *re) {
+  const MatParams mpe = group_params(mp, ps, le);
+  constexpr int lex[8] = {0, 1, 3, 2, 4, 5, 7, 6};
+  float Ja[9], rdet;
+  if constexpr (GEO) {
+#pragma unroll
+    for (int k = 0; k < 9; ++k) Ja[k] = gv[k * gs];
+    rdet = gv[9 * gs];
+  } else {
+    float wx[8][3];
+    hex8_geometry_modes(0, cs, cn, X, wx);
+    rdet = hex8_affine_adjugate(wx, Ja);
+  }
+  float A[8][3];
+  hex8sf_x2_forces<LAW, PU>(wu, Ja, rdet, mpe, ps, e_count, le, A);
 #pragma unroll
   for (int a = 0; a < 8; ++a) store_slot<3>(re, pv[a * pvs], A[lex[a]]);
 }

@@ -7,6 +7,7 @@
 #include <functional>
 #include <limits>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "akb_capi.h"
@@ -14,6 +15,7 @@
 #include "fe_kernels.cuh"
 #include "host_common.h"
 #include "launch.h"
+#include "patch.h"
 
 namespace akb {
 static thread_local std::string g_last_error;
@@ -288,6 +290,10 @@ struct akb_model {
   // step kernels launched with programmatic stream serialization: each one
   // is scheduled while its predecessor drains and waits for it on the device
   bool pdl = false;
+  // fused step (patch.h): one launch per step over patches of nodes, when the
+  // model has a plan for it and no kernel of the two-kernel step was chosen
+  PatchArgs patch;
+  bool patch_ready = false, patch_on = false;
   // persistent multi-step kernel: 0 never (default: on B200 the 100-step
   // graphs of the two-kernel step are faster at every measured size), 1 for
   // small single-group meshes, 2 whenever the model allows it
@@ -679,9 +685,57 @@ int ensure_fint(akb_model *m) {
   return AKB_OK;
 }
 
+bool use_patches(const akb_model *m) {
+#ifdef AKB_BOUNDS_CHECK
+  return false;  // the bounds-checking build runs the checked two-kernel step only
+#endif
+  return m->patch_ready && m->patch_on;
+}
+
+// a kernel of the two-kernel step was chosen by hand: it is the one to run
+void leave_patches(akb_model *m) { m->patch_on = false; }
+
+// the fused step's launch from the prediction u into u_next
+cudaError_t launch_patches(akb_model *m, PatchArgs pa, const GroupArgs &ps, bool pdl) {
+  const Group &gr = m->groups[0];
+  pa.need_index = ps.eig || gr.law == LAW_PLASTIC ? 1 : 0;
+  pa.fext = m->dfext;
+  pa.mass = m->dmass;
+  pa.blocked = m->dblocked;
+  pa.dt = m->dt;
+  pa.inst_dt = m->dinst_dt;
+  const MatParams mp = m->mats[gr.mat0].params();
+  return m->precision == AKB_PRECISION_MIXED
+             ? launch_patch_step_mixed(m->et, gr.law, pa, mp, ps, pdl, m->stream)
+             : launch_patch_step_fp64(m->et, gr.law, pa, mp, ps, pdl, m->stream);
+}
+
+// element forces and node update as one launch
+int patch_step(akb_model *m, bool store_fint) {
+  AKB_TRY(thermal_eval(m, true));
+  PatchArgs pa = m->patch;
+  pa.u = m->u_pred();
+  pa.u_next = m->u();
+  pa.v = m->dv;
+  pa.a = m->da;
+  pa.fint = m->dfint;
+  pa.inst_end = m->dinst_end;
+  pa.step = m->dstep;
+  pa.status = m->dstatus;
+  pa.flags = NU_CORRECT | NU_PREDICT | (m->fext_zero ? NU_FEXT_ZERO : 0) |
+             (store_fint ? NU_FINT : 0);
+  const cudaError_t e = launch_patches(m, pa, group_args(m, m->groups[0], true), m->pdl);
+  if (e != cudaSuccess) return fail(AKB_ECUDA, std::string("fused step: ") + cudaGetErrorString(e));
+  AKB_TRY(prescribe(m, m->u(), true));
+  m->fint_valid = store_fint;
+  return AKB_OK;
+}
+
 // one explicit step: [predictor,] element forces, node update (+ next
 // predictor); afterwards the prediction buffer becomes the model's u
-int one_step(akb_model *m, bool any_plastic, cudaEvent_t e1 = nullptr,
+// The fused step leaves no elemental forces behind, so the last of a sequence
+// of its steps (last) stores the internal force.
+int one_step(akb_model *m, bool any_plastic, bool last = true, cudaEvent_t e1 = nullptr,
              cudaEvent_t e2 = nullptr) {
   if (!m->predicted) AKB_TRY(predict(m));
   // previous displacement and increment: the step goes from u() to its
@@ -689,9 +743,14 @@ int one_step(akb_model *m, bool any_plastic, cudaEvent_t e1 = nullptr,
   if (m->track_history)
     AKB_CUDA(launch_history(m->geom(), m->u(), m->u_pred(), m->dprev, m->dincr, m->stream));
   if (e1) AKB_CUDA(cudaEventRecord(e1, m->stream));
-  AKB_TRY(element_forces(m, true));
-  if (e2) AKB_CUDA(cudaEventRecord(e2, m->stream));
-  AKB_TRY(node_update(m, true));
+  if (use_patches(m)) {
+    AKB_TRY(patch_step(m, last));
+    if (e2) AKB_CUDA(cudaEventRecord(e2, m->stream));
+  } else {
+    AKB_TRY(element_forces(m, true));
+    if (e2) AKB_CUDA(cudaEventRecord(e2, m->stream));
+    AKB_TRY(node_update(m, true));
+  }
   if (m->dstep) AKB_CUDA(launch_step_advance(m->geom(), m->stream));
   m->ucur = 1 - m->ucur;  // u_{n+1} is now the model's displacement
   if (any_plastic) m->cur = 1 - m->cur;
@@ -716,6 +775,7 @@ int capture_graph(akb_model *m, bool any_plastic, akb_model::StepGraph **out = n
   if (!g) {
     const int ucur0 = m->ucur, cur0 = m->cur;
     const int64_t steps0 = m->steps_done;
+    const bool fint0 = m->fint_valid;
     // graphs replay steps without a thermal term (thermal_steady): capture
     // them from that state, with the device table already matching it
     std::vector<Material> mats0 = m->mats;
@@ -727,12 +787,14 @@ int capture_graph(akb_model *m, bool any_plastic, akb_model::StepGraph **out = n
     AKB_TRY(sync_mtab(m));
     AKB_CUDA(cudaStreamBeginCapture(m->stream, cudaStreamCaptureModeThreadLocal));
     int rc = AKB_OK;
-    for (int64_t s = 0; s < m->graph_steps && rc == AKB_OK; ++s) rc = one_step(m, any_plastic);
+    for (int64_t s = 0; s < m->graph_steps && rc == AKB_OK; ++s)
+      rc = one_step(m, any_plastic, s + 1 == m->graph_steps);
     cudaGraph_t graph = nullptr;
     cudaError_t e = cudaStreamEndCapture(m->stream, &graph);
     m->ucur = ucur0;
     m->cur = cur0;
     m->steps_done = steps0;
+    m->fint_valid = fint0;
     for (size_t k = 0; k < m->mats.size(); ++k) {
       m->mats[k].th_prev = mats0[k].th_prev;
       m->mats[k].th_cur = mats0[k].th_cur;
@@ -777,7 +839,7 @@ int run_graph(akb_model *m, bool any_plastic) {
   AKB_TRY(sync_mtab(m));
   AKB_CUDA(cudaGraphLaunch(g->exec, m->stream));
   m->steps_done += g->steps;
-  m->fint_valid = false;
+  m->fint_valid = use_patches(m);
   return AKB_OK;
 }
 
@@ -933,6 +995,234 @@ int reduce_to_host(akb_model *m, const double *x, int64_t n, bool op_min, double
   AKB_CUDA(launch_reduce(x, n, op_min ? 1 : 0, m->dpartials, m->dresult, m->stream));
   AKB_CUDA(cudaMemcpyAsync(out, m->dresult, sizeof(double), cudaMemcpyDeviceToHost, m->stream));
   AKB_CUDA(cudaStreamSynchronize(m->stream));
+  return AKB_OK;
+}
+
+// ---- plan of the fused step ------------------------------------------------
+
+// Owned nodes of a patch at most, s per edge; 0 where the two-kernel step is
+// the faster one.  Regular boxes are assumed: the rule also sizes the plan's
+// memory before there is a mesh.
+//
+// Tetrahedra and hexahedra: a patch evaluates about ((s + 1) / s)^3 times its
+// share of the elements, so large meshes take the largest patch that leaves
+// two (FP64) or three (mixed) blocks per SM their shared memory (mixed batch
+// of 4.5 M tetrahedra: 145 us per step with 216 nodes, 159 with 125).  A mesh
+// with less than about three patches per SM is bound by the SM with the most
+// work: the edge with the least of it (mixed, us per step: 3 k tetrahedra 3.3
+// with 8 nodes and 5.2 with 216, 10 k 3.7 with 27, 48 k 4.4 with 125, 6.0 with
+// 216 and 10.1 with 8).  Hexahedra, whose packed kernel is bound by its
+// arithmetic, gain from the single launch while every SM has one patch at
+// most and lose by the repeated elements beyond (us per step, fused / two
+// kernels: 4 k 4.9 / 7.4, 8 k 5.0 / 8.0, 16 k 8.4 / 8.6, 27 k 8.7 / 9.5, 262 k
+// 44.7 / 41.4).
+//
+// Plastic triangles: a small mesh's step is as long as the rounds its
+// patches' six warps need for all (32 elements, point) items (us per step,
+// two kernels / fused with one round / with two: 2 k triangles of 6 points
+// FP64 18.5 / 6.7 / 9.3, 8 k of 3 points mixed 12.8 / 7.5 / 10.2).  With more
+// patches than are resident at once the two kernels, which read every point's
+// state once, are faster (512^2 x 2: 111 against 154).
+int patch_nodes(int et, int rule, int precision, int64_t N, int64_t E, int ninst) {
+  const bool mixed = precision == AKB_PRECISION_MIXED;
+  const double sms = 148.;
+  const double planes = std::pow((double)N / ninst, 1. / dim_of(et));
+  int best = 0;
+  double least = 0.;
+  if (et == AKB_TRIANGLE_6) {
+    for (int s = 12; s >= 2; --s) {
+      const double slabs = std::ceil(planes / s - 1e-6), a = planes / slabs;
+      // resident blocks per SM, fewer with the slots of 6 points
+      if (ninst * slabs * slabs > sms * (rule ? 2. : mixed ? 4. : 3.)) break;
+      const double elements = 2. * (a / 2. + 1.) * (a / 2. + 1.);
+      const double rounds = std::ceil(std::ceil(elements / 32.) * (rule ? 6. : 3.) / 6.);
+      if (least == 0. || rounds < least) {
+        least = rounds;
+        best = s;
+      }
+    }
+    return best * best;
+  }
+  const bool tet = et == AKB_TETRAHEDRON_4;
+  const int most = tet && mixed ? 6 : 5;
+  if (tet) best = most;
+  for (int s = most; s >= 2; --s) {
+    const double slabs = std::ceil(planes / s - 1e-6);
+    const double patches = ninst * slabs * slabs * slabs;
+    if (patches > (tet ? 3. * sms : sms)) break;
+    const double work = std::ceil(patches / sms) * (double)E / (double)N *
+                        std::pow(planes / slabs + 1., 3.);
+    if (least == 0. || work < least) {
+      least = work;
+      best = s;
+    }
+  }
+  return best * best * best;
+}
+
+// rows of the per-element tables the fused kernel reads and the size of one
+// value (0 rows: there is no fused kernel for these elements)
+struct PatchTables {
+  int rows = 0;
+  size_t value = 0;
+};
+PatchTables patch_tables(int et, int law, int precision, int nq) {
+  PatchTables t;
+  const bool mixed = precision == AKB_PRECISION_MIXED;
+  if (et == AKB_TRIANGLE_6) t.rows = law == LAW_PLASTIC ? 13 * nq : 0;
+  else if (law == LAW_PLASTIC) t.rows = 0;
+  else if (et == AKB_TETRAHEDRON_4) t.rows = mixed ? 10 : 13;
+  else if (et == AKB_HEXAHEDRON_8 && mixed) t.rows = 10;
+  t.value = mixed ? sizeof(float) : sizeof(double);
+  return t;
+}
+
+// bytes of a plan's arrays at their capacity, in one allocation
+size_t patch_capacity_bytes(const PatchCaps &c, int64_t N, int nn, const PatchTables &t) {
+  size_t bytes = 0;
+  auto take = [&](int64_t n, size_t size) { bytes += ((size_t)n * size + 255) / 256 * 256; };
+  take(c.patches, sizeof(PatchHead));
+  take(c.nodes, sizeof(int32_t));
+  take(N, sizeof(PatchOwn));
+  take(c.elems, sizeof(int32_t));
+  take(c.elems, 2 * sizeof(uint16_t) * (nn <= 4 ? 4 : 8) + t.rows * t.value);
+  return bytes;
+}
+
+// device bytes of a plan (the same for any mesh of these sizes)
+int64_t patch_bytes(int et, int rule, int law, int precision, int64_t N, int64_t E, int ninst) {
+  const PatchTables t = patch_tables(et, law, precision, et == AKB_TRIANGLE_6 && rule ? 6 : 3);
+  if (t.rows == 0 || N == 0 || E == 0) return 0;
+  const int own = patch_nodes(et, rule, precision, N, E, ninst);
+  if (own == 0) return 0;
+  const PatchCaps c = patch_caps(dim_of(et), N, E, ninst, own);
+  return (int64_t)patch_capacity_bytes(c, N, nodes_per_element(et), t);
+}
+
+// Builds the plan on a thread of its own while initFull goes on with the
+// device (it only reads the host arrays it is given, which outlive it).
+struct PatchTask {
+  PatchMesh mesh;
+  PatchCaps caps;
+  PatchPlan plan;
+  std::vector<int32_t> mat;
+  bool wanted = false, ok = false;
+  std::thread worker;
+  ~PatchTask() { wait(); }
+  void wait() {
+    if (worker.joinable()) worker.join();
+  }
+  void build() {
+    try {
+      ok = build_patches(mesh, caps, plan);
+    } catch (const std::exception &) {
+      ok = false;  // out of host memory or threads: the two-kernel step runs
+    }
+  }
+};
+
+// starts the plan where the model may have one: a single law group of an
+// element type and law with a fused kernel, of a size it is the faster at
+void start_patches(akb_model *m, const std::vector<int32_t> &conn_soa,
+                   const std::vector<int32_t> &ptr, const std::vector<int32_t> &pos,
+                   PatchTask &task) {
+#ifdef AKB_BOUNDS_CHECK
+  return;
+#endif
+  if (m->groups.size() != 1 || m->N == 0 || m->E == 0) return;
+  const Group &gr = m->groups[0];
+  for (auto &mt : m->mats)
+    if (mt.c33) return;
+  PatchMesh &pm = task.mesh;
+  pm.max_own = patch_nodes(m->et, m->rule, m->precision, m->N, m->E, m->ninst);
+  if (pm.max_own == 0 || patch_tables(m->et, gr.law, m->precision, m->nq).rows == 0) return;
+  pm.D = m->dim;
+  pm.NN = m->nn;
+  pm.N = m->N;
+  pm.E = m->E;
+  pm.X = m->X.data();
+  pm.conn = conn_soa.data();
+  pm.ptr = ptr.data();
+  pm.pos = pos.data();
+  pm.inst_off = m->inst_node_off.data();
+  pm.ninst = m->ninst;
+  if (gr.nmat > 1) {
+    task.mat.resize(m->E);
+    for (int64_t ie = 0; ie < m->E; ++ie) task.mat[ie] = m->mat_user[m->perm[ie]];
+    pm.mat = task.mat.data();
+  }
+  task.caps = patch_caps(m->dim, m->N, m->E, m->ninst, pm.max_own);
+  task.wanted = true;
+  try {
+    task.worker = std::thread([&task] { task.build(); });
+  } catch (const std::exception &) {
+    task.build();
+  }
+}
+
+// the finished plan's arrays on the device
+int finish_patches(akb_model *m, PatchTask &task) {
+  task.wait();
+  const bool hex = m->et == AKB_HEXAHEDRON_8, mixed = m->precision == AKB_PRECISION_MIXED;
+  if (!task.wanted || !task.ok || (hex && !(m->all_affine && m->dgeo))) return AKB_OK;
+  const Group &gr = m->groups[0];
+  const PatchTables t = patch_tables(m->et, gr.law, m->precision, m->nq);
+  const PatchPlan &plan = task.plan;
+  PatchArgs &pa = m->patch;
+  const int points = m->et == AKB_TRIANGLE_6 ? m->nq : 1;  // slot arrays
+  pa.smem = patch_smem(m->dim, plan.max_local, plan.max_slots * points, t.value);
+  if (pa.smem + kPatchStageSmem > kPatchMaxSmem) return AKB_OK;
+  const size_t bytes =
+      patch_capacity_bytes(task.caps, m->N, m->nn, t);  // the capacity, whatever the mesh needs
+  char *base = nullptr;
+  AKB_TRY(m->alloc(&base, bytes));
+  cudaStream_t s = m->stream;
+  // the lists in one upload, the chunks behind them; the local indices the
+  // chunks are made of are on the device for the time being
+  const int64_t n = (int64_t)plan.elems.size();
+  size_t at = 0;
+  auto take = [&](size_t size) {
+    const size_t here = at;
+    at += (size + 255) / 256 * 256;
+    return here;
+  };
+  const size_t o_head = take(plan.head.size() * sizeof(PatchHead));
+  const size_t o_nodes = take(plan.nodes.size() * sizeof(int32_t));
+  const size_t o_own = take(plan.own.size() * sizeof(PatchOwn));
+  const size_t o_elems = take(plan.elems.size() * sizeof(int32_t));
+  const size_t o_tab = at;
+  const size_t lb = plan.conn.size() * sizeof(uint16_t);
+  std::vector<char> lists(o_tab), local(2 * lb);
+  std::memcpy(lists.data() + o_head, plan.head.data(), plan.head.size() * sizeof(PatchHead));
+  std::memcpy(lists.data() + o_nodes, plan.nodes.data(), plan.nodes.size() * sizeof(int32_t));
+  std::memcpy(lists.data() + o_own, plan.own.data(), plan.own.size() * sizeof(PatchOwn));
+  std::memcpy(lists.data() + o_elems, plan.elems.data(), plan.elems.size() * sizeof(int32_t));
+  std::memcpy(local.data(), plan.conn.data(), lb);
+  std::memcpy(local.data() + lb, plan.slot.data(), lb);
+  AKB_CUDA(cudaMemcpyAsync(base, lists.data(), lists.size(), cudaMemcpyHostToDevice, s));
+  pa.npatch = (int64_t)plan.head.size();
+  pa.multi = 0;
+  for (const PatchHead &h : plan.head) pa.multi |= gr.nmat > 1 && h.mat < 0 && h.n_elem > 0;
+  pa.head = (const PatchHead *)(base + o_head);
+  pa.nodes = (const int32_t *)(base + o_nodes);
+  pa.own = (const PatchOwn *)(base + o_own);
+  pa.elems = (const int32_t *)(base + o_elems);
+  pa.tab = base + o_tab;
+  pa.e_count = m->E;
+  pa.nq = m->nq;
+  char *dlocal = nullptr;
+  AKB_CUDA(cudaMallocAsync((void **)&dlocal, std::max<size_t>(local.size(), 16), s));
+  cudaError_t e = cudaMemcpyAsync(dlocal, local.data(), local.size(), cudaMemcpyHostToDevice, s);
+  const void *ta = hex ? (const void *)m->dgeo : mixed ? (const void *)m->fB : m->dB;
+  const void *tb = hex ? nullptr : mixed ? (const void *)m->fwJ : m->dwJ;
+  if (e == cudaSuccess)
+    e = launch_patch_chunks(plan.NNP, n, pa.elems, (const uint16_t *)dlocal,
+                            (const uint16_t *)(dlocal + lb), m->E, hex ? t.rows : t.rows - m->nq,
+                            ta, hex ? 0 : m->nq, tb, t.value, base + o_tab, s);
+  cudaFreeAsync(dlocal, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);  // the host copies are freed
+  if (e != cudaSuccess) return fail(AKB_ECUDA, std::string("fused step: ") + cudaGetErrorString(e));
+  m->patch_ready = m->patch_on = true;
   return AKB_OK;
 }
 
@@ -1269,6 +1559,7 @@ int akb_model_init_full(akb_model *m, int method, int precision) {
   // the order of the lumped-mass assembly, which runs over all elements of
   // the type in user order (solid_mechanics_model_mass.cc:115-128).
   std::vector<int32_t> ptr(N + 1, 0), ent((size_t)E * nn), pos((size_t)E * nn);
+  PatchTask patches;
   for (int64_t ie = 0; ie < E; ++ie)
     for (int a = 0; a < nn; ++a) ptr[conn_soa[(size_t)a * E + ie] + 1]++;
   for (int64_t i = 0; i < N; ++i) ptr[i + 1] += ptr[i];
@@ -1279,6 +1570,7 @@ int akb_model_init_full(akb_model *m, int method, int precision) {
       for (int64_t ie = mt.e_begin; ie < mt.e_begin + mt.e_count; ++ie)
         for (int a = 0; a < nn; ++a) pos[(size_t)a * E + ie] = fill[conn_soa[(size_t)a * E + ie]]++;
     }
+    start_patches(m, conn_soa, ptr, pos, patches);
     std::copy(ptr.begin(), ptr.end() - 1, fill.begin());
     for (int64_t e = 0; e < E; ++e) {
       const int64_t ie = iperm[e];
@@ -1445,6 +1737,7 @@ int akb_model_init_full(akb_model *m, int method, int precision) {
     AKB_CUDA(cudaMemcpyAsync(m->dmslot, mslot.data(), sizeof(int32_t) * E, cudaMemcpyHostToDevice, s));
     AKB_CUDA(cudaStreamSynchronize(s));
   }
+  AKB_TRY(finish_patches(m, patches));
   // batch: instance of each node, per-instance time steps, element ranges
   if (m->ninst > 1) {
     const int ni = m->ninst;
@@ -1920,7 +2213,7 @@ int akb_model_solve_step(akb_model *m, int64_t nsteps) {
   // a step with a thermal term in the plastic trial stress (the first after
   // initFull or a standalone assembly of a heated material) runs eagerly
   if (nsteps > 0 && !thermal_steady(m)) {
-    AKB_TRY(one_step(m, any_plastic));
+    AKB_TRY(one_step(m, any_plastic, nsteps == 1));
     --nsteps;
     m->forces_evaluated = true;
     m->snap_valid = false;
@@ -1934,7 +2227,7 @@ int akb_model_solve_step(akb_model *m, int64_t nsteps) {
   int64_t left = nsteps;
   // a step whose prediction is stale runs eagerly (it launches the predictor)
   if (left > 0 && !m->predicted) {
-    AKB_TRY(one_step(m, any_plastic));
+    AKB_TRY(one_step(m, any_plastic, left == 1));
     --left;
   }
   const int64_t G = m->graph_steps;
@@ -1942,7 +2235,7 @@ int akb_model_solve_step(akb_model *m, int64_t nsteps) {
     AKB_TRY(run_graph(m, any_plastic));
     left -= G;
   }
-  for (; left > 0; --left) AKB_TRY(one_step(m, any_plastic));
+  for (; left > 0; --left) AKB_TRY(one_step(m, any_plastic, left == 1));
   if (nsteps > 0) {
     m->forces_evaluated = true;
     m->snap_valid = false;
@@ -2006,6 +2299,7 @@ int akb_estimate_device_bytes(int et, int rule, int64_t N, int64_t E, int law, i
   if (law == LAW_NEOHOOKEAN && d == 2) t += r(8 * E * nq);  // plane-stress C33
   // mixed hexahedra: the adjugate table of a mesh of parallelepipeds
   if (precision == AKB_PRECISION_MIXED && et == AKB_HEXAHEDRON_8) t += r(4 * 10 * E);
+  t += patch_bytes(et, rule, law, precision, N, E, 1);
   *bytes = t;
   return AKB_OK;
 }
@@ -2021,6 +2315,8 @@ int akb_estimate_batch_device_bytes(int et, int rule, int64_t N, int64_t E, int 
   // stop steps; the material table and the step counter
   *bytes += r(4 * N) + 3 * r(4 * E) + 3 * r(8 * ni) + r(8 * (ni + 1)) +
             r((int64_t)sizeof(MatParams) * ni) + r(8);
+  *bytes += patch_bytes(et, rule, law, precision, N, E, nb_instances) -
+            patch_bytes(et, rule, law, precision, N, E, 1);
   return AKB_OK;
 }
 
@@ -2163,7 +2459,7 @@ int akb_model_autotune(akb_model *m, int repeats) {
     if (gr.c33) c33_n = std::max(c33_n, gr.e_count * m->nq);
   double *t_c33 = nullptr;
   if (c33_n > 0) AKB_CUDA(cudaMallocAsync((void **)&t_c33, sizeof(double) * c33_n, s));
-  auto elem_launch = [&](Group &gr, const ElemTuning &tn) {
+  auto scratch_args = [&](const Group &gr) {
     GroupArgs ps = group_args(m, gr, false);
     if (gr.c33) ps.c33 = t_c33;
     if (gr.law == LAW_PLASTIC) {
@@ -2173,6 +2469,10 @@ int akb_model_autotune(akb_model *m, int repeats) {
       ps.iso = t_iso;
       ps.update_energy = 0;
     }
+    return ps;
+  };
+  auto elem_launch = [&](Group &gr, const ElemTuning &tn) {
+    const GroupArgs ps = scratch_args(gr);
     const MatParams mp = m->mats[gr.mat0].params();
     if (m->precision == AKB_PRECISION_MIXED)
       return launch_element_forces_mixed(g, gr.law, gr.e_begin, gr.e_count, m->tab, m->fB,
@@ -2324,6 +2624,29 @@ int akb_model_autotune(akb_model *m, int repeats) {
     }
     if (rc == AKB_OK) m->pdl = ms[1] < ms[0];
     g.pdl = m->pdl ? 1 : 0;
+    // the fused step, where the model has it, against the best of them
+    float best = std::min(ms[0], ms[1]);
+    if (rc == AKB_OK && m->patch_ready) m->patch_on = false;
+    for (int pdl = 0; pdl < 2 && rc == AKB_OK && m->patch_ready; ++pdl) {
+      PatchArgs pa = m->patch;
+      pa.u = m->u();
+      pa.u_next = t_u;
+      pa.v = t_v;
+      pa.a = t_a;
+      pa.status = t_status;
+      pa.flags = flags;
+      auto step = [&]() {
+        cudaError_t e = cudaSuccess;
+        for (int r = 0; r < 8 && e == cudaSuccess; ++r) 
+          e = launch_patches(m, pa, scratch_args(m->groups[0]), pdl != 0);
+        return e;
+      };
+      float t = 0.f;
+      if (!time_it(step, &t) || t >= best) continue;
+      best = t;
+      m->patch_on = true;
+      m->pdl = pdl != 0;
+    }
   }
   // the slot array again holds the forces of the current state, computed
   // with the chosen shapes
@@ -2350,6 +2673,7 @@ int akb_model_set_node_shape(akb_model *m, int node_block, int staged) {
   AKB_CUDA(cudaStreamSynchronize(m->stream));
   m->node_block = node_block;
   m->node_form = staged;
+  leave_patches(m);
   for (auto &x : m->graphs) cudaGraphExecDestroy(x.exec);
   m->graphs.clear();
   return AKB_OK;
@@ -2404,6 +2728,7 @@ int akb_model_set_affine_kernel(akb_model *m, int on) {
   }
   AKB_CUDA(cudaStreamSynchronize(m->stream));
   m->affine_kernel = on;
+  leave_patches(m);
   // the packed form exists for meshes of parallelepipeds only: without the
   // kernel compiled for them, the scalar form with the same points per
   // iteration (2 or 8; 4 becomes 2) and a register cap that does not spill
@@ -2435,6 +2760,26 @@ int akb_model_set_dependent_launch(akb_model *m, int on) {
 int akb_model_get_dependent_launch(const akb_model *m, int *on) {
   if (!m || !on) return fail(AKB_EINVAL, "null argument");
   *on = m->pdl ? 1 : 0;
+  return AKB_OK;
+}
+
+int akb_model_set_fused_step(akb_model *m, int on) {
+  AKB_TRY(check_model(m, true));
+  if (on != 0 && on != 1) return fail(AKB_EINVAL, "on must be 0 or 1");
+  if (on && !m->patch_ready)
+    return fail(AKB_EUNSUPPORTED, "this model has no fused step");
+  // the two-kernel step's elemental forces are not kept by fused steps
+  AKB_TRY(ensure_fint(m));
+  AKB_CUDA(cudaStreamSynchronize(m->stream));
+  m->patch_on = on != 0;
+  for (auto &x : m->graphs) cudaGraphExecDestroy(x.exec);
+  m->graphs.clear();
+  return AKB_OK;
+}
+
+int akb_model_get_fused_step(const akb_model *m, int *on) {
+  if (!m || !on) return fail(AKB_EINVAL, "null argument");
+  *on = use_patches(m) ? 1 : 0;
   return AKB_OK;
 }
 
@@ -2540,6 +2885,7 @@ int akb_model_set_launch_shape(akb_model *m, int law, int element_block,
     }
   if (!found) return fail(AKB_EINVAL, "no material of this law in the model");
   m->node_block = node_block;
+  leave_patches(m);
   AKB_CUDA(cudaStreamSynchronize(m->stream));
   for (auto &x : m->graphs) cudaGraphExecDestroy(x.exec);
   m->graphs.clear();
@@ -2562,6 +2908,7 @@ int akb_model_set_prefetch(akb_model *m, int law, int waves) {
       found = true;
     }
   if (!found) return fail(AKB_EINVAL, "no material of this law in the model");
+  leave_patches(m);
   AKB_CUDA(cudaStreamSynchronize(m->stream));
   for (auto &x : m->graphs) cudaGraphExecDestroy(x.exec);
   m->graphs.clear();
@@ -2583,6 +2930,7 @@ int akb_model_set_recompute_geometry(akb_model *m, int law, int on) {
       found = true;
     }
   if (!found) return fail(AKB_EINVAL, "no material of this law in the model");
+  leave_patches(m);
   AKB_CUDA(cudaStreamSynchronize(m->stream));
   for (auto &x : m->graphs) cudaGraphExecDestroy(x.exec);
   m->graphs.clear();
@@ -2608,6 +2956,7 @@ int akb_model_set_streamed_points(akb_model *m, int law, int on) {
       found = true;
     }
   if (!found) return fail(AKB_EINVAL, "no material of this law in the model");
+  leave_patches(m);
   AKB_CUDA(cudaStreamSynchronize(m->stream));
   for (auto &x : m->graphs) cudaGraphExecDestroy(x.exec);
   m->graphs.clear();
@@ -2695,7 +3044,7 @@ int akb_model_profile_steps(akb_model *m, int64_t nsteps, double *total_ms, doub
   AKB_CUDA(cudaEventRecord(ev[0], m->stream));
   for (int64_t s = 0; s < nsteps && rc == AKB_OK; ++s) {
     // phases: [predictor if needed], element forces, node update (+ predictor)
-    rc = one_step(m, any_plastic, ev[s * 3 + 1], ev[s * 3 + 2]);
+    rc = one_step(m, any_plastic, s + 1 == nsteps, ev[s * 3 + 1], ev[s * 3 + 2]);
     if (rc == AKB_OK) cudaEventRecord(ev[s * 3 + 3], m->stream);
   }
   cudaError_t e = cudaStreamSynchronize(m->stream);
@@ -2891,6 +3240,59 @@ int akb_model_get_energy(akb_model *m, const char *id, double *value) {
   return AKB_OK;
 }
 
+int akb_patch_plan_check(int et, const double *nodes, int64_t N, const int32_t *conn, int64_t E,
+                         int nb_instances, const int64_t *node_offsets, int max_own,
+                         int64_t *stats) {
+  if (!nodes || !conn || !node_offsets || !stats) return fail(AKB_EINVAL, "null argument");
+  if (et < AKB_TETRAHEDRON_4 || et > AKB_TRIANGLE_6) return fail(AKB_EINVAL, "unknown element type");
+  if (N < 1 || E < 1 || max_own < 1 || nb_instances < 1 || node_offsets[0] != 0 ||
+      node_offsets[nb_instances] != N)
+    return fail(AKB_EINVAL, "bad sizes");
+  for (int k = 0; k < nb_instances; ++k)
+    if (node_offsets[k] > node_offsets[k + 1]) return fail(AKB_EINVAL, "bad instance offsets");
+  const int nn = nodes_per_element(et);
+  for (int64_t k = 0; k < E * nn; ++k)
+    if (conn[k] < 0 || conn[k] >= N) return fail(AKB_EINVAL, "connectivity refers to a missing node");
+  PatchMesh pm;
+  pm.D = dim_of(et);
+  pm.NN = nn;
+  pm.N = N;
+  pm.E = E;
+  pm.X = nodes;
+  pm.inst_off = node_offsets;
+  pm.ninst = nb_instances;
+  pm.max_own = max_own;
+  try {
+    std::vector<int32_t> soa((size_t)E * nn), ptr(N + 1, 0), pos((size_t)E * nn);
+    for (int64_t e = 0; e < E; ++e)
+      for (int a = 0; a < nn; ++a) {
+        soa[(size_t)a * E + e] = conn[e * nn + a];
+        ptr[conn[e * nn + a] + 1]++;
+      }
+    for (int64_t i = 0; i < N; ++i) ptr[i + 1] += ptr[i];
+    std::vector<int32_t> fill(ptr.begin(), ptr.end() - 1);
+    for (int64_t e = 0; e < E; ++e)
+      for (int a = 0; a < nn; ++a) pos[(size_t)a * E + e] = fill[conn[e * nn + a]]++;
+    pm.conn = soa.data();
+    pm.ptr = ptr.data();
+    pm.pos = pos.data();
+    PatchCaps caps;
+    caps.patches = N;
+    caps.nodes = caps.elems = std::numeric_limits<int32_t>::max();
+    PatchPlan plan;
+    if (!build_patches(pm, caps, plan)) return fail(AKB_EUNSUPPORTED, "no plan for this mesh");
+    if (!check_patches(pm, plan)) return fail(AKB_ESTATE, "the plan is wrong");
+    stats[0] = (int64_t)plan.head.size();
+    stats[1] = 0;
+    for (const PatchHead &h : plan.head) stats[1] += h.n_elem;
+    stats[2] = plan.max_local;
+    stats[3] = plan.max_slots;
+  } catch (const std::exception &x) {
+    return fail(AKB_ENOMEM, x.what());
+  }
+  return AKB_OK;
+}
+
 int akb_bounds_checked(void) {
 #ifdef AKB_BOUNDS_CHECK
   return 1;
@@ -2995,7 +3397,7 @@ struct akb_exchange {
     cudaGraphExec_t exec = nullptr;
     std::vector<int> ucur, cur;
     std::vector<double> dt;
-    std::vector<char> fext_zero;
+    std::vector<char> fext_zero, fused;
     int64_t steps = 0;
   };
   std::vector<Graph> graphs;
@@ -3041,7 +3443,7 @@ bool any_plastic_of(const akb_model *m) {
 
 // one step of every model with its halo exchange, enqueued on the models'
 // streams (inside or outside a capture)
-int exchange_step(akb_exchange *x) {
+int exchange_step(akb_exchange *x, bool last = true) {
   for (auto *m : x->parts) {
     DeviceGuard g(m->device);
     if (!m->predicted) AKB_TRY(predict(m));
@@ -3066,7 +3468,7 @@ int exchange_step(akb_exchange *x) {
   }
   for (auto *m : x->parts) {
     DeviceGuard g(m->device);
-    AKB_TRY(one_step(m, any_plastic_of(m)));
+    AKB_TRY(one_step(m, any_plastic_of(m), last));
   }
   return AKB_OK;
 }
@@ -3081,7 +3483,7 @@ int exchange_graph(akb_exchange *x) {
     for (size_t k = 0; same && k < P; ++k) {
       const akb_model *m = x->parts[k];
       same = c.ucur[k] == m->ucur && c.cur[k] == m->cur && c.dt[k] == m->dt &&
-             c.fext_zero[k] == (char)m->fext_zero;
+             c.fext_zero[k] == (char)m->fext_zero && c.fused[k] == (char)use_patches(m);
     }
     if (same) g = &c;
   }
@@ -3093,6 +3495,7 @@ int exchange_graph(akb_exchange *x) {
       ng.cur.push_back(m->cur);
       ng.dt.push_back(m->dt);
       ng.fext_zero.push_back((char)m->fext_zero);
+      ng.fused.push_back((char)use_patches(m));
     }
     ng.steps = x->graph_steps;
     std::vector<int64_t> steps0(P);
@@ -3108,7 +3511,8 @@ int exchange_graph(akb_exchange *x) {
     for (auto *m : x->parts)
       if (rc == AKB_OK && cudaStreamWaitEvent(m->stream, x->fork, 0) != cudaSuccess)
         rc = fail(AKB_ECUDA, "capture fork");
-    for (int64_t s = 0; s < x->graph_steps && rc == AKB_OK; ++s) rc = exchange_step(x);
+    for (int64_t s = 0; s < x->graph_steps && rc == AKB_OK; ++s)
+      rc = exchange_step(x, s + 1 == x->graph_steps);
     for (size_t k = 0; k < P && rc == AKB_OK; ++k)
       if (cudaEventRecord(x->joins[k], x->parts[k]->stream) != cudaSuccess ||
           cudaStreamWaitEvent(x->main, x->joins[k], 0) != cudaSuccess)
@@ -3151,7 +3555,7 @@ int exchange_graph(akb_exchange *x) {
   for (auto *m : x->parts) {
     AKB_CUDA(cudaStreamWaitEvent(m->stream, x->done, 0));
     m->steps_done += g->steps;
-    m->fint_valid = false;
+    m->fint_valid = use_patches(m);
   }
   // the graph's last unpacks precede its end, which the models' streams wait for
   for (auto &l : x->links) l.consumed_pending = false;
@@ -3258,7 +3662,7 @@ int akb_exchange_solve_step(akb_exchange *x, int64_t nsteps) {
   // steps whose models must first predict, or whose plastic trial stress
   // has a thermal term, run eagerly; then whole graphs on one GPU
   while (left > 0 && (!x->one_device || G == 0 || left < G || !exchange_steady(x))) {
-    AKB_TRY(exchange_step(x));
+    AKB_TRY(exchange_step(x, left == 1));
     --left;
     if (x->one_device && G > 0 && left >= G && exchange_steady(x)) break;
   }
@@ -3266,7 +3670,7 @@ int akb_exchange_solve_step(akb_exchange *x, int64_t nsteps) {
     AKB_TRY(exchange_graph(x));
     left -= G;
   }
-  for (; left > 0; --left) AKB_TRY(exchange_step(x));
+  for (; left > 0; --left) AKB_TRY(exchange_step(x, left == 1));
   if (nsteps > 0)
     for (auto *m : x->parts) {
       m->forces_evaluated = true;

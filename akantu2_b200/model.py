@@ -611,6 +611,16 @@ class SolidMechanicsModel:
         _capi.check(_capi.lib().akb_model_get_node_shape(self._h, ctypes.byref(b), ctypes.byref(st)))
         return b.value, st.value
 
+    def setFusedStep(self, on=True):
+        """The element forces and the node update of a step as one launch over
+        patches of nodes (True), or as two kernels; results are unchanged."""
+        _capi.check(_capi.lib().akb_model_set_fused_step(self._h, int(bool(on))))
+
+    def getFusedStep(self):
+        on = ctypes.c_int()
+        _capi.check(_capi.lib().akb_model_get_fused_step(self._h, ctypes.byref(on)))
+        return bool(on.value)
+
     def setDependentLaunch(self, on=True):
         """Step kernels launched with programmatic stream serialization (each
         scheduled while its predecessor drains); results are unchanged."""

@@ -507,7 +507,8 @@ def run_ours(args, rep=None, emit=True, extra=False):
         nprof = min(args.steps, 20)
         tot, phases = m.profileSteps(nprof)
         step_b, kern_b = algorithmic_bytes(args.config, mesh, prec, args.qp_rule)
-        elem_ms = phases[1] / nprof
+        elem_ms = phases[1] / nprof  # the fused step, where the model runs it
+        fused = m.getFusedStep()
         peak, peak_kind = read_peaks()
         results[prec] = {
             "ms_per_step": ms / args.steps,
@@ -515,8 +516,8 @@ def run_ours(args, rep=None, emit=True, extra=False):
             "phase_ms_per_step": {"predictor": phases[0] / nprof,
                                   "element_forces": phases[1] / nprof,
                                   "node_update": phases[2] / nprof},
-            "roofline": roofline_entry(kern_b, elem_ms, peak, peak_kind,
-                                       None if args.qp_rule else
+            "roofline": roofline_entry(step_b if fused else kern_b, elem_ms, peak, peak_kind,
+                                       None if args.qp_rule or fused else
                                        read_traffic(args.config, prec)),
             "roofline_step": {"bytes_per_element_step": step_b / E,
                               "achieved": step_b / (ms / args.steps / 1e3) / 1e9,
@@ -530,9 +531,10 @@ def run_ours(args, rep=None, emit=True, extra=False):
                    f"{ms_resident / args.steps:.5f} ms per step with the model L2-resident "
                    "(100-step graphs)") if fits_l2 else
                   f"inputs larger than L2 ({footprint / 1e6:.0f} MB on the device; no flush)",
-            # per step: the element-force kernel, the node update (with the next
-            # predictor) and, for the ramp, the prescribed-motion kernel
-            "gpu_launches": args.steps * (3 if args.config == "tri6" else 2),
+            # per step: the element-force kernel and the node update (with the
+            # next predictor), or the fused step; for the ramp, the
+            # prescribed-motion kernel
+            "gpu_launches": args.steps * ((1 if fused else 2) + (args.config == "tri6")),
             # the state after the timed steps must be finite (device status word)
             "state_finite": m.getStatus() == 0 and bool(np.all(np.isfinite(m.getDisplacement()))),
         }
@@ -808,20 +810,21 @@ def run_batch(args, rep=None, emit=True, extra=False):
         nprof = min(args.steps, 20)
         _, phases = b.profileSteps(nprof)
         step_b, kern_b = algorithmic_bytes("batch", b.mesh, prec)
-        elem_ms = phases[1] / nprof
+        elem_ms = phases[1] / nprof  # the fused step, where the batch runs it
+        fused = b.getFusedStep()
         results[prec] = {
             "ms_per_step": ms / args.steps,
             "value": aggregate_rate(E * args.steps, world, ms),
             "phase_ms_per_step": {"predictor": phases[0] / nprof,
                                   "element_forces": phases[1] / nprof,
                                   "node_update": phases[2] / nprof},
-            "roofline": roofline_entry(kern_b, elem_ms, peak, peak_kind,
-                                       read_traffic("batch", prec)),
+            "roofline": roofline_entry(step_b if fused else kern_b, elem_ms, peak, peak_kind,
+                                       None if fused else read_traffic("batch", prec)),
             "roofline_step": {"bytes_per_element_step": step_b / E,
                               "achieved": step_b / (ms / args.steps / 1e3) / 1e9,
                               "frac": step_b / (ms / args.steps / 1e3) / 1e9 / peak},
             "clocks": clk.summary(),
-            "gpu_launches": args.steps * 2,
+            "gpu_launches": args.steps * (1 if fused else 2),
             "state_finite": b.getStatus() == 0 and bool(np.all(np.isfinite(b.getDisplacement()))),
         }
         if prec == precisions[0] and not extra:
@@ -1088,10 +1091,10 @@ def run_partitioned(args):
                        "subdomain_elements_rank0": local_elems,
                        "l2": "inputs larger than L2 (no flush)"},
             "clocks": clk.summary(),
-            # per step and subdomain: element forces, node update, the ramp
-            # (tri6), one halo pack and one unpack per neighbor (rank 0's
-            # subdomains)
-            "gpu_launches": args.steps * sum(2 + (1 if args.config == "tri6" else 0) +
+            # per step and subdomain: element forces and node update or the
+            # fused step, the ramp (tri6), one halo pack and one unpack per
+            # neighbor (rank 0's subdomains)
+            "gpu_launches": args.steps * sum((1 if lc.model.getFusedStep() else 2) + (1 if args.config == "tri6" else 0) +
                                              2 * len(lc.sub.neighbors) for lc in pm.locals),
         }
         print(json.dumps(line), flush=True)

@@ -418,6 +418,27 @@ int akb_model_set_launch_shape(akb_model *model, int law, int element_block,
  * Every form sums every node's slots in the same order. */
 int akb_model_set_node_shape(akb_model *model, int node_block, int staged);
 int akb_model_get_node_shape(const akb_model *model, int *node_block, int *staged);
+/* Fused step: the element forces and the node update of a step as one launch
+ * over compact patches of nodes (each block evaluates every element that
+ * touches its nodes and keeps the elemental forces in shared memory).  On
+ * after initFull where the model has it: one law group of tetrahedra
+ * (elastic, neohookean), of mixed-precision hexahedra (elastic, neohookean;
+ * at most about 15,000) that are all parallelepipeds, or of plastic
+ * triangles (at most about 20,000).  Choosing a launch shape, prefetch, geometry, streamed law
+ * or node form of the two-kernel step turns it off; AKB_EUNSUPPORTED when a
+ * model without it is asked for it.  The same numbers as the two-kernel step.
+ * No reference counterpart (a launch setting of this library). */
+int akb_model_set_fused_step(akb_model *model, int on);
+int akb_model_get_fused_step(const akb_model *model, int *on);
+/* Builds the fused step's plan of a mesh on the host, with at most max_own
+ * owned nodes per patch, and checks every index its kernel would use (for
+ * tests; no GPU).  node_offsets [nb_instances + 1]: the nodes of each instance
+ * of a batch ({0, nb_nodes} for one mesh).  stats: patches, patch elements
+ * (border elements counted in each patch), most nodes and most slots of a
+ * patch.  AKB_ESTATE when the plan is wrong. */
+int akb_patch_plan_check(int element_type, const double *nodes, int64_t nb_nodes,
+                         const int32_t *conn, int64_t nb_elements, int nb_instances,
+                         const int64_t *node_offsets, int max_own, int64_t *stats);
 /* TimeStepSolverDefault::predictor / corrector bookkeeping
  * (time_step_solver_default.cc:171-221): with tracking on, every step also
  * stores the displacement it starts from (AKB_PREVIOUS_DISPLACEMENT) and
