@@ -1713,18 +1713,38 @@ __global__ void __launch_bounds__(32 * NQ)
   }
 }
 
+// 8 bytes from global to shared memory without passing through registers
+__device__ __forceinline__ void copy_async_8(double *dst, const double *src) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy_async_wait() {
+  asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+}
+// one value read where it is used (ld_table's reason, from shared memory)
+__device__ __forceinline__ double ld_shared(const double *p) {
+  double v;
+  asm volatile("ld.shared.f64 %0, [%1];"
+               : "=d"(v)
+               : "r"((unsigned)__cvta_generic_to_shared(p))
+               : "memory");
+  return v;
+}
+
 // The FP64 law of one (element, point), the operations of
 // element_law<D, NN, LAW, double, false> in the same order, streamed: the
 // nodal displacements are read from the block's staging us[c][lane], the
-// point's dN/dx row b_a = B[(q ND + a D + j) E + e] is loaded node by node
-// where the gradient and the force use it, and each force component c is
-// handed to put(c, value) as soon as it is formed.  Nothing of size NN x D
-// stays in registers, which leaves room for more resident warps.
-template <int D, int NN, int LAW, class Put>
-__device__ __forceinline__ void element_law_streamed(const double (*us)[32], int lane,
-                                                     const double *Bq, int64_t E, double w,
-                                                     const MatParams &mp, const GroupArgs &ps,
-                                                     int64_t ne, int64_t le, int q, Put put) {
+// point's dN/dx row node by node where the gradient and the force use it, and
+// each force component c goes to row[c][lane] as soon as it is formed.
+// Nothing of size NN x D stays in registers, which leaves room for more
+// resident warps.  STAGED: the row is in row[c][lane], where the force
+// replaces it; otherwise entry c is at Bq[c E].
+template <int D, int NN, int LAW, bool STAGED>
+__device__ __forceinline__ void element_law_streamed(const double (*us)[32], double (*row)[32],
+                                                     int lane, const double *Bq, int64_t E,
+                                                     double w, const MatParams &mp,
+                                                     const GroupArgs &ps, int64_t ne, int64_t le,
+                                                     int q) {
   // grad u = u B^T (shape_functions_inline_impl.hh:303-310): g(i, j) =
   // u_0,i b_0,j, then + u_a,i b_a,j for a ascending
   double g[D * D];
@@ -1732,7 +1752,8 @@ __device__ __forceinline__ void element_law_streamed(const double (*us)[32], int
   for (int a = 0; a < NN; ++a) {
     double ba[D];
 #pragma unroll
-    for (int j = 0; j < D; ++j) ba[j] = Bq[(int64_t)(a * D + j) * E];
+    for (int j = 0; j < D; ++j)
+      ba[j] = STAGED ? row[a * D + j][lane] : Bq[(int64_t)(a * D + j) * E];
 #pragma unroll
     for (int j = 0; j < D; ++j)
 #pragma unroll
@@ -1751,9 +1772,11 @@ __device__ __forceinline__ void element_law_streamed(const double (*us)[32], int
     for (int a = 0; a < NN; ++a) {
       double ba[D];
 #pragma unroll
-      for (int j = 0; j < D; ++j) ba[j] = ld_table(Bq + (int64_t)(a * D + j) * E);
+      for (int j = 0; j < D; ++j)
+        ba[j] = STAGED ? ld_shared(&row[a * D + j][lane]) : ld_table(Bq + (int64_t)(a * D + j) * E);
 #pragma unroll
-      for (int k = 0; k < D; ++k) put(a * D + k, finite_force_component<D, double>(ba, g, Sv, k) * w);
+      for (int k = 0; k < D; ++k)
+        row[a * D + k][lane] = finite_force_component<D, double>(ba, g, Sv, k) * w;
     }
   } else {
     double sig[D * D];
@@ -1767,13 +1790,14 @@ __device__ __forceinline__ void element_law_streamed(const double (*us)[32], int
     for (int a = 0; a < NN; ++a) {
       double ba[D];
 #pragma unroll
-      for (int j = 0; j < D; ++j) ba[j] = ld_table(Bq + (int64_t)(a * D + j) * E);
+      for (int j = 0; j < D; ++j)
+        ba[j] = STAGED ? ld_shared(&row[a * D + j][lane]) : ld_table(Bq + (int64_t)(a * D + j) * E);
 #pragma unroll
       for (int i = 0; i < D; ++i) {
         double s = sig[i] * ba[0];
 #pragma unroll
         for (int j = 1; j < D; ++j) s = s + sig[i + D * j] * ba[j];
-        put(a * D + i, s * w);
+        row[a * D + i][lane] = s * w;
       }
     }
   }
@@ -1783,8 +1807,14 @@ __device__ __forceinline__ void element_law_streamed(const double (*us)[32], int
 // point, lane = element), the same gather, the same sums over q in
 // increasing order, bit for bit; every point's NN x D force components go to
 // shared memory [q][component][lane] as they are formed and are summed in
-// one round.  Dynamic shared memory: (NN D + NQ NN D) x 32 doubles (55,296
-// bytes for hexahedra in 3D, above the 48 KB of static shared memory).
+// one round.  The elastic law, whose arithmetic is short against the latency
+// of its dN/dx rows, has them copied there first, without registers and
+// before the preceding kernel ends (no step changes them), the forces taking
+// their place: 64^3 box 163.5 us per step against 187.9 read from L2 and 180.3
+// held in registers.  The neohookean law is bound by the FP64 and
+// shared-memory pipes (193.7 against 196.5 us staged).  Dynamic shared
+// memory: (NN D + NQ NN D) x 32 doubles (55,296 bytes for hexahedra in 3D,
+// above the 48 KB of static shared memory).
 template <int D, int NN, int NQ, int LAW>
 __global__ void __launch_bounds__(32 * NQ)
     k_element_forces_pqs(int64_t e_begin, int64_t e_count, int64_t E,
@@ -1792,17 +1822,25 @@ __global__ void __launch_bounds__(32 * NQ)
                          const double *__restrict__ B, const double *__restrict__ wJ,
                          const double *__restrict__ u, MatParams mp, GroupArgs ps,
                          double *__restrict__ re) {
-  pdl_begin();
   constexpr int ND = NN * D;
+  constexpr bool STAGED = LAW != LAW_NEOHOOKEAN;
   extern __shared__ double pqs_smem[];
   double(*us)[32] = reinterpret_cast<double(*)[32]>(pqs_smem);
   double(*red)[ND][32] = reinterpret_cast<double(*)[ND][32]>(pqs_smem + ND * 32);
   const int lane = threadIdx.x & 31;
   const int q = threadIdx.x >> 5;
   const int64_t le = (int64_t)blockIdx.x * 32 + lane;
+  const int64_t e = e_begin + le;
+  const double *Bq = B + (int64_t)q * ND * E + e;
+  if constexpr (STAGED) {
+    if (le < e_count) {
+#pragma unroll
+      for (int c = 0; c < ND; ++c) copy_async_8(&red[q][c][lane], Bq + (int64_t)c * E);
+    }
+  }
+  pdl_begin();
   const bool active = le < e_count && element_active(ps, le) &&
                       element_indices_ok<NN>(ps, conn, pos, E, e_begin + le);
-  const int64_t e = e_begin + le;
   if (active) {
     for (int a = q; a < NN; a += NQ) {
       const int64_t node = conn[(int64_t)a * E + e];
@@ -1810,13 +1848,12 @@ __global__ void __launch_bounds__(32 * NQ)
       for (int i = 0; i < D; ++i) us[a * D + i][lane] = u[node * D + i];
     }
   }
+  if constexpr (STAGED) copy_async_wait();
   __syncthreads();
   if (active) {
     const double w = wJ[(int64_t)q * E + e];
     const MatParams mpe = group_params(mp, ps, le);
-    element_law_streamed<D, NN, LAW>(us, lane, B + (int64_t)q * ND * E + e, E, w, mpe, ps,
-                                     e_count, le, q,
-                                     [&](int c, double v) { red[q][c][lane] = v; });
+    element_law_streamed<D, NN, LAW, STAGED>(us, red[q], lane, Bq, E, w, mpe, ps, e_count, le, q);
   }
   __syncthreads();
   if (active) {

@@ -34,14 +34,6 @@
 
 namespace akb {
 
-__device__ __forceinline__ void copy_async_8(double *dst, const double *src) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src) : "memory");
-}
-__device__ __forceinline__ void copy_async_wait() {
-  asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
-}
-
 __device__ __forceinline__ void prefetch_l2_line(const void *p) {
   asm volatile("prefetch.global.L2 [%0];" ::"l"(__cvta_generic_to_global(p)));
 }

@@ -1530,11 +1530,12 @@ int akb_model_init_full(akb_model *m, int method, int precision) {
       }
       // plain FP64 hexahedra, neohookean and plastic: the streamed per-point
       // law (64 instead of 126 and 128 instead of 168 registers), measured on
-      // B200: 128^3 neohookean element launch 1.342 against 1.572 ms, 48^3
-      // plastic 0.119 against 0.199 ms; elastic keeps the form holding its
-      // values in registers (1.277 against 1.316 ms streamed)
-      if (m->et == AKB_HEXAHEDRON_8 && precision == AKB_PRECISION_FP64 && gr.law != LAW_ELASTIC)
-        gr.tune.pqs = 1;
+      // B200: 128^3 neohookean element launch 1.342 against 1.572 ms, 64^3
+      // plastic step 0.282 against 0.490 ms.  Elastic: streamed from two waves
+      // of its blocks on (us per step, held / streamed: 28^3 15.5 / 16.2, 32^3
+      // 20.0 / 20.4, 36^3 32.1 / 30.0, 48^3 80.6 / 74.5, 64^3 183.0 / 165.0)
+      if (m->et == AKB_HEXAHEDRON_8 && precision == AKB_PRECISION_FP64)
+        gr.tune.pqs = gr.law != LAW_ELASTIC || E >= 2 * 148 * 4 * 32;
       gr.nmat++;
       gr.e_count += mt.e_count;
       mt.group = (int)m->groups.size() - 1;
@@ -1543,8 +1544,12 @@ int akb_model_init_full(akb_model *m, int method, int precision) {
   }
   // dependent launches: measured on B200 from 3k to 2M elements, 4-15 %
   // shorter steps on meshes below ~50k elements and even above, except FP64
-  // hexahedra (the per-point kernel), whose 16^3 and 32^3 steps were slower
-  m->pdl = !(m->et == AKB_HEXAHEDRON_8 && precision == AKB_PRECISION_FP64);
+  // hexahedra (the per-point kernel), whose 16^3 and 32^3 steps were slower;
+  // elastic ones of one wave of its blocks gain (us per step, plain /
+  // dependent: 8^3 7.75 / 7.48, 12^3 8.41 / 7.60, 20^3 9.66 / 9.27; 24^3 12.06
+  // / 12.56)
+  m->pdl = !(m->et == AKB_HEXAHEDRON_8 && precision == AKB_PRECISION_FP64) ||
+           (E <= 148 * 2 * 32 && m->groups.size() == 1 && m->groups[0].law == LAW_ELASTIC);
   std::vector<int64_t> iperm(E);  // user element -> internal element
   for (int64_t ie = 0; ie < E; ++ie) iperm[m->perm[ie]] = ie;
   std::vector<int32_t> conn_soa((size_t)nn * E);
