@@ -289,9 +289,12 @@ template <class EV, int THREADS> __host__ __device__ constexpr size_t patch_stag
 }
 
 // One step of patch blockIdx.x.  KAHAN: compensated sum (mixed path); MULTI:
-// a patch may hold several materials.  THREADS and MINB set how many warps
+// a patch may hold several materials; EARLY: the thread's first owned node is
+// read ahead, what no step changes before the preceding kernel has ended and
+// its state before the elements (otherwise its lines are prefetched into L2).
+// THREADS and MINB set how many warps
 // share a patch's shared memory and what their registers are capped at.
-template <class EV, bool KAHAN, bool MULTI, int THREADS, int MINB>
+template <class EV, bool KAHAN, bool MULTI, bool EARLY, int THREADS, int MINB>
 __global__ void __launch_bounds__(THREADS, MINB)
     k_patch_step(const __grid_constant__ PatchArgs pa, const __grid_constant__ MatParams mp,
                  const __grid_constant__ GroupArgs ps) {
@@ -330,6 +333,15 @@ __global__ void __launch_bounds__(THREADS, MINB)
     const int i = threadIdx.x + k * THREADS;
     id[k] = i < h.n_local ? nodes[i] : 0;
   }
+  PatchOwn o0;
+  NodeState<D> st0;
+  if constexpr (EARLY) {
+    if (threadIdx.x < h.n_own) {
+      o0 = own[threadIdx.x];
+      st0.m = pa.mass[o0.node];
+      st0.bl = pa.blocked[o0.node];
+    }
+  }
   pdl_begin();
   // a stopped instance keeps its state (k_node_update_retire)
   if (pa.inst_end && *pa.step >= pa.inst_end[h.inst]) {
@@ -353,12 +365,25 @@ __global__ void __launch_bounds__(THREADS, MINB)
 #pragma unroll
     for (int c = 0; c < D; ++c) copy_async_8(us + i * D + c, pa.u + n * D + c);
   }
-  // the owned nodes' state, which the update reads last, into L2 meanwhile
-  for (int i = threadIdx.x; i < h.n_own; i += THREADS) {
-    const int64_t node = own[i].node;
-    prefetch_l2_line(pa.a + node * D);
-    prefetch_l2_line(pa.v + node * D);
-    prefetch_l2_line(pa.mass + node);
+  auto load_state = [&](int64_t node, NodeState<D> &st) {
+#pragma unroll
+    for (int c = 0; c < D; ++c) {
+      const int64_t k = node * D + c;
+      st.a[c] = pa.a[k];
+      st.v[c] = pa.v[k];
+      st.f[c] = (pa.flags & NU_FEXT_ZERO) ? 0. : pa.fext[k];
+    }
+  };
+  if constexpr (EARLY) {
+    if (threadIdx.x < h.n_own) load_state(o0.node, st0);
+  } else {
+    // the owned nodes' state, which the update reads last, into L2 meanwhile
+    for (int i = threadIdx.x; i < h.n_own; i += THREADS) {
+      const int64_t node = own[i].node;
+      prefetch_l2_line(pa.a + node * D);
+      prefetch_l2_line(pa.v + node * D);
+      prefetch_l2_line(pa.mass + node);
+    }
   }
   const MatParams mph = (ps.mtab && h.mat >= 0) ? ps.mtab[h.mat] : mp;
   const double dt = pa.inst_dt ? pa.inst_dt[h.inst] : pa.dt;
@@ -399,19 +424,20 @@ __global__ void __launch_bounds__(THREADS, MINB)
   // the node update, one thread per owned node
   const int row = h.n_own * D;
   for (int i = threadIdx.x; i < h.n_own; i += THREADS) {
-    const PatchOwn o = own[i];
-    const int64_t node = o.node;
+    PatchOwn o;
     NodeState<D> st;
-    st.m = pa.mass[node];
-    st.bl = pa.blocked[node];
-#pragma unroll
-    for (int c = 0; c < D; ++c) {
-      const int64_t k = node * D + c;
-      st.a[c] = pa.a[k];
-      st.v[c] = pa.v[k];
-      st.f[c] = (pa.flags & NU_FEXT_ZERO) ? 0. : pa.fext[k];
-      st.u[c] = us[o.local * D + c];
+    if (EARLY && i < THREADS) {
+      o = o0;
+      st = st0;
+    } else {
+      o = own[i];
+      st.m = pa.mass[o.node];
+      st.bl = pa.blocked[o.node];
+      load_state(o.node, st);
     }
+    const int64_t node = o.node;
+#pragma unroll
+    for (int c = 0; c < D; ++c) st.u[c] = us[o.local * D + c];
     double acc[D], comp[D];
 #pragma unroll
     for (int c = 0; c < D; ++c) acc[c] = comp[c] = 0.;

@@ -1020,7 +1020,9 @@ int reduce_to_host(akb_model *m, const double *x, int64_t n, bool op_min, double
 // Plastic triangles: a small mesh's step is as long as the rounds its
 // patches' six warps need for all (32 elements, point) items (us per step,
 // two kernels / fused with one round / with two: 2 k triangles of 6 points
-// FP64 18.5 / 6.7 / 9.3, 8 k of 3 points mixed 12.8 / 7.5 / 10.2).  With more
+// FP64 18.5 / 6.7 / 9.3, 8 k of 3 points mixed 12.8 / 7.5 / 10.2); of the edges
+// with the fewest rounds the smallest that gives an SM one patch (2 k of 3
+// points mixed, 6.5 with 121 patches, 7.9 with 64), else the largest.  With more
 // patches than are resident at once the two kernels, which read every point's
 // state once, are faster (512^2 x 2: 111 against 154).
 int patch_nodes(int et, int rule, int precision, int64_t N, int64_t E, int ninst) {
@@ -1031,12 +1033,13 @@ int patch_nodes(int et, int rule, int precision, int64_t N, int64_t E, int ninst
   double least = 0.;
   if (et == AKB_TRIANGLE_6) {
     for (int s = 12; s >= 2; --s) {
-      const double slabs = std::ceil(planes / s - 1e-6), a = planes / slabs;
+      const double slabs = std::ceil(planes / s - 1e-6), side = std::ceil(planes / slabs - 1e-6);
       // resident blocks per SM, fewer with the slots of 6 points
-      if (ninst * slabs * slabs > sms * (rule ? 2. : mixed ? 4. : 3.)) break;
-      const double elements = 2. * (a / 2. + 1.) * (a / 2. + 1.);
-      const double rounds = std::ceil(std::ceil(elements / 32.) * (rule ? 6. : 3.) / 6.);
-      if (least == 0. || rounds < least) {
+      const double patches = ninst * slabs * slabs;
+      if (patches > sms * (rule ? 2. : mixed ? 4. : 3.)) break;
+      const double cells = std::floor((side + 1.) / 2.) + 1.;  // that its node planes touch
+      const double rounds = std::ceil(std::ceil(2. * cells * cells / 32.) * (rule ? 6. : 3.) / 6.);
+      if (least == 0. || rounds < least || (rounds == least && patches <= sms)) {
         least = rounds;
         best = s;
       }
@@ -1201,6 +1204,7 @@ int finish_patches(akb_model *m, PatchTask &task) {
   std::memcpy(local.data() + lb, plan.slot.data(), lb);
   AKB_CUDA(cudaMemcpyAsync(base, lists.data(), lists.size(), cudaMemcpyHostToDevice, s));
   pa.npatch = (int64_t)plan.head.size();
+  pa.max_own = task.mesh.max_own;
   pa.multi = 0;
   for (const PatchHead &h : plan.head) pa.multi |= gr.nmat > 1 && h.mat < 0 && h.n_elem > 0;
   pa.head = (const PatchHead *)(base + o_head);

@@ -87,8 +87,11 @@ inline size_t patch_smem(int D, int max_local, int max_slots, size_t slot_value)
 constexpr size_t kPatchMaxSmem = 232448;  // 227 KB, the most one block can have
 constexpr size_t kPatchStageSmem = 18432;  // staged element tables of the hexahedron kernel
 
+constexpr int64_t kPatchSms = 148;
+
 struct PatchArgs {
   int64_t npatch = 0;
+  int max_own = 0;  // owned nodes of a patch at most
   const PatchHead *head = nullptr;
   const int32_t *nodes = nullptr;
   const PatchOwn *own = nullptr;
