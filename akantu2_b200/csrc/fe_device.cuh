@@ -10,6 +10,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "presc.h"
+
 namespace akb {
 
 enum { ET_TET4 = 0, ET_HEX8 = 1, ET_TRI6 = 2 };

@@ -1910,8 +1910,9 @@ __device__ __forceinline__ void accumulate_slot(const double *rv, double *acc, d
 // the node update after the gather: f_int = acc, residual, solve, corrector
 // and predictor of node i (its nodal state is loaded after the gather: loaded
 // before it, with the slots, the update was measured slower, 0.120 against
-// 0.107 ms on the 128^3 hexahedral box, at 66 instead of 50 registers)
-template <int D>
+// 0.107 ms on the 128^3 hexahedral box, at 66 instead of 50 registers).
+// RAMP: the prescribed dofs of u_next are left to prescribe_block
+template <int D, bool RAMP = false>
 __device__ __forceinline__ void node_apply(int64_t i, const double *acc, const double *fext,
                                            const double *mass, const uint8_t *blocked,
                                            double *fint, double *a, double *v, const double *u,
@@ -1956,7 +1957,7 @@ __device__ __forceinline__ void node_apply(int64_t i, const double *acc, const d
       a[k] = an;
       bad |= !isfinite(an);
     }
-    if (flags & NU_PREDICT) {
+    if ((flags & NU_PREDICT) && !(RAMP && ((bl >> (kPrescribedBit + c)) & 1))) {
       const double uk = u[k];
       u_next[k] = free_dof ? __dadd_rn(uk, __dadd_rn(__dmul_rn(dt, vk),
                                                      __dmul_rn(hdt, __dmul_rn(dt, an))))
@@ -1964,6 +1965,30 @@ __device__ __forceinline__ void node_apply(int64_t i, const double *acc, const d
     }
   }
   if (bad) atomicOr(status, 1u);
+}
+
+// One block advances the ramp by a step and writes the prescribed dofs of the
+// displacement u; explicitly rounded, the same in every translation unit.  A
+// node update writes every other dof of u, so it runs as an extra block of
+// the update's launch instead of a launch of its own after it (100 us of 100
+// steps of a small mesh).
+__device__ __forceinline__ void prescribe_block(const PrescArgs &pr, double *u, bool advance) {
+  __shared__ double a_sh;
+  if (threadIdx.x == 0) {
+    double a = *pr.acc;
+    if (advance) {
+      const int64_t k = *pr.step + 1;
+      const double vk = __dmul_rn(pr.v_max, fmin(1.0, __ddiv_rn((double)k, pr.ramp)));
+      a = __dadd_rn(a, __dmul_rn(pr.dt, vk));
+      *pr.step = k;
+      *pr.acc = a;
+    }
+    a_sh = a;
+  }
+  __syncthreads();
+  const double a = a_sh;
+  for (int64_t i = threadIdx.x; i < pr.count; i += blockDim.x)
+    u[pr.dofs[i]] = __dadd_rn(pr.u0[i], a);
 }
 
 // 32 bytes of the slot array as one load (sm_100 256-bit global load): two
@@ -2020,7 +2045,7 @@ __device__ __forceinline__ void load_node_state(NodeState<D> &st, int64_t i, con
 }
 
 // node_apply on preloaded inputs: the same operations in the same order
-template <int D>
+template <int D, bool RAMP = false>
 __device__ __forceinline__ void node_apply_state(int64_t i, const double *acc,
                                                  const NodeState<D> &st, double *fint, double *a,
                                                  double *v, double *u_next, double dt,
@@ -2062,7 +2087,7 @@ __device__ __forceinline__ void node_apply_state(int64_t i, const double *acc,
       a[k] = an;
       bad |= !isfinite(an);
     }
-    if (flags & NU_PREDICT) {
+    if ((flags & NU_PREDICT) && !(RAMP && ((bl >> (kPrescribedBit + c)) & 1))) {
       const double uk = st.u[c];
       u_next[k] = free_dof ? __dadd_rn(uk, __dadd_rn(__dmul_rn(dt, vk),
                                                      __dmul_rn(hdt, __dmul_rn(dt, an))))
@@ -2142,7 +2167,7 @@ __device__ __forceinline__ void gather_slots(int32_t p0, int32_t p1, const RT *r
 }
 
 // the gather and the node update of node i (WIDE: 32-byte slot loads)
-template <int D, class RT, bool KAHAN, bool WIDE = false>
+template <int D, class RT, bool KAHAN, bool WIDE = false, bool RAMP = false>
 __device__ __forceinline__ void node_body(int64_t i, const int32_t *ptr,
                                           const RT *re,
                                           const double *fext,
@@ -2162,14 +2187,14 @@ __device__ __forceinline__ void node_body(int64_t i, const int32_t *ptr,
   }
   const int32_t p0 = ptr[i], p1 = ptr[i + 1];
   gather_slots<D, RT, KAHAN, WIDE>(p0, p1, re, acc, comp);
-  node_apply<D>(i, acc, fext, mass, blocked, fint, a, v, u, u_next, dt, node_inst, inst_dt, flags,
+  node_apply<D, RAMP>(i, acc, fext, mass, blocked, fint, a, v, u, u_next, dt, node_inst, inst_dt, flags,
                 status);
 }
 
 
 // launched with up to 1024 threads per block (the autotuner's candidates):
 // at most 64 registers
-template <int D, class RT, bool KAHAN, bool WIDE = false>
+template <int D, class RT, bool KAHAN, bool WIDE = false, bool RAMP = false>
 __global__ void __launch_bounds__(1024) k_node_update(int64_t N, const int32_t *__restrict__ ptr,
                               const RT *__restrict__ re, const double *__restrict__ fext,
                               const double *__restrict__ mass,
@@ -2178,11 +2203,12 @@ __global__ void __launch_bounds__(1024) k_node_update(int64_t N, const int32_t *
                               const double *__restrict__ u, double *__restrict__ u_next,
                               double dt, const int32_t *__restrict__ node_inst,
                               const double *__restrict__ inst_dt, int flags,
-                              unsigned int *__restrict__ status) {
+                              unsigned int *__restrict__ status, const PrescArgs pr) {
   pdl_begin();
+  if (RAMP && blockIdx.x == gridDim.x - 1) return prescribe_block(pr, u_next, true);
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N || !node_range_ok(ptr, N, i, status)) return;
-  node_body<D, RT, KAHAN, WIDE>(i, ptr, re, fext, mass, blocked, fint, a, v, u, u_next, dt,
+  node_body<D, RT, KAHAN, WIDE, RAMP>(i, ptr, re, fext, mass, blocked, fint, a, v, u, u_next, dt,
                                 node_inst, inst_dt, flags, status);
 }
 
@@ -2191,7 +2217,7 @@ __global__ void __launch_bounds__(1024) k_node_update(int64_t N, const int32_t *
 // wait on the preceding kernel (a dependent launch starts them under that
 // kernel's tail), and its a, v, f_ext and u before the slot gather, so that
 // they are in flight together with it rather than after it
-template <int D, class RT, bool KAHAN, bool WIDE = false>
+template <int D, class RT, bool KAHAN, bool WIDE = false, bool RAMP = false>
 __global__ void __launch_bounds__(1024)
     k_node_update_early(int64_t N, const int32_t *__restrict__ ptr, const RT *__restrict__ re,
                         const double *__restrict__ fext, const double *__restrict__ mass,
@@ -2199,7 +2225,7 @@ __global__ void __launch_bounds__(1024)
                         double *__restrict__ a, double *__restrict__ v,
                         const double *__restrict__ u, double *__restrict__ u_next, double dt,
                         const int32_t *__restrict__ node_inst, const double *__restrict__ inst_dt,
-                        int flags, unsigned int *__restrict__ status) {
+                        int flags, unsigned int *__restrict__ status, const PrescArgs pr) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const bool in = i < N;
   int32_t p0 = 0, p1 = 0;
@@ -2213,6 +2239,7 @@ __global__ void __launch_bounds__(1024)
     st.bl = blocked[i];
   }
   pdl_begin();
+  if (RAMP && blockIdx.x == gridDim.x - 1) return prescribe_block(pr, u_next, true);
   if (!in || !node_range_ok(ptr, N, i, status)) return;
   if (flags & NU_CORRECT) load_node_state<D>(st, i, fext, a, v, u, flags);
   double acc[D], comp[D];
@@ -2222,7 +2249,7 @@ __global__ void __launch_bounds__(1024)
     comp[c] = 0.;
   }
   gather_slots<D, RT, KAHAN, WIDE>(p0, p1, re, acc, comp);
-  node_apply_state<D>(i, acc, st, fint, a, v, u_next, dt, node_inst, inst_dt, flags, status);
+  node_apply_state<D, RAMP>(i, acc, st, fint, a, v, u_next, dt, node_inst, inst_dt, flags, status);
 }
 
 // Node update of a batch whose instances stop after their own step counts:
@@ -2281,7 +2308,7 @@ constexpr int kStagedBytes = 32768;
 
 __device__ __forceinline__ int swizzle(int w) { return w ^ ((w >> 3) & 7); }
 
-template <int D, class RT, bool KAHAN, int BLOCK>
+template <int D, class RT, bool KAHAN, int BLOCK, bool RAMP = false>
 __global__ void __launch_bounds__(BLOCK)
     k_node_update_staged(int64_t N, const int32_t *__restrict__ ptr, const RT *__restrict__ re,
                          const double *__restrict__ fext, const double *__restrict__ mass,
@@ -2290,8 +2317,9 @@ __global__ void __launch_bounds__(BLOCK)
                          const double *__restrict__ u, double *__restrict__ u_next, double dt,
                          const int32_t *__restrict__ node_inst,
                          const double *__restrict__ inst_dt, int flags,
-                         unsigned int *__restrict__ status) {
+                         unsigned int *__restrict__ status, const PrescArgs pr) {
   pdl_begin();
+  if (RAMP && blockIdx.x == gridDim.x - 1) return prescribe_block(pr, u_next, true);
   using V = typename SlotVec<D, RT>::type;
   constexpr int WPS = SlotVec<D, RT>::per_slot;  // vectors per slot
   constexpr int CAPW = kStagedBytes / (int)sizeof(V);
@@ -2332,7 +2360,7 @@ __global__ void __launch_bounds__(BLOCK)
     }
   }
   if (i >= N) return;
-  node_apply<D>(i, acc, fext, mass, blocked, fint, a, v, u, u_next, dt, node_inst, inst_dt, flags,
+  node_apply<D, RAMP>(i, acc, fext, mass, blocked, fint, a, v, u, u_next, dt, node_inst, inst_dt, flags,
                 status);
 }
 

@@ -302,6 +302,10 @@ __global__ void __launch_bounds__(THREADS, MINB)
   using Chunk = typename EV::Chunk;
   constexpr int D = EV::D, W = THREADS / 32, U = EV::kIds;
   extern __shared__ __align__(16) char patch_sm[];
+  if (pa.presc.count && blockIdx.x == gridDim.x - 1) {
+    pdl_begin();
+    return prescribe_block(pa.presc, pa.u_next, true);
+  }
   const PatchHead h = pa.head[blockIdx.x];
   const int32_t *nodes = pa.nodes + h.node0;
   const PatchOwn *own = pa.own + h.own0;
@@ -455,7 +459,7 @@ __global__ void __launch_bounds__(THREADS, MINB)
       }
       accumulate_slot<D, KAHAN>(rv, acc, comp);
     }
-    node_apply_state<D>(node, acc, st, pa.fint, pa.a, pa.v, pa.u_next, dt, nullptr, nullptr,
+    node_apply_state<D, true>(node, acc, st, pa.fint, pa.a, pa.v, pa.u_next, dt, nullptr, nullptr,
                         pa.flags, pa.status);
   }
 }

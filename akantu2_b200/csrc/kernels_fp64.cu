@@ -127,32 +127,40 @@ cudaError_t launch_node_update_fp64(const DevGeom &g, const double *re, const do
                        g.node_inst, g.inst_dt, g.inst_end, (const int64_t *)g.step, flags, status);
   }
   if (g.N == 0) return cudaSuccess;
+  const unsigned extra = g.presc.count ? 1 : 0;  // the block of the prescribed motion
 #ifdef AKB_BOUNDS_CHECK
   if (form == 1) form = 0;  // the bounds-checking build checks each node's own slot range
 #endif
+  auto go = [&](auto kern, int block) {
+    return launch_step(g.pdl, kern, grid_for(g.N, block) + extra, block, s, g.N, g.ptr, re, fext,
+                       mass, blocked, fint, a, v, u, u_next, dt, g.node_inst, g.inst_dt, flags,
+                       status, g.presc);
+  };
   if (form == 1) {
     AKB_DISPATCH_NODE_BLOCK(node_block, {
-      auto kern = g.D == 3 ? k_node_update_staged<3, double, false, NB>
-                           : k_node_update_staged<2, double, false, NB>;
-      return launch_step(g.pdl, kern, grid_for(g.N, NB), NB, s, g.N, g.ptr, re, fext, mass,
-                         blocked, fint, a, v, u, u_next, dt, g.node_inst, g.inst_dt, flags,
-                         status);
+      if (extra)
+        return go(g.D == 3 ? k_node_update_staged<3, double, false, NB, true>
+                           : k_node_update_staged<2, double, false, NB, true>, NB);
+      return go(g.D == 3 ? k_node_update_staged<3, double, false, NB>
+                         : k_node_update_staged<2, double, false, NB>, NB);
     });
   }
   // slots read 32 bytes at a time when the array's alignment allows it
   const bool wide = ((uintptr_t)re & 31) == 0;
-  auto kern = g.D == 3 ? (wide ? k_node_update<3, double, false, true>
-                               : k_node_update<3, double, false>)
-                       : (wide ? k_node_update<2, double, false, true>
-                               : k_node_update<2, double, false>);
-  if (form == 2)
-    kern = g.D == 3 ? (wide ? k_node_update_early<3, double, false, true>
-                            : k_node_update_early<3, double, false>)
-                    : (wide ? k_node_update_early<2, double, false, true>
-                            : k_node_update_early<2, double, false>);
-  return launch_step(g.pdl, kern, grid_for(g.N, node_block), node_block, s, g.N, g.ptr, re,
-                     fext, mass, blocked, fint, a, v, u, u_next, dt, g.node_inst, g.inst_dt,
-                     flags, status);
+  auto pick = [&](auto ramp) {
+    constexpr bool R = decltype(ramp)::value;
+    auto kern = g.D == 3 ? (wide ? k_node_update<3, double, false, true, R>
+                                 : k_node_update<3, double, false, false, R>)
+                         : (wide ? k_node_update<2, double, false, true, R>
+                                 : k_node_update<2, double, false, false, R>);
+    if (form == 2)
+      kern = g.D == 3 ? (wide ? k_node_update_early<3, double, false, true, R>
+                              : k_node_update_early<3, double, false, false, R>)
+                      : (wide ? k_node_update_early<2, double, false, true, R>
+                              : k_node_update_early<2, double, false, false, R>);
+    return go(kern, node_block);
+  };
+  return extra ? pick(std::true_type()) : pick(std::false_type());
 }
 
 // prescribed motion: before step k (k = 1, 2, ... since the motion was set)
@@ -162,32 +170,13 @@ cudaError_t launch_node_update_fp64(const DevGeom &g, const double *re, const do
 // running sum (advance != 0; else the sum of the coming step is applied
 // again), then the block writes the dofs into the displacement the coming
 // step starts from.
-__global__ void k_prescribe(int64_t count, const int64_t *__restrict__ dofs,
-                            const double *__restrict__ u0, double v_max, double ramp_steps,
-                            double dt, double *__restrict__ acc, int64_t *__restrict__ step,
-                            double *__restrict__ u, int advance) {
+__global__ void k_prescribe(PrescArgs pr, double *__restrict__ u, int advance) {
   pdl_begin();
-  __shared__ double a_sh;
-  if (threadIdx.x == 0) {
-    double a = *acc;
-    if (advance) {
-      const int64_t k = *step + 1;
-      const double vk = v_max * fmin(1.0, (double)k / ramp_steps);
-      a = a + dt * vk;
-      *step = k;
-      *acc = a;
-    }
-    a_sh = a;
-  }
-  __syncthreads();
-  const double a = a_sh;
-  for (int64_t i = threadIdx.x; i < count; i += blockDim.x) u[dofs[i]] = u0[i] + a;
+  prescribe_block(pr, u, advance != 0);
 }
-cudaError_t launch_prescribe(int64_t count, const int64_t *dofs, const double *u0, double v_max,
-                             int64_t ramp_steps, double dt, double *acc, int64_t *step,
-                             double *u, bool advance, bool pdl, cudaStream_t s) {
-  return launch_step(pdl, k_prescribe, 1, 512, s, count, dofs, u0, v_max, (double)ramp_steps,
-                     dt, acc, step, u, advance ? 1 : 0);
+cudaError_t launch_prescribe(const PrescArgs &pr, double *u, bool advance, bool pdl,
+                             cudaStream_t s) {
+  return launch_step(pdl, k_prescribe, 1, 512, s, pr, u, advance ? 1 : 0);
 }
 
 cudaError_t launch_step_advance(const DevGeom &g, cudaStream_t s) {

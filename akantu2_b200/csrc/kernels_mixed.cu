@@ -185,30 +185,40 @@ cudaError_t launch_node_update_mixed(const DevGeom &g, const float *re, const do
                        g.node_inst, g.inst_dt, g.inst_end, (const int64_t *)g.step, flags, status);
   }
   if (g.N == 0) return cudaSuccess;
+  const unsigned extra = g.presc.count ? 1 : 0;  // the block of the prescribed motion
 #ifdef AKB_BOUNDS_CHECK
   if (form == 1) form = 0;  // the bounds-checking build checks each node's own slot range
 #endif
+  auto go = [&](auto kern, int block) {
+    return launch_step(g.pdl, kern, grid_for(g.N, block) + extra, block, s, g.N, g.ptr, re, fext,
+                       mass, blocked, fint, a, v, u, u_next, dt, g.node_inst, g.inst_dt, flags,
+                       status, g.presc);
+  };
   if (form == 1) {
     AKB_DISPATCH_NODE_BLOCK(node_block, {
-      auto kern = g.D == 3 ? k_node_update_staged<3, float, true, NB>
-                           : k_node_update_staged<2, float, true, NB>;
-      return launch_step(g.pdl, kern, grid_for(g.N, NB), NB, s, g.N, g.ptr, re, fext, mass,
-                         blocked, fint, a, v, u, u_next, dt, g.node_inst, g.inst_dt, flags,
-                         status);
+      if (extra)
+        return go(g.D == 3 ? k_node_update_staged<3, float, true, NB, true>
+                           : k_node_update_staged<2, float, true, NB, true>, NB);
+      return go(g.D == 3 ? k_node_update_staged<3, float, true, NB>
+                         : k_node_update_staged<2, float, true, NB>, NB);
     });
   }
   // slots read 32 bytes at a time when the array's alignment allows it
   const bool wide = ((uintptr_t)re & 31) == 0;
-  auto kern = g.D == 3 ? (wide ? k_node_update<3, float, true, true> : k_node_update<3, float, true>)
-                       : (wide ? k_node_update<2, float, true, true> : k_node_update<2, float, true>);
-  if (form == 2)
-    kern = g.D == 3 ? (wide ? k_node_update_early<3, float, true, true>
-                            : k_node_update_early<3, float, true>)
-                    : (wide ? k_node_update_early<2, float, true, true>
-                            : k_node_update_early<2, float, true>);
-  return launch_step(g.pdl, kern, grid_for(g.N, node_block), node_block, s, g.N, g.ptr, re,
-                     fext, mass, blocked, fint, a, v, u, u_next, dt, g.node_inst, g.inst_dt,
-                     flags, status);
+  auto pick = [&](auto ramp) {
+    constexpr bool R = decltype(ramp)::value;
+    auto kern = g.D == 3 ? (wide ? k_node_update<3, float, true, true, R>
+                                 : k_node_update<3, float, true, false, R>)
+                         : (wide ? k_node_update<2, float, true, true, R>
+                                 : k_node_update<2, float, true, false, R>);
+    if (form == 2)
+      kern = g.D == 3 ? (wide ? k_node_update_early<3, float, true, true, R>
+                              : k_node_update_early<3, float, true, false, R>)
+                      : (wide ? k_node_update_early<2, float, true, true, R>
+                              : k_node_update_early<2, float, true, false, R>);
+    return go(kern, node_block);
+  };
+  return extra ? pick(std::true_type()) : pick(std::false_type());
 }
 
 cudaError_t launch_hex8_affine_geometry(const DevGeom &g, float *geo, cudaStream_t s) {

@@ -69,6 +69,8 @@ struct DevGeom {
   // at which each instance stops and the device step counter (null otherwise)
   const int64_t *inst_end = nullptr;
   int64_t *step = nullptr;
+  // prescribed motion written by the node update's launch (count 0: none)
+  PrescArgs presc;
 };
 
 // ---- init ------------------------------------------------------------------
@@ -139,9 +141,8 @@ cudaError_t launch_step_advance(const DevGeom &g, cudaStream_t s);
 // prescribed velocity ramp on a set of dofs (u indices node * D + c), written
 // into the displacement the next step starts from; acc and step live on the
 // device so that captured graphs replay it
-cudaError_t launch_prescribe(int64_t count, const int64_t *dofs, const double *u0, double v_max,
-                             int64_t ramp_steps, double dt, double *acc, int64_t *step,
-                             double *u, bool advance, bool pdl, cudaStream_t s);
+cudaError_t launch_prescribe(const PrescArgs &pr, double *u, bool advance, bool pdl,
+                             cudaStream_t s);
 
 // persistent multi-step kernel (one law group; sa describes the steps);
 // qu: points per iteration of mixed hexahedra (1 or 2)

@@ -306,6 +306,7 @@ struct akb_model {
   unsigned int bar_late_us = 0;
   // prescribed velocity ramp on a set of dofs (akb_model_set_prescribed_velocity_ramp)
   int64_t presc_count = 0, presc_ramp = 1;
+  std::vector<int64_t> presc_dofs;
   double presc_vmax = 0.;
   int64_t *dpresc_dofs = nullptr, *dpresc_step = nullptr;
   double *dpresc_u0 = nullptr, *dpresc_acc = nullptr;
@@ -630,13 +631,24 @@ int element_forces(akb_model *m, bool in_step) {
   return AKB_OK;
 }
 
+PrescArgs presc_args(const akb_model *m) {
+  PrescArgs pr;
+  pr.count = m->presc_count;
+  pr.dofs = m->dpresc_dofs;
+  pr.u0 = m->dpresc_u0;
+  pr.v_max = m->presc_vmax;
+  pr.ramp = (double)m->presc_ramp;
+  pr.dt = m->dt;
+  pr.acc = m->dpresc_acc;
+  pr.step = m->dpresc_step;
+  return pr;
+}
+
 // the prescribed dofs of the step that starts from u_start: advanced to the
 // next step of the ramp, or the value of the coming step applied again
 int prescribe(akb_model *m, double *u_start, bool advance) {
   if (m->presc_count == 0) return AKB_OK;
-  AKB_CUDA(launch_prescribe(m->presc_count, m->dpresc_dofs, m->dpresc_u0, m->presc_vmax,
-                            m->presc_ramp, m->dt, m->dpresc_acc, m->dpresc_step, u_start,
-                            advance, m->pdl, m->stream));
+  AKB_CUDA(launch_prescribe(presc_args(m), u_start, advance, m->pdl, m->stream));
   m->presc_ahead = true;
   return AKB_OK;
 }
@@ -663,6 +675,10 @@ int node_update(akb_model *m, bool correct) {
   if (correct && m->fext_zero) flags |= NU_FEXT_ZERO;
   const double *u = m->u_pred();
   double *u_next = m->u();
+  // the next step's prescribed dofs are written by the same launch (a batch
+  // with stopping instances has an update kernel of its own)
+  const bool with_ramp = correct && !m->dinst_end;
+  if (with_ramp) g.presc = presc_args(m);
   if (m->precision == AKB_PRECISION_MIXED)
     e = launch_node_update_mixed(g, (const float *)m->dre, m->dfext, m->dmass, m->dblocked,
                                  m->dfint, m->da, m->dv, u, u_next, m->dt, flags, m->dstatus,
@@ -672,7 +688,8 @@ int node_update(akb_model *m, bool correct) {
                                 m->dfint, m->da, m->dv, u, u_next, m->dt, flags, m->dstatus,
                                 m->node_block, m->node_form, m->stream);
   if (e != cudaSuccess) return fail(AKB_ECUDA, std::string("node update: ") + cudaGetErrorString(e));
-  if (correct) AKB_TRY(prescribe(m, u_next, true));
+  if (with_ramp) m->presc_ahead = m->presc_count > 0 || m->presc_ahead;
+  else if (correct) AKB_TRY(prescribe(m, u_next, true));
   m->fint_valid = !correct;
   return AKB_OK;
 }
@@ -724,9 +741,12 @@ int patch_step(akb_model *m, bool store_fint) {
   pa.status = m->dstatus;
   pa.flags = NU_CORRECT | NU_PREDICT | (m->fext_zero ? NU_FEXT_ZERO : 0) |
              (store_fint ? NU_FINT : 0);
+  const bool with_ramp = !m->dinst_end;  // as in node_update
+  if (with_ramp) pa.presc = presc_args(m);
   const cudaError_t e = launch_patches(m, pa, group_args(m, m->groups[0], true), m->pdl);
   if (e != cudaSuccess) return fail(AKB_ECUDA, std::string("fused step: ") + cudaGetErrorString(e));
-  AKB_TRY(prescribe(m, m->u(), true));
+  if (with_ramp) m->presc_ahead = m->presc_count > 0 || m->presc_ahead;
+  else AKB_TRY(prescribe(m, m->u(), true));
   m->fint_valid = store_fint;
   return AKB_OK;
 }
@@ -1974,6 +1994,8 @@ int akb_model_set_nodal(akb_model *m, int field, const void *host, int64_t nbyte
     for (int64_t i = 0; i < m->N; ++i)
       for (int c = 0; c < m->dim; ++c)
         if (b[i * m->dim + c]) mask[i] |= (uint8_t)(1u << c);
+    for (int64_t k : m->presc_dofs)
+      mask[k / m->dim] |= (uint8_t)(1u << (kPrescribedBit + k % m->dim));
     AKB_CUDA(cudaMemcpyAsync(m->dblocked, mask.data(), m->N, cudaMemcpyHostToDevice, m->stream));
     AKB_CUDA(cudaStreamSynchronize(m->stream));
     m->predicted = false;
@@ -2356,13 +2378,18 @@ int akb_model_set_prescribed_velocity_ramp(akb_model *m, const int64_t *dofs, in
   for (auto &x : m->graphs) cudaGraphExecDestroy(x.exec);
   m->graphs.clear();
   m->presc_count = 0;
-  if (count == 0) return AKB_OK;
-  // the dofs are blocked from now on
+  if (count == 0 && m->presc_dofs.empty()) return AKB_OK;
+  // the dofs are blocked from now on, and marked as prescribed
   std::vector<uint8_t> mask(m->N);
   AKB_CUDA(cudaMemcpyAsync(mask.data(), m->dblocked, m->N, cudaMemcpyDeviceToHost, s));
   AKB_CUDA(cudaStreamSynchronize(s));
-  for (int64_t k = 0; k < count; ++k) mask[dofs[k] / m->dim] |= (uint8_t)(1u << (dofs[k] % m->dim));
+  for (uint8_t &x : mask) x &= (uint8_t)((1u << kPrescribedBit) - 1);
+  m->presc_dofs.assign(dofs, dofs + count);
+  for (int64_t k : m->presc_dofs)
+    mask[k / m->dim] |= (uint8_t)((1u | 1u << kPrescribedBit) << (k % m->dim));
   AKB_CUDA(cudaMemcpyAsync(m->dblocked, mask.data(), m->N, cudaMemcpyHostToDevice, s));
+  AKB_CUDA(cudaStreamSynchronize(s));
+  if (count == 0) return AKB_OK;
   // starting displacement of the dofs
   std::vector<double> u(nd), u0(count);
   AKB_CUDA(cudaMemcpyAsync(u.data(), m->u(), sizeof(double) * nd, cudaMemcpyDeviceToHost, s));

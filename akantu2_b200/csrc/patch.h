@@ -10,6 +10,8 @@
 
 #include <vector>
 
+#include "presc.h"
+
 namespace akb {
 
 struct GroupArgs;
@@ -84,7 +86,8 @@ inline size_t patch_smem(int D, int max_local, int max_slots, size_t slot_value)
   const size_t nod = ((size_t)max_local * D + 1) & ~(size_t)1;
   return sizeof(double) * nod + slot_value * (size_t)max_slots * D;
 }
-constexpr size_t kPatchMaxSmem = 232448;  // 227 KB, the most one block can have
+// 227 KB, the most one block can have, less the kernel's static variables
+constexpr size_t kPatchMaxSmem = 232448 - 1024;
 constexpr size_t kPatchStageSmem = 18432;  // staged element tables of the hexahedron kernel
 
 constexpr int64_t kPatchSms = 148;
@@ -113,6 +116,7 @@ struct PatchArgs {
   const int64_t *inst_end = nullptr, *step = nullptr;
   int flags = 0;
   unsigned int *status = nullptr;
+  PrescArgs presc;  // prescribed motion, written by an extra block
 };
 
 // fills the chunks: conn and slot [entries][NNP], and rows value rows of

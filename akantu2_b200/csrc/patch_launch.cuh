@@ -28,7 +28,8 @@ cudaError_t launch_patch(const PatchArgs &pa, const MatParams &mp, const GroupAr
   static_assert(patch_stage_bytes<EV, THREADS>() <= kPatchStageSmem, "staging");
   const size_t smem = pa.smem + patch_stage_bytes<EV, THREADS>();
   if (smem > kPatchMaxSmem) return cudaErrorInvalidConfiguration;
-  return launch_step_smem(pdl, kern, (unsigned)pa.npatch, THREADS, smem, s, pa, mp, ps);
+  return launch_step_smem(pdl, kern, (unsigned)pa.npatch + (pa.presc.count ? 1 : 0), THREADS,
+                          smem, s, pa, mp, ps);
 }
 
 template <class EV, bool KAHAN, bool EARLY, int THREADS, int MINB>
