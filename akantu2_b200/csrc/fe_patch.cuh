@@ -291,10 +291,11 @@ template <class EV, int THREADS> __host__ __device__ constexpr size_t patch_stag
 // One step of patch blockIdx.x.  KAHAN: compensated sum (mixed path); MULTI:
 // a patch may hold several materials; EARLY: the thread's first owned node is
 // read ahead, what no step changes before the preceding kernel has ended and
-// its state before the elements (otherwise its lines are prefetched into L2).
+// its state before the elements (otherwise its lines are prefetched into L2);
+// AHEAD: the next wave's tables are prefetched into L2.
 // THREADS and MINB set how many warps
 // share a patch's shared memory and what their registers are capped at.
-template <class EV, bool KAHAN, bool MULTI, bool EARLY, int THREADS, int MINB>
+template <class EV, bool KAHAN, bool MULTI, bool EARLY, bool AHEAD, int THREADS, int MINB>
 __global__ void __launch_bounds__(THREADS, MINB)
     k_patch_step(const __grid_constant__ PatchArgs pa, const __grid_constant__ MatParams mp,
                  const __grid_constant__ GroupArgs ps) {
@@ -388,6 +389,23 @@ __global__ void __launch_bounds__(THREADS, MINB)
       prefetch_l2_line(pa.v + node * D);
       prefetch_l2_line(pa.mass + node);
     }
+  }
+  // the lists and element tables of the block that follows this one on its
+  // SM, from DRAM into L2
+  constexpr int kWave = (int)kPatchSms * MINB;
+  if (AHEAD && threadIdx.x == 32 && blockIdx.x + kWave < pa.npatch) {
+    const PatchHead hn = pa.head[blockIdx.x + kWave];
+    auto fetch = [](const void *lo, const void *hi) {
+      const uint64_t a = (uint64_t)__cvta_generic_to_global(lo) & ~(uint64_t)15;
+      const uint64_t z = ((uint64_t)__cvta_generic_to_global(hi) + 15) & ~(uint64_t)15;
+      if (z > a)
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a), "r"((unsigned)(z - a))
+                     : "memory");
+    };
+    fetch(pa.nodes + hn.node0, pa.nodes + hn.node0 + hn.n_local);
+    fetch(pa.own + hn.own0, pa.own + hn.own0 + hn.n_own);
+    const char *cn = static_cast<const char *>(pa.tab) + (int64_t)hn.chunk0 * Chunk::kBytes;
+    fetch(cn, cn + (int64_t)((hn.n_elem + 31) >> 5) * Chunk::kBytes);
   }
   const MatParams mph = (ps.mtab && h.mat >= 0) ? ps.mtab[h.mat] : mp;
   const double dt = pa.inst_dt ? pa.inst_dt[h.inst] : pa.dt;

@@ -56,6 +56,7 @@ cudaError_t launch_tet(const PatchArgs &pa, const MatParams &mp, const GroupArgs
                        cudaStream_t s) {
   if (pa.npatch <= kPatchSms && pa.max_own <= 27)
     return launch_patch<EV, true, true, 256, 1>(pa, mp, ps, pdl, s);
+  if (pa.ahead) return launch_patch<EV, true, false, 256, 3, true>(pa, mp, ps, pdl, s);
   return launch_patch<EV, true, false, 256, 3>(pa, mp, ps, pdl, s);
 }
 // triangles: with one patch per SM the state first and all points of two

@@ -1234,6 +1234,11 @@ int finish_patches(akb_model *m, PatchTask &task) {
   pa.tab = base + o_tab;
   pa.e_count = m->E;
   pa.nq = m->nq;
+  // beyond L2 (126 MB): the tables of the next wave of patches are prefetched
+  // (us per step, without / with: batch of 64 cubes, mixed, 148 / 137, FP64 242 /
+  // 223; 1.3 M tetrahedra, FP64, 73.7 / 72.8; mixed, whose 104 MB stay in L2,
+  // 45.9 / 47.6)
+  pa.ahead = (size_t)n * (2 * sizeof(uint16_t) * plan.NNP + t.rows * t.value) > (size_t)126 << 20;
   char *dlocal = nullptr;
   AKB_CUDA(cudaMallocAsync((void **)&dlocal, std::max<size_t>(local.size(), 16), s));
   cudaError_t e = cudaMemcpyAsync(dlocal, local.data(), local.size(), cudaMemcpyHostToDevice, s);

@@ -94,6 +94,7 @@ constexpr int64_t kPatchSms = 148;
 
 struct PatchArgs {
   int64_t npatch = 0;
+  bool ahead = false;  // the plan is larger than L2
   int max_own = 0;  // owned nodes of a patch at most
   const PatchHead *head = nullptr;
   const int32_t *nodes = nullptr;

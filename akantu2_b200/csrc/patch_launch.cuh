@@ -8,10 +8,10 @@
 
 namespace akb {
 
-template <class EV, bool KAHAN, bool MULTI, bool EARLY, int THREADS, int MINB>
-cudaError_t launch_patch(const PatchArgs &pa, const MatParams &mp, const GroupArgs &ps, bool pdl,
+template <class EV, bool KAHAN, bool MULTI, bool EARLY, bool AHEAD, int THREADS, int MINB>
+cudaError_t launch_patch_kernel(const PatchArgs &pa, const MatParams &mp, const GroupArgs &ps, bool pdl,
                          cudaStream_t s) {
-  auto kern = k_patch_step<EV, KAHAN, MULTI, EARLY, THREADS, MINB>;
+  auto kern = k_patch_step<EV, KAHAN, MULTI, EARLY, AHEAD, THREADS, MINB>;
   // shared memory above 48 KB is allowed once per kernel and device (a
   // host-side attribute of the current device, no stream work)
   static std::atomic<unsigned long long> opted{0ull};
@@ -32,11 +32,13 @@ cudaError_t launch_patch(const PatchArgs &pa, const MatParams &mp, const GroupAr
                           smem, s, pa, mp, ps);
 }
 
-template <class EV, bool KAHAN, bool EARLY, int THREADS, int MINB>
+template <class EV, bool KAHAN, bool EARLY, int THREADS, int MINB, bool AHEAD = false>
 cudaError_t launch_patch(const PatchArgs &pa, const MatParams &mp, const GroupArgs &ps, bool pdl,
                          cudaStream_t s) {
-  return pa.multi ? launch_patch<EV, KAHAN, true, EARLY, THREADS, MINB>(pa, mp, ps, pdl, s)
-                  : launch_patch<EV, KAHAN, false, EARLY, THREADS, MINB>(pa, mp, ps, pdl, s);
+  return pa.multi
+             ? launch_patch_kernel<EV, KAHAN, true, EARLY, AHEAD, THREADS, MINB>(pa, mp, ps, pdl, s)
+             : launch_patch_kernel<EV, KAHAN, false, EARLY, AHEAD, THREADS, MINB>(pa, mp, ps, pdl,
+                                                                                 s);
 }
 
 }  // namespace akb

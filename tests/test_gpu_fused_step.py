@@ -195,3 +195,12 @@ def test_fused_heated_plastic_triangles():
     for m in models:
         m.solveStep(105)
     _same(models)
+
+
+@pytest.mark.parametrize("precision,cells", [("fp64", (57, 59, 58)), ("mixed", (67, 69, 68))])
+def test_fused_step_whose_tables_are_larger_than_l2(precision, cells):
+    """patches that prefetch the next wave's tables, up to the last one"""
+    models = _pair(_box("_tetrahedron_4", *cells), [UNIT_NEOHOOKEAN], precision)
+    for m in models:
+        m.solveStep(5)
+    _same(models)
