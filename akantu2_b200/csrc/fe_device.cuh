@@ -217,13 +217,15 @@ __device__ __forceinline__ void plastic_update(double lambda, double mu, double 
   for (int k = 1; k < 9; ++k) ss = ss + dev[k] * dev[k];
   const double eff = sqrt(3. / 2. * ss);
   const bool yield = (eff - iso_cur - sigma_y) > 0;
-  const double dp = yield ? (eff - sigma_y - iso_prev) / (3 * mu + h) : 0.;
-  *iso = iso_prev + h * dp;
-  const double nrm = sqrt(ss);
   const double tol = 1e2 * 2.220446049250313080847e-16;  // Math::tolerance
+  double dp = 0.;
 #pragma unroll
   for (int k = 0; k < DD; ++k) deps[k] = 0.;
-  if (fabs(eff) > nrm * tol) {
+  // the divisions and the second root only where the point yields: elsewhere
+  // dp is 0 and every component of deps is 0 (or -0)
+  if (yield) dp = (eff - sigma_y - iso_prev) / (3 * mu + h);
+  *iso = iso_prev + h * dp;
+  if (yield && fabs(eff) > sqrt(ss) * tol) {
 #pragma unroll
     for (int j = 0; j < D; ++j)
 #pragma unroll
