@@ -1102,6 +1102,69 @@ template <class T> __device__ __forceinline__ void iwht8(T (*v)[3]) {
       }
 }
 
+// ln(1 + x) and 1 / (1 + x) of the sum-factorised FP64 kernel, the FP64 pipe
+// being what bounds it.  For |x| <= 1/32 (x is the volume change of a point)
+// ln by its Taylor series to x^12 (the next term is 2^-63 of the first), even
+// and odd coefficients apart for half the chain, and the reciprocal from the
+// geometric series to x^3 (off by x^4 <= 2^-20) and one third-order correction
+// y (1 + e + e^2) (off by e^3 <= 2^-60): 18 operations.
+__device__ __forceinline__ void log1p_and_reciprocal(double x, double *ln, double *r) {
+  const double d = op_add(1., x);
+  if (fabs(x) <= 0.03125) {
+    const double x2 = op_mul(x, x);
+    double ev = -1. / 12., od = 1. / 11.;
+    ev = op_fma(ev, x2, -1. / 10.);
+    od = op_fma(od, x2, 1. / 9.);
+    ev = op_fma(ev, x2, -1. / 8.);
+    od = op_fma(od, x2, 1. / 7.);
+    ev = op_fma(ev, x2, -1. / 6.);
+    od = op_fma(od, x2, 1. / 5.);
+    ev = op_fma(ev, x2, -1. / 4.);
+    od = op_fma(od, x2, 1. / 3.);
+    ev = op_fma(ev, x2, -1. / 2.);
+    *ln = op_fma(op_fma(od, x, ev), x2, x);
+    const double y = op_add(op_fma(op_add(1., -x), x2, 1.), -x);
+    const double e = op_fma(-d, y, 1.);
+    *r = op_fma(y, op_fma(e, e, e), y);
+  } else {
+    *ln = log1p(x);
+    *r = 1. / d;
+  }
+}
+
+// neohookean_piola of weight 1 for the sum-factorised FP64 kernel: the same
+// tensor by the cofactor expansion of neohookean_piola_x2 (82 instead of about
+// 150 FP64 operations a point)
+__device__ __forceinline__ void neohookean_piola_cof(double lambda, double mu, const double *g,
+                                                     double *P) {
+  double adj[9];
+#pragma unroll
+  for (int j = 0; j < 3; ++j)
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      // adj(H)(i, j) = cofactor (j, i) of H
+      const int j1 = (j + 1) % 3, j2 = (j + 2) % 3, i1 = (i + 1) % 3, i2 = (i + 2) % 3;
+      adj[i + 3 * j] =
+          op_fma(g[j1 + 3 * i1], g[j2 + 3 * i2], -op_mul(g[j1 + 3 * i2], g[j2 + 3 * i1]));
+    }
+  const double t = op_add(op_add(g[0], g[4]), g[8]);
+  const double i2 = op_add(op_add(adj[0], adj[4]), adj[8]);
+  const double detH = op_fma(g[6], adj[2], op_fma(g[3], adj[1], op_mul(g[0], adj[0])));
+  const double dm1 = op_add(op_add(t, i2), detH);
+  double lnJ, rdet;
+  log1p_and_reciprocal(dm1, &lnJ, &rdet);
+  const double c = op_mul(op_fma(lambda, lnJ, -mu), rdet);
+  const double a0 = op_fma(c, t, op_mul(op_fma(mu, dm1, op_mul(lambda, lnJ)), rdet));
+#pragma unroll
+  for (int j = 0; j < 3; ++j)
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const double p =
+          op_fma(c, op_add(adj[j + 3 * i], -g[j + 3 * i]), op_mul(mu, g[i + 3 * j]));
+      P[i + 3 * j] = i == j ? op_add(p, a0) : p;
+    }
+}
+
 // weighted flux P of one point for the sum-factorised kernels: r_a = P . dN_a/dx
 // (FP32 element math on the mixed path, FP64 on the fast FP64 path: the
 // same formulas, first Piola-Kirchhoff stress in the displacement gradient)
@@ -1114,6 +1177,8 @@ __device__ __forceinline__ void mixed_flux(const T *g, T w, const MatParams &mp,
       T S[D * D];
       finite_pk2<D, T>(mp, g, S);
       first_piola<D, T>(g, S, w, P);
+    } else if constexpr (D == 3 && std::is_same<T, double>::value) {
+      neohookean_piola_cof(mp.lambda, mp.mu, g, P);
     } else {
       neohookean_piola<D, T>((T)mp.lambda, (T)mp.mu, g, w, P);
     }
@@ -1282,6 +1347,96 @@ __device__ __forceinline__ void hex8sf_forces(T (*wx)[3], T (*wu)[3], T *Ja, T r
   iwht8(A);
 }
 
+// hex8sf_forces of a parallelepiped in FP64, from its adjugate and 1/det: the
+// two points of a pair (q and q + 1, at xi = -+1/sqrt(3)) share what does not
+// depend on xi, 1/det goes into the displacement modes once, and their fluxes
+// are projected as sum and difference, which is what the modes accumulate:
+// 177 operations a pair beside the law instead of 270.  PU pairs per unrolled
+// iteration.  The FP64 pipe is the bound (ncu, neohookean, 64^3: 48 % of its
+// peak, then the gathers' latency at 12 resident warps).  Neohookean, with
+// neohookean_piola_cof, us per step before / after: 30^3 16.4 / 14.3, 72^3 108 /
+// 96, 128^3 535 / 471; plastic, 48^3: 101 / 90.  Elastic, bound by memory, keeps
+// hex8sf_forces (72^3 86.5, here 89.2); 4 blocks of 128 registers spill (72^3
+// 104), with the adjugate in shared memory too (104).
+template <int LAW, int PU>
+__device__ __forceinline__ void hex8sf_forces_pairs(double (*wu)[3], const double *Ja,
+                                                    double rdet, const MatParams &mpe,
+                                                    const GroupArgs &ps, int64_t e_count,
+                                                    int64_t le, double (*A)[3]) {
+  wht8(wu);
+  constexpr double g1 = 0.577350269189625764509, g2 = 1. / 3.;  // Gauss coordinate, its square
+  const double r1 = op_mul(g1, rdet), r2 = op_mul(g2, rdet);
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    wu[1][c] *= rdet; wu[2][c] *= rdet; wu[4][c] *= rdet;
+    wu[3][c] *= r1; wu[5][c] *= r1; wu[6][c] *= r1; wu[7][c] *= r2;
+  }
+#pragma unroll
+  for (int m = 1; m < 8; ++m)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) A[m][c] = 0.;
+#pragma unroll 1
+  for (int po = 0; po < 4; po += PU)
+#pragma unroll
+  for (int pi = 0; pi < PU; ++pi) {
+    const int q = 2 * (po + pi);
+    const double sy = (q & 2) ? 1. : -1., sz = (q & 4) ? 1. : -1.;
+    // grad u (i, j) = sum_k adj(j, k) du_i/dxi_k of both points; the rows of
+    // the derivative: k = 0 the same at both, k = 1, 2 a sum -+ a difference
+    double ga[9], gb[9];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const double d1 = op_fma(sz, wu[7][i], wu[3][i]), d2 = op_fma(sy, wu[7][i], wu[5][i]);
+      const double p0 = op_fma(sz, d2, op_fma(sy, wu[3][i], wu[1][i]));
+      const double p1 = op_fma(sz, wu[6][i], wu[2][i]), p2 = op_fma(sy, wu[6][i], wu[4][i]);
+      const double a1 = op_add(p1, -d1), a2 = op_add(p2, -d2);
+      const double b1 = op_add(p1, d1), b2 = op_add(p2, d2);
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        const double s = op_mul(Ja[j], p0);
+        ga[i + 3 * j] = op_fma(Ja[j + 6], a2, op_fma(Ja[j + 3], a1, s));
+        gb[i + 3 * j] = op_fma(Ja[j + 6], b2, op_fma(Ja[j + 3], b1, s));
+      }
+    }
+    subtract_eigen<3, double>(ps, e_count, le, q, ga);
+    subtract_eigen<3, double>(ps, e_count, le, q + 1, gb);
+    double Pa[9], Pb[9];
+    mixed_flux<3, LAW, double>(ga, 1., mpe, ps, e_count, le, q, Pa);
+    mixed_flux<3, LAW, double>(gb, 1., mpe, ps, e_count, le, q + 1, Pb);
+    // H(k, m) = sum_J P(k, J) adj(J, m) of the sum S of the two fluxes and of
+    // their difference D
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const double s0 = op_add(Pa[k], Pb[k]), s1 = op_add(Pa[k + 3], Pb[k + 3]),
+                   s2 = op_add(Pa[k + 6], Pb[k + 6]);
+      const double t0 = op_add(Pb[k], -Pa[k]), t1 = op_add(Pb[k + 3], -Pa[k + 3]),
+                   t2 = op_add(Pb[k + 6], -Pa[k + 6]);
+      const double S0 = op_fma(s2, Ja[2], op_fma(s1, Ja[1], op_mul(s0, Ja[0])));
+      const double S1 = op_fma(s2, Ja[5], op_fma(s1, Ja[4], op_mul(s0, Ja[3])));
+      const double S2 = op_fma(s2, Ja[8], op_fma(s1, Ja[7], op_mul(s0, Ja[6])));
+      const double D1 = op_fma(t2, Ja[5], op_fma(t1, Ja[4], op_mul(t0, Ja[3])));
+      const double D2 = op_fma(t2, Ja[8], op_fma(t1, Ja[7], op_mul(t0, Ja[6])));
+      // the sum over the pair of sx H is D, of H is S
+      const double e3 = op_fma(sy, S0, D1), e6 = op_fma(sy, S2, op_mul(sz, S1));
+      A[1][k] = op_add(A[1][k], S0);
+      A[2][k] = op_add(A[2][k], S1);
+      A[4][k] = op_add(A[4][k], S2);
+      A[3][k] = op_add(A[3][k], e3);
+      A[5][k] = op_add(A[5][k], op_fma(sz, S0, D2));
+      A[6][k] = op_add(A[6][k], e6);
+      A[7][k] = op_add(A[7][k], op_fma(sz, e3, op_mul(sy, D2)));
+    }
+  }
+  constexpr double c0 = 1. / 512, c1 = g1 / 512, c2 = g2 / 512;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    A[0][c] = 0.;
+    A[1][c] *= c0; A[2][c] *= c0; A[4][c] *= c0;
+    A[3][c] *= c1; A[5][c] *= c1; A[6][c] *= c1; A[7][c] *= c2;
+  }
+  iwht8(A);
+}
+
 template <int LAW, int QU, bool AFF = false, bool GEO = false, class T = float>
 __device__ __forceinline__ void element_hex8sf(int64_t le, int64_t e_begin, int64_t e_count,
                                                int64_t E, const int32_t *conn,
@@ -1317,7 +1472,10 @@ __device__ __forceinline__ void element_hex8sf(int64_t le, int64_t e_begin, int6
     rdet_a = geo[(int64_t)9 * E + e];
   }
   T A[8][3];
-  hex8sf_forces<LAW, QU, AFF, GEO, T>(wx, wu, Ja, rdet_a, mpe, ps, e_count, le, A);
+  if constexpr (GEO && LAW != LAW_ELASTIC && std::is_same<T, double>::value)
+    hex8sf_forces_pairs<LAW, (QU > 1 ? QU / 2 : 1)>(wu, Ja, rdet_a, mpe, ps, e_count, le, A);
+  else
+    hex8sf_forces<LAW, QU, AFF, GEO, T>(wx, wu, Ja, rdet_a, mpe, ps, e_count, le, A);
 #pragma unroll
   for (int a = 0; a < 8; ++a) store_slot<3>(re, pos[(int64_t)a * E + e], A[lex[a]]);
 }

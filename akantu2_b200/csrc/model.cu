@@ -1717,8 +1717,8 @@ int akb_model_init_full(akb_model *m, int method, int precision) {
       AKB_CUDA(launch_hex8_affine_geometry_fp64(g, m->dgeo64, s));
     }
     // 2 points per iteration, registers capped for 3 blocks per SM: measured
-    // on the 128^3 box, element launch 0.417 ms (neohookean) and 0.299 ms
-    // (elastic) against 0.517 and 0.396 uncapped (2 blocks of 192 registers)
+    // per step, 95.5 us (neohookean, 72^3) and 61.6 us (elastic, 64^3) against
+    // 110.7 and 66.4 uncapped (2 blocks per SM)
     for (auto &gr : m->groups) gr.tune = ElemTuning{128, 2, 3};
     m->pdl = true;
   }

@@ -64,6 +64,30 @@ def test_fp64_fast_register_caps_are_bit_identical():
         assert np.array_equal(runs[0][0], other[0]) and np.array_equal(runs[0][1], other[1])
 
 
+@pytest.mark.parametrize("points", [1, 2, 8])
+@pytest.mark.parametrize("volume", [0.0, 0.031, 0.0312499, 0.0312501, -0.031251, 0.3, -0.3])
+def test_fp64_fast_at_a_volume_change(volume, points):
+    """the neohookean law on both sides of the range of its series (a volume
+    change of 1/32), against the plain FP64 path, to the bar above"""
+    mesh = akb.box_hex8(5)
+    u0 = ((1 + volume) ** (1 / 3) - 1) * mesh.nodes
+    out = []
+    for precision in ("fp64_fast", "fp64"):
+        m = akb.SolidMechanicsModel(mesh)
+        m.addMaterial("neohookean", rho=1.0, E=1.0, nu=0.3)
+        m.initFull(akb._explicit_lumped_mass, precision=precision)
+        if precision == "fp64_fast":
+            m.setLaunchShape("neohookean", 128, points, 256, 1)
+        m.setNodal("displacement", u0)
+        m.setNodal("velocity", sinusoidal_velocity(mesh.nodes, 0.03))
+        m.setTimeStep(0.4 * m.getStableTimeStep())
+        m.solveStep(20)
+        out.append((m.getDisplacement().copy(), m.getInternalForce().copy()))
+        assert m.getStatus() == 0
+    for a, b in zip(*out):
+        assert np.abs(b).max() > 0 and np.abs(a - b).max() <= 1e-12 * np.abs(b).max()
+
+
 def test_fp64_fast_leaves_other_elements_on_the_plain_path():
     """tetrahedra and triangles have no sum-factorised kernel: the fast FP64
     path runs them exactly as the plain one (bit-identical to the oracle)"""
