@@ -1045,8 +1045,14 @@ int reduce_to_host(akb_model *m, const double *x, int64_t n, bool op_min, double
 // points mixed, 6.5 with 121 patches, 7.9 with 64), else the largest.  With more
 // patches than are resident at once the two kernels, which read every point's
 // state once, are faster (512^2 x 2: 111 against 154).
-int patch_nodes(int et, int rule, int precision, int64_t N, int64_t E, int ninst) {
+// The finite-deformation laws of FP64 tetrahedra: up to 50,000 elements.  Past
+// that their FP64 operations (a logarithm each) are the bound, of which the
+// patches evaluate those of the border elements again (us per step, two kernels
+// / fused: 25 k 9.5 / 7.7, 48 k 10.2 / 8.3, 64 k 11.3 / 11.9, 162 k 16.3 / 21.2,
+// 1.3 M 102 / 117; elastic 1.3 M 94 / 74).
+int patch_nodes(int et, int rule, int law, int precision, int64_t N, int64_t E, int ninst) {
   const bool mixed = precision == AKB_PRECISION_MIXED;
+  if (!mixed && law == LAW_NEOHOOKEAN && E > 50000) return 0;
   const double sms = 148.;
   const double planes = std::pow((double)N / ninst, 1. / dim_of(et));
   int best = 0;
@@ -1116,7 +1122,7 @@ size_t patch_capacity_bytes(const PatchCaps &c, int64_t N, int nn, const PatchTa
 int64_t patch_bytes(int et, int rule, int law, int precision, int64_t N, int64_t E, int ninst) {
   const PatchTables t = patch_tables(et, law, precision, et == AKB_TRIANGLE_6 && rule ? 6 : 3);
   if (t.rows == 0 || N == 0 || E == 0) return 0;
-  const int own = patch_nodes(et, rule, precision, N, E, ninst);
+  const int own = patch_nodes(et, rule, law, precision, N, E, ninst);
   if (own == 0) return 0;
   const PatchCaps c = patch_caps(dim_of(et), N, E, ninst, own);
   return (int64_t)patch_capacity_bytes(c, N, nodes_per_element(et), t);
@@ -1157,7 +1163,7 @@ void start_patches(akb_model *m, const std::vector<int32_t> &conn_soa,
   for (auto &mt : m->mats)
     if (mt.c33) return;
   PatchMesh &pm = task.mesh;
-  pm.max_own = patch_nodes(m->et, m->rule, m->precision, m->N, m->E, m->ninst);
+  pm.max_own = patch_nodes(m->et, m->rule, gr.law, m->precision, m->N, m->E, m->ninst);
   if (pm.max_own == 0 || patch_tables(m->et, gr.law, m->precision, m->nq).rows == 0) return;
   pm.D = m->dim;
   pm.NN = m->nn;
