@@ -26,6 +26,13 @@ template <class... KArgs, class... Args>
 inline cudaError_t launch_step_smem(bool pdl, void (*kernel)(KArgs...), unsigned grid,
                                     unsigned block, size_t smem, cudaStream_t s,
                                     Args... args) {
+  if (launch_probe) {
+    int resident = 0;
+    const cudaError_t e =
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kernel, (int)block, smem);
+    launch_probe->waves += (double)grid / (148. * std::max(resident, 1));
+    return e;
+  }
   if (!pdl) {
     kernel<<<grid, block, smem, s>>>(args...);
     return cudaGetLastError();

@@ -28,15 +28,16 @@ constexpr int kMaxNN = 8;
 // with the programmatic-serialization attribute may start while the kernel
 // before it on the stream finishes; it waits here (griddepcontrol.wait)
 // until that kernel has completed and its writes are visible, before it
-// reads anything.  Kernels of at most kEarlyTriggerBlocks blocks (one wave)
-// let the next kernel launch at once; larger grids let it launch when they
-// end, so that its waiting blocks do not hold SM slots their later waves
-// need.  Without the attribute both instructions do nothing.
-constexpr unsigned kEarlyTriggerBlocks = 1184;  // 148 SMs x 8
-__device__ __forceinline__ void pdl_begin() {
+// reads anything.  With trigger it then lets the next kernel launch at once;
+// without, when it ends.  A step triggers where the blocks of its kernels are
+// resident all together: a next kernel that finds room for a part of its
+// blocks only starts late with the others (us per step, trigger / none / no
+// dependent launch: FP64 tet4 94 k 11.6 / - / 12.1, 105 k 23.1 / - / 13.1; hex8
+// 47 k 11.4 / - / 11.5, 64 k 16.4 / - / 13.2).  Without the attribute both
+// instructions do nothing.
+__device__ __forceinline__ void pdl_begin(bool trigger = true) {
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  if (gridDim.x * gridDim.y <= kEarlyTriggerBlocks)
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (trigger) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
 // L2 prefetch (cp.async.bulk.prefetch.L2: nothing reaches the SM) of the
@@ -124,6 +125,7 @@ struct GroupArgs {
   double *c33;               // [q][ne] plane-stress neohookean out-of-plane stretch
                              // (updated in place by every stress evaluation), or null
   int update_energy;         // 1 inside solveStep (afterSolveStep), 0 otherwise
+  int trigger;               // the next kernel may launch at once (pdl_begin)
   // eigen gradient of the displacement [q][d*d][ne] (double), subtracted from
   // the gradient before the law (material.cc:147), or null when zero
   const double *eig;
@@ -486,7 +488,7 @@ __global__ void k_predict(int64_t N, const uint8_t *__restrict__ blocked,
                           const double *__restrict__ a, double dt,
                           const int32_t *__restrict__ node_inst,
                           const double *__restrict__ inst_dt, double *__restrict__ u_pred) {
-  pdl_begin();
+  pdl_begin(gridDim.x <= 1184);  // one wave
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N * D) return;
   const int64_t node = i / D;
@@ -862,7 +864,7 @@ __global__ void __launch_bounds__(BLOCK, MINB)
                                  MatParams mp, GroupArgs ps, RT *__restrict__ re, int64_t pf) {
   (void)pf;
   __shared__ T s_r[NN * D * BLOCK];
-  pdl_begin();
+  pdl_begin(ps.trigger);
   const int64_t le = (int64_t)blockIdx.x * BLOCK + threadIdx.x;
   if (le >= e_count || !element_active(ps, le)) return;
   if (!element_indices_ok<NN>(ps, conn, pos, E, e_begin + le)) return;
@@ -941,7 +943,7 @@ __global__ void __launch_bounds__(BLOCK, MINB)
                         RT *__restrict__ re, int64_t pf) {
   if constexpr (PF)
     prefetch_pe_rows<D, NN, NQ, LAW, T>(pf, e_begin, e_count, E, conn, pos, B, wJ, ps);
-  pdl_begin();
+  pdl_begin(ps.trigger);
   const int64_t le = (int64_t)blockIdx.x * BLOCK + threadIdx.x;
   if (le >= e_count || !element_active(ps, le)) return;
   if (!element_indices_ok<NN>(ps, conn, pos, E, e_begin + le)) return;
@@ -960,7 +962,7 @@ __global__ void __launch_bounds__(BLOCK, MINB)
                         RT *__restrict__ re, int64_t pf) {
   if constexpr (PF)
     prefetch_pe_rows<D, NN, NQ, LAW, T>(pf, e_begin, e_count, E, conn, pos, nullptr, nullptr, ps);
-  pdl_begin();
+  pdl_begin(ps.trigger);
   const int64_t le = (int64_t)blockIdx.x * BLOCK + threadIdx.x;
   if (le >= e_count || !element_active(ps, le)) return;
   if (!element_indices_ok<NN>(ps, conn, pos, E, e_begin + le)) return;
@@ -1049,7 +1051,7 @@ __global__ void __launch_bounds__(BLOCK)
                          const double *__restrict__ X, QuadTable tab,
                          const double *__restrict__ u, MatParams mp, GroupArgs ps,
                          float *__restrict__ re) {
-  pdl_begin();
+  pdl_begin(ps.trigger);
   const int64_t le = (int64_t)blockIdx.x * BLOCK + threadIdx.x;
   if (le >= e_count || !element_active(ps, le)) return;
   if (!element_indices_ok<NN>(ps, conn, pos, E, e_begin + le)) return;
@@ -1770,7 +1772,7 @@ __global__ void __launch_bounds__(BLOCK, MINB)
                                const double *__restrict__ u, MatParams mp, GroupArgs ps,
                                float *__restrict__ re, int64_t pf) {
   if constexpr (PF) prefetch_hex8_rows<GEO>(pf, e_begin, e_count, E, conn, pos, geo);
-  pdl_begin();
+  pdl_begin(ps.trigger);
   const int64_t le = (int64_t)blockIdx.x * BLOCK + threadIdx.x;
   if (le >= e_count || !element_active(ps, le)) return;
   if (!element_indices_ok<8>(ps, conn, pos, E, e_begin + le)) return;
@@ -1787,7 +1789,7 @@ __global__ void __launch_bounds__(BLOCK, MINB)
                             const double *__restrict__ X, const T *__restrict__ geo,
                             const double *__restrict__ u, MatParams mp, GroupArgs ps,
                             T *__restrict__ re) {
-  pdl_begin();
+  pdl_begin(ps.trigger);
   const int64_t le = (int64_t)blockIdx.x * BLOCK + threadIdx.x;
   if (le >= e_count || !element_active(ps, le)) return;
   if (!element_indices_ok<8>(ps, conn, pos, E, e_begin + le)) return;
@@ -1813,7 +1815,7 @@ __global__ void __launch_bounds__(32 * NQ)
                         const T *__restrict__ B, const T *__restrict__ wJ,
                         const double *__restrict__ u, MatParams mp, GroupArgs ps,
                         RT *__restrict__ re) {
-  pdl_begin();
+  pdl_begin(ps.trigger);
   constexpr int ND = NN * D;
   constexpr bool REL = !std::is_same<T, double>::value;  // relative gather in FP32
   constexpr int CH = (ND + NQ - 1) / NQ;  // components reduced per round and thread
@@ -1996,7 +1998,7 @@ __global__ void __launch_bounds__(32 * NQ)
       for (int c = 0; c < ND; ++c) copy_async_8(&red[q][c][lane], Bq + (int64_t)c * E);
     }
   }
-  pdl_begin();
+  pdl_begin(ps.trigger);
   const bool active = le < e_count && element_active(ps, le) &&
                       element_indices_ok<NN>(ps, conn, pos, E, e_begin + le);
   if (active) {
@@ -2043,9 +2045,10 @@ __global__ void __launch_bounds__(32 * NQ)
 //        NU_FINT      store the internal force (else it is gathered again on
 //                     request by a flags == NU_FINT launch)
 //        NU_FEXT_ZERO the external force is identically zero: not read
+//        NU_TRIGGER   the next kernel may launch at once (pdl_begin)
 //                     (0 + f_ext + f_int == f_int)
 // KAHAN selects a compensated FP64 sum (mixed path).
-enum { NU_CORRECT = 1, NU_PREDICT = 2, NU_FINT = 4, NU_FEXT_ZERO = 8 };
+enum { NU_CORRECT = 1, NU_PREDICT = 2, NU_FINT = 4, NU_FEXT_ZERO = 8, NU_TRIGGER = 16 };
 
 // one slot into the internal-force sum, sign -1 (dof_manager.cc:65-120),
 // optionally compensated
@@ -2371,7 +2374,7 @@ __global__ void __launch_bounds__(1024) k_node_update(int64_t N, const int32_t *
                               double dt, const int32_t *__restrict__ node_inst,
                               const double *__restrict__ inst_dt, int flags,
                               unsigned int *__restrict__ status, const PrescArgs pr) {
-  pdl_begin();
+  pdl_begin(flags & NU_TRIGGER);
   if (RAMP && blockIdx.x == gridDim.x - 1) return prescribe_block(pr, u_next, true);
   const int64_t i = node_block<RAMP>() * blockDim.x + threadIdx.x;
   if (i >= N || !node_range_ok(ptr, N, i, status)) return;
@@ -2405,7 +2408,7 @@ __global__ void __launch_bounds__(1024)
     st.m = mass[i];
     st.bl = blocked[i];
   }
-  pdl_begin();
+  pdl_begin(flags & NU_TRIGGER);
   if (RAMP && blockIdx.x == gridDim.x - 1) return prescribe_block(pr, u_next, true);
   if (!in || !node_range_ok(ptr, N, i, status)) return;
   if (flags & NU_CORRECT) load_node_state<D>(st, i, fext, a, v, u, flags);
@@ -2436,7 +2439,7 @@ __global__ void __launch_bounds__(1024) k_node_update_retire(int64_t N, const in
                                      const int64_t *__restrict__ inst_end,
                                      const int64_t *__restrict__ step, int flags,
                                      unsigned int *__restrict__ status) {
-  pdl_begin();
+  pdl_begin(flags & NU_TRIGGER);
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N || !node_range_ok(ptr, N, i, status)) return;
   // a batch of one instance has no node -> instance table
@@ -2485,7 +2488,7 @@ __global__ void __launch_bounds__(BLOCK)
                          const int32_t *__restrict__ node_inst,
                          const double *__restrict__ inst_dt, int flags,
                          unsigned int *__restrict__ status, const PrescArgs pr) {
-  pdl_begin();
+  pdl_begin(flags & NU_TRIGGER);
   if (RAMP && blockIdx.x == gridDim.x - 1) return prescribe_block(pr, u_next, true);
   using V = typename SlotVec<D, RT>::type;
   constexpr int WPS = SlotVec<D, RT>::per_slot;  // vectors per slot

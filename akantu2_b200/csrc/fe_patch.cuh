@@ -303,8 +303,12 @@ __global__ void __launch_bounds__(THREADS, MINB)
   using Chunk = typename EV::Chunk;
   constexpr int D = EV::D, W = THREADS / 32, U = EV::kIds;
   extern __shared__ __align__(16) char patch_sm[];
+  // one kernel a step: it lets the next one launch at once up to 8 patches per
+  // SM (only where two steps' patches are resident together, 3 k tetrahedra
+  // 3.15 against 3.68 us per step, 160 k 12.3 against 12.8)
+  const bool trigger = gridDim.x <= 8 * kPatchSms;
   if (pa.presc.count && blockIdx.x == gridDim.x - 1) {
-    pdl_begin();
+    pdl_begin(trigger);
     return prescribe_block(pa.presc, pa.u_next, true);
   }
   const PatchHead h = pa.head[blockIdx.x];
@@ -347,7 +351,7 @@ __global__ void __launch_bounds__(THREADS, MINB)
       st0.bl = pa.blocked[o0.node];
     }
   }
-  pdl_begin();
+  pdl_begin(trigger);
   // a stopped instance keeps its state (k_node_update_retire)
   if (pa.inst_end && *pa.step >= pa.inst_end[h.inst]) {
     copy_async_wait();

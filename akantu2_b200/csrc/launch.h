@@ -45,6 +45,13 @@ struct ElemTuning {
 // evaluated as packed FP32 pairs (2, 4 or 8 points per iteration)
 constexpr int kPackedPoints = 256;
 
+// While a thread has one, its step kernels are not launched: the probe counts
+// the waves of resident blocks that their grids fill.
+struct LaunchProbe {
+  double waves = 0.;
+};
+inline thread_local LaunchProbe *launch_probe = nullptr;
+
 // device view of the mesh, internal element order
 struct DevGeom {
   int et, D, NN, NQ;

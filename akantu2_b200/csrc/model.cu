@@ -267,6 +267,12 @@ struct akb_model {
     int64_t steps = 0;
   };
   std::vector<StepGraph> graphs;
+  // after a change of what the launches are made from
+  void drop_graphs() {
+    for (auto &g : graphs) cudaGraphExecDestroy(g.exec);
+    graphs.clear();
+    trigger = -1;
+  }
   int64_t graph_steps = 100;  // steps per captured graph (even; 0 disables)
   int stream_priority = 0;    // of the model's stream, when priority_set
   bool priority_set = false;
@@ -290,6 +296,9 @@ struct akb_model {
   // step kernels launched with programmatic stream serialization: each one
   // is scheduled while its predecessor drains and waits for it on the device
   bool pdl = false;
+  // whether its kernels let the next one launch at once: their blocks are all
+  // resident together (-1: not looked at since the launches last changed)
+  int trigger = -1;
   // fused step (patch.h): one launch per step over patches of nodes, when the
   // model has a plan for it and no kernel of the two-kernel step was chosen
   PatchArgs patch;
@@ -359,7 +368,7 @@ struct akb_model {
   ~akb_model() {
     if (aio.in) cudaStreamSynchronize(aio.in);
     if (aio.out) cudaStreamSynchronize(aio.out);
-    for (auto &g : graphs) cudaGraphExecDestroy(g.exec);
+    drop_graphs();
     for (void *p : allocs) cudaFreeAsync(p, stream);
     for (int k = 0; k < AsyncIO::kIn; ++k)
       for (cudaEvent_t e : {aio.in_ready[k], aio.in_used[k]})
@@ -537,6 +546,7 @@ GroupArgs group_args(akb_model *m, const Group &mt, bool in_step) {
   ps.nb_nodes = m->N;
   ps.nb_slots = m->E * m->nn;
   ps.status = m->dstatus;
+  ps.trigger = in_step && m->trigger > 0;
   if (m->dinst_end) {
     ps.einst = m->delem_inst + mt.e_begin;
     ps.inst_end = m->dinst_end;
@@ -609,8 +619,7 @@ bool thermal_steady(const akb_model *m) {
 
 // elemental forces at the predicted displacement (inside a step) or at the
 // model's displacement (standalone assembly)
-int element_forces(akb_model *m, bool in_step) {
-  AKB_TRY(thermal_eval(m, in_step));
+int launch_forces(akb_model *m, bool in_step) {
   DevGeom g = m->geom();
   const double *u = in_step ? m->u_pred() : m->u();
   for (auto &gr : m->groups) {
@@ -629,6 +638,11 @@ int element_forces(akb_model *m, bool in_step) {
     if (e != cudaSuccess) return fail(AKB_ECUDA, std::string("element forces: ") + cudaGetErrorString(e));
   }
   return AKB_OK;
+}
+
+int element_forces(akb_model *m, bool in_step) {
+  AKB_TRY(thermal_eval(m, in_step));
+  return launch_forces(m, in_step);
 }
 
 PrescArgs presc_args(const akb_model *m) {
@@ -668,17 +682,17 @@ int predict(akb_model *m) {
 // u_pred into the other buffer (which held the displacement of the previous
 // step); the internal force is only gathered when asked for (ensure_fint).
 // Standalone (correct == false): the internal force only.
-int node_update(akb_model *m, bool correct) {
+int launch_nodes(akb_model *m, bool correct) {
   DevGeom g = m->geom();
   cudaError_t e;
   int flags = correct ? (NU_CORRECT | NU_PREDICT) : NU_FINT;
   if (correct && m->fext_zero) flags |= NU_FEXT_ZERO;
+  if (correct && m->trigger > 0) flags |= NU_TRIGGER;
   const double *u = m->u_pred();
   double *u_next = m->u();
   // the next step's prescribed dofs are written by the same launch (a batch
   // with stopping instances has an update kernel of its own)
-  const bool with_ramp = correct && !m->dinst_end;
-  if (with_ramp) g.presc = presc_args(m);
+  if (correct && !m->dinst_end) g.presc = presc_args(m);
   if (m->precision == AKB_PRECISION_MIXED)
     e = launch_node_update_mixed(g, (const float *)m->dre, m->dfext, m->dmass, m->dblocked,
                                  m->dfint, m->da, m->dv, u, u_next, m->dt, flags, m->dstatus,
@@ -688,10 +702,27 @@ int node_update(akb_model *m, bool correct) {
                                 m->dfint, m->da, m->dv, u, u_next, m->dt, flags, m->dstatus,
                                 m->node_block, m->node_form, m->stream);
   if (e != cudaSuccess) return fail(AKB_ECUDA, std::string("node update: ") + cudaGetErrorString(e));
-  if (with_ramp) m->presc_ahead = m->presc_count > 0 || m->presc_ahead;
-  else if (correct) AKB_TRY(prescribe(m, u_next, true));
+  return AKB_OK;
+}
+
+int node_update(akb_model *m, bool correct) {
+  AKB_TRY(launch_nodes(m, correct));
+  if (correct && !m->dinst_end) m->presc_ahead = m->presc_count > 0 || m->presc_ahead;
+  else if (correct) AKB_TRY(prescribe(m, m->u(), true));
   m->fint_valid = !correct;
   return AKB_OK;
+}
+
+// whether the two kernels' blocks are resident all together (pdl_begin)
+int find_trigger(akb_model *m) {
+  if (m->trigger >= 0) return AKB_OK;
+  LaunchProbe probe;
+  launch_probe = &probe;
+  int rc = launch_forces(m, true);
+  if (rc == AKB_OK) rc = launch_nodes(m, true);
+  launch_probe = nullptr;
+  if (rc == AKB_OK) m->trigger = probe.waves <= 1.;
+  return rc;
 }
 
 // the internal force of the last force evaluation, gathered again from the
@@ -767,6 +798,7 @@ int one_step(akb_model *m, bool any_plastic, bool last = true, cudaEvent_t e1 = 
     AKB_TRY(patch_step(m, last));
     if (e2) AKB_CUDA(cudaEventRecord(e2, m->stream));
   } else {
+    AKB_TRY(find_trigger(m));
     AKB_TRY(element_forces(m, true));
     if (e2) AKB_CUDA(cudaEventRecord(e2, m->stream));
     AKB_TRY(node_update(m, true));
@@ -992,8 +1024,7 @@ int fill_group_eigen(akb_model *m, int gi) {
   const int64_t ne = gr.e_count, rows = (int64_t)m->nq * dd;
   if (!gr.eig) {
     AKB_TRY(m->alloc(&gr.eig, sizeof(double) * std::max<int64_t>(rows * ne, 1)));
-    for (auto &g : m->graphs) cudaGraphExecDestroy(g.exec);
-    m->graphs.clear();
+    m->drop_graphs();
   }
   std::vector<double> h((size_t)(rows * ne), 0.);
   for (auto &mt : m->mats) {
@@ -1577,14 +1608,18 @@ int akb_model_init_full(akb_model *m, int method, int precision) {
     }
     for (int64_t e = 0; e < E; ++e) m->perm[start[m->mat_user[e]]++] = e;
   }
-  // dependent launches: measured on B200 from 3k to 2M elements, 4-15 %
-  // shorter steps on meshes below ~50k elements and even above, except FP64
-  // hexahedra (the per-point kernel), whose 16^3 and 32^3 steps were slower;
-  // elastic ones of one wave of its blocks gain (us per step, plain /
-  // dependent: 8^3 7.75 / 7.48, 12^3 8.41 / 7.60, 20^3 9.66 / 9.27; 24^3 12.06
-  // / 12.56)
-  m->pdl = !(m->et == AKB_HEXAHEDRON_8 && precision == AKB_PRECISION_FP64) ||
-           (E <= 148 * 2 * 32 && m->groups.size() == 1 && m->groups[0].law == LAW_ELASTIC);
+  // dependent launches: shorter steps at every size (us per step, plain /
+  // dependent: tet4 25 k, FP64, 9.0 / 8.5, 384 k 29.6 / 29.2; hex8 64 k, mixed, 13.1
+  // / 12.7; FP64 hexahedra, elastic 6^3 7.6 / 7.4, 24^3 11.9 / 11.3, 44^3 58.1 /
+  // 58.0, neohookean 16^3 11.1 / 10.6, 28^3 21.7 / 21.0) but for FP64 hexahedra of
+  // the other laws with one to four of their blocks per SM (neohookean 20^3 13.2 /
+  // 13.8, 24^3 16.1 / 16.8), and unmeasured for mixtures of laws
+  m->pdl = true;
+  if (m->et == AKB_HEXAHEDRON_8 && precision == AKB_PRECISION_FP64) {
+    const int law = m->groups.size() == 1 ? m->groups[0].law : LAW_PLASTIC;
+    m->pdl = law == LAW_ELASTIC ||
+             (law == LAW_NEOHOOKEAN && (E <= 148 * 32 || E > 148 * 4 * 32));
+  }
   std::vector<int64_t> iperm(E);  // user element -> internal element
   for (int64_t ie = 0; ie < E; ++ie) iperm[m->perm[ie]] = ie;
   std::vector<int32_t> conn_soa((size_t)nn * E);
@@ -1938,8 +1973,7 @@ int akb_batch_set_instance_steps(akb_model *m, const int64_t *steps) {
                              m->stream));
     AKB_CUDA(cudaStreamSynchronize(m->stream));
     // captured graphs and the persistent kernel know no stopping instances
-    for (auto &x : m->graphs) cudaGraphExecDestroy(x.exec);
-    m->graphs.clear();
+    m->drop_graphs();
     m->inst_end.assign(ni, std::numeric_limits<int64_t>::max());
   }
   for (int k = 0; k < ni; ++k)
@@ -2386,8 +2420,7 @@ int akb_model_set_prescribed_velocity_ramp(akb_model *m, const int64_t *dofs, in
     if (dofs[k] < 0 || dofs[k] >= nd) return fail(AKB_EINVAL, "dof index out of range");
   cudaStream_t s = m->stream;
   AKB_CUDA(cudaStreamSynchronize(s));
-  for (auto &x : m->graphs) cudaGraphExecDestroy(x.exec);
-  m->graphs.clear();
+  m->drop_graphs();
   m->presc_count = 0;
   if (count == 0 && m->presc_dofs.empty()) return AKB_OK;
   // the dofs are blocked from now on, and marked as prescribed
@@ -2646,7 +2679,10 @@ int akb_model_autotune(akb_model *m, int repeats) {
   // dependent launch on or off: whole steps (element forces of every group,
   // node update into the scratch state) in the chosen shapes
   if (rc == AKB_OK) {
-    const int flags = NU_CORRECT | NU_PREDICT | (m->fext_zero ? NU_FEXT_ZERO : 0);
+    m->trigger = -1;
+    rc = find_trigger(m);
+    const int flags = NU_CORRECT | NU_PREDICT | (m->fext_zero ? NU_FEXT_ZERO : 0) |
+                      (m->trigger > 0 ? NU_TRIGGER : 0);
     float ms[2] = {0.f, 0.f};
     for (int pdl = 0; pdl < 2 && rc == AKB_OK; ++pdl) {
       g.pdl = pdl;
@@ -2705,8 +2741,7 @@ int akb_model_autotune(akb_model *m, int repeats) {
   if (e0) cudaEventDestroy(e0);
   if (e1) cudaEventDestroy(e1);
   // captured graphs hold the old launch shapes
-  for (auto &x : m->graphs) cudaGraphExecDestroy(x.exec);
-  m->graphs.clear();
+  m->drop_graphs();
   return rc;
 }
 
@@ -2721,8 +2756,7 @@ int akb_model_set_node_shape(akb_model *m, int node_block, int staged) {
   m->node_block = node_block;
   m->node_form = staged;
   leave_patches(m);
-  for (auto &x : m->graphs) cudaGraphExecDestroy(x.exec);
-  m->graphs.clear();
+  m->drop_graphs();
   return AKB_OK;
 }
 
@@ -2758,8 +2792,7 @@ int akb_model_set_increment_tracking(akb_model *m, int on) {
   }
   m->track_history = on != 0;
   // captured steps hold the launches of the previous setting
-  for (auto &x : m->graphs) cudaGraphExecDestroy(x.exec);
-  m->graphs.clear();
+  m->drop_graphs();
   return AKB_OK;
 }
 
@@ -2784,8 +2817,7 @@ int akb_model_set_affine_kernel(akb_model *m, int on) {
       const int pts = gr.tune.qu & 0xff;
       gr.tune = ElemTuning{128, pts == 8 ? 8 : 2, pts == 8 ? 1 : 4};
     }
-  for (auto &x : m->graphs) cudaGraphExecDestroy(x.exec);
-  m->graphs.clear();
+  m->drop_graphs();
   return AKB_OK;
 }
 
@@ -2799,8 +2831,7 @@ int akb_model_set_dependent_launch(akb_model *m, int on) {
   AKB_TRY(check_model(m, true));
   AKB_CUDA(cudaStreamSynchronize(m->stream));
   m->pdl = on != 0;
-  for (auto &x : m->graphs) cudaGraphExecDestroy(x.exec);
-  m->graphs.clear();
+  m->drop_graphs();
   return AKB_OK;
 }
 
@@ -2819,8 +2850,7 @@ int akb_model_set_fused_step(akb_model *m, int on) {
   AKB_TRY(ensure_fint(m));
   AKB_CUDA(cudaStreamSynchronize(m->stream));
   m->patch_on = on != 0;
-  for (auto &x : m->graphs) cudaGraphExecDestroy(x.exec);
-  m->graphs.clear();
+  m->drop_graphs();
   return AKB_OK;
 }
 
@@ -2876,8 +2906,7 @@ int akb_model_set_launch_shape(akb_model *m, int law, int element_block,
     if (!found) return fail(AKB_EINVAL, "no material of this law in the model");
     m->node_block = node_block;
     AKB_CUDA(cudaStreamSynchronize(m->stream));
-    for (auto &x : m->graphs) cudaGraphExecDestroy(x.exec);
-    m->graphs.clear();
+    m->drop_graphs();
     return AKB_OK;
   }
   const bool sf = m->et == AKB_HEXAHEDRON_8 && m->precision == AKB_PRECISION_MIXED;
@@ -2934,8 +2963,7 @@ int akb_model_set_launch_shape(akb_model *m, int law, int element_block,
   m->node_block = node_block;
   leave_patches(m);
   AKB_CUDA(cudaStreamSynchronize(m->stream));
-  for (auto &x : m->graphs) cudaGraphExecDestroy(x.exec);
-  m->graphs.clear();
+  m->drop_graphs();
   return AKB_OK;
 }
 
@@ -2957,8 +2985,7 @@ int akb_model_set_prefetch(akb_model *m, int law, int waves) {
   if (!found) return fail(AKB_EINVAL, "no material of this law in the model");
   leave_patches(m);
   AKB_CUDA(cudaStreamSynchronize(m->stream));
-  for (auto &x : m->graphs) cudaGraphExecDestroy(x.exec);
-  m->graphs.clear();
+  m->drop_graphs();
   return AKB_OK;
 }
 
@@ -2979,8 +3006,7 @@ int akb_model_set_recompute_geometry(akb_model *m, int law, int on) {
   if (!found) return fail(AKB_EINVAL, "no material of this law in the model");
   leave_patches(m);
   AKB_CUDA(cudaStreamSynchronize(m->stream));
-  for (auto &x : m->graphs) cudaGraphExecDestroy(x.exec);
-  m->graphs.clear();
+  m->drop_graphs();
   return AKB_OK;
 }
 
@@ -3005,8 +3031,7 @@ int akb_model_set_streamed_points(akb_model *m, int law, int on) {
   if (!found) return fail(AKB_EINVAL, "no material of this law in the model");
   leave_patches(m);
   AKB_CUDA(cudaStreamSynchronize(m->stream));
-  for (auto &x : m->graphs) cudaGraphExecDestroy(x.exec);
-  m->graphs.clear();
+  m->drop_graphs();
   return AKB_OK;
 }
 

@@ -204,3 +204,23 @@ def test_fused_step_whose_tables_are_larger_than_l2(precision, cells):
     for m in models:
         m.solveStep(5)
     _same(models)
+
+
+@pytest.mark.parametrize("n", [36, 38, 43])
+def test_dependent_launches_around_one_wave(n):
+    """two-kernel steps whose kernels are resident together, not quite, and of
+    more than one wave: with and without dependent launches the same bits, with a
+    setting changed between two sequences"""
+    mesh = akb.box_hex8(n)
+    models = []
+    for dependent in (True, False):
+        m = gpu_model(mesh, [UNIT_NEOHOOKEAN], precision="mixed")
+        assert not m.getFusedStep()
+        m.setDependentLaunch(dependent)
+        m.setNodal("velocity", sinusoidal_velocity(mesh.nodes, 0.03))
+        m.setTimeStep(0.8 * m.getStableTimeStep())
+        m.solveStep(103)
+        m.setNodeShape(64, 0)
+        m.solveStep(2)
+        models.append(m)
+    _same(models)
