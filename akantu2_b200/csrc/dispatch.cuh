@@ -30,6 +30,7 @@ inline cudaError_t launch_step_smem(bool pdl, void (*kernel)(KArgs...), unsigned
     int resident = 0;
     const cudaError_t e =
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kernel, (int)block, smem);
+    launch_probe->blocks = grid;
     launch_probe->waves += (double)grid / (148. * std::max(resident, 1));
     return e;
   }

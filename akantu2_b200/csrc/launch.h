@@ -45,10 +45,11 @@ struct ElemTuning {
 // evaluated as packed FP32 pairs (2, 4 or 8 points per iteration)
 constexpr int kPackedPoints = 256;
 
-// While a thread has one, its step kernels are not launched: the probe counts
+// While a thread has one, its step kernels are not launched: the probe adds up
 // the waves of resident blocks that their grids fill.
 struct LaunchProbe {
   double waves = 0.;
+  unsigned blocks = 0;  // of the last grid
 };
 inline thread_local LaunchProbe *launch_probe = nullptr;
 

@@ -296,8 +296,8 @@ struct akb_model {
   // step kernels launched with programmatic stream serialization: each one
   // is scheduled while its predecessor drains and waits for it on the device
   bool pdl = false;
-  // whether its kernels let the next one launch at once: their blocks are all
-  // resident together (-1: not looked at since the launches last changed)
+  // which of its two kernels lets the next one launch at once, 1: element
+  // forces, 2: node update (-1: not looked at since the launches last changed)
   int trigger = -1;
   // fused step (patch.h): one launch per step over patches of nodes, when the
   // model has a plan for it and no kernel of the two-kernel step was chosen
@@ -546,7 +546,7 @@ GroupArgs group_args(akb_model *m, const Group &mt, bool in_step) {
   ps.nb_nodes = m->N;
   ps.nb_slots = m->E * m->nn;
   ps.status = m->dstatus;
-  ps.trigger = in_step && m->trigger > 0;
+  ps.trigger = in_step && m->trigger > 0 && (m->trigger & 1);
   if (m->dinst_end) {
     ps.einst = m->delem_inst + mt.e_begin;
     ps.inst_end = m->dinst_end;
@@ -687,7 +687,7 @@ int launch_nodes(akb_model *m, bool correct) {
   cudaError_t e;
   int flags = correct ? (NU_CORRECT | NU_PREDICT) : NU_FINT;
   if (correct && m->fext_zero) flags |= NU_FEXT_ZERO;
-  if (correct && m->trigger > 0) flags |= NU_TRIGGER;
+  if (correct && m->trigger > 0 && (m->trigger & 2)) flags |= NU_TRIGGER;
   const double *u = m->u_pred();
   double *u_next = m->u();
   // the next step's prescribed dofs are written by the same launch (a batch
@@ -713,15 +713,21 @@ int node_update(akb_model *m, bool correct) {
   return AKB_OK;
 }
 
-// whether the two kernels' blocks are resident all together (pdl_begin)
+// Both where the two kernels' blocks are resident all together (pdl_begin).  A
+// node update of up to 8 blocks per SM also before element kernels of more,
+// whose many waves start under it (us per step, without / with: FP64
+// tetrahedra, 236 k 21.2 / 20.8, 384 k 29.2 / 28.5).
 int find_trigger(akb_model *m) {
   if (m->trigger >= 0) return AKB_OK;
   LaunchProbe probe;
   launch_probe = &probe;
   int rc = launch_forces(m, true);
+  const unsigned elem_blocks = probe.blocks;
   if (rc == AKB_OK) rc = launch_nodes(m, true);
   launch_probe = nullptr;
-  if (rc == AKB_OK) m->trigger = probe.waves <= 1.;
+  const unsigned many = 8 * kPatchSms;
+  if (rc == AKB_OK)
+    m->trigger = probe.waves <= 1. ? 3 : elem_blocks > many && probe.blocks <= many ? 2 : 0;
   return rc;
 }
 
@@ -1076,14 +1082,14 @@ int reduce_to_host(akb_model *m, const double *x, int64_t n, bool op_min, double
 // points mixed, 6.5 with 121 patches, 7.9 with 64), else the largest.  With more
 // patches than are resident at once the two kernels, which read every point's
 // state once, are faster (512^2 x 2: 111 against 154).
-// The finite-deformation laws of FP64 tetrahedra: up to 50,000 elements.  Past
+// The finite-deformation laws of FP64 tetrahedra: up to 32,000 elements.  Past
 // that their FP64 operations (a logarithm each) are the bound, of which the
 // patches evaluate those of the border elements again (us per step, two kernels
-// / fused: 25 k 9.5 / 7.7, 48 k 10.2 / 8.3, 64 k 11.3 / 11.9, 162 k 16.3 / 21.2,
-// 1.3 M 102 / 117; elastic 1.3 M 94 / 74).
+// / fused: 25 k 9.5 / 7.7, 48 k 10.2 / 8.3 (a cube) and 11.0 / 12.0 (a flat box), 64 k
+// 11.3 / 11.9, 162 k 16.3 / 21.2, 1.3 M 102 / 117; elastic 1.3 M 94 / 74).
 int patch_nodes(int et, int rule, int law, int precision, int64_t N, int64_t E, int ninst) {
   const bool mixed = precision == AKB_PRECISION_MIXED;
-  if (!mixed && law == LAW_NEOHOOKEAN && E > 50000) return 0;
+  if (!mixed && law == LAW_NEOHOOKEAN && E > 32000) return 0;
   const double sms = 148.;
   const double planes = std::pow((double)N / ninst, 1. / dim_of(et));
   int best = 0;
@@ -2682,7 +2688,7 @@ int akb_model_autotune(akb_model *m, int repeats) {
     m->trigger = -1;
     rc = find_trigger(m);
     const int flags = NU_CORRECT | NU_PREDICT | (m->fext_zero ? NU_FEXT_ZERO : 0) |
-                      (m->trigger > 0 ? NU_TRIGGER : 0);
+                      (m->trigger > 0 && (m->trigger & 2) ? NU_TRIGGER : 0);
     float ms[2] = {0.f, 0.f};
     for (int pdl = 0; pdl < 2 && rc == AKB_OK; ++pdl) {
       g.pdl = pdl;
