@@ -2046,9 +2046,10 @@ __global__ void __launch_bounds__(32 * NQ)
 //                     request by a flags == NU_FINT launch)
 //        NU_FEXT_ZERO the external force is identically zero: not read
 //        NU_TRIGGER   the next kernel may launch at once (pdl_begin)
+//        NU_DOWN      the nodes from the last one down (node_block)
 //                     (0 + f_ext + f_int == f_int)
 // KAHAN selects a compensated FP64 sum (mixed path).
-enum { NU_CORRECT = 1, NU_PREDICT = 2, NU_FINT = 4, NU_FEXT_ZERO = 8, NU_TRIGGER = 16 };
+enum { NU_CORRECT = 1, NU_PREDICT = 2, NU_FINT = 4, NU_FEXT_ZERO = 8, NU_TRIGGER = 16, NU_DOWN = 32 };
 
 // one slot into the internal-force sum, sign -1 (dof_manager.cc:65-120),
 // optionally compensated
@@ -2353,13 +2354,13 @@ __device__ __forceinline__ void node_body(int64_t i, const int32_t *ptr,
 }
 
 
-// The block of nodes of a thread block of the node updates: from the last one
-// down, as the element kernel has just written the slots of the last nodes
-// (they are in L2), and leaves the next step's elements the displacements of
-// the first ones there (us per step, before / after: hex8 mixed 128^3 285.8 /
-// 282.5, 96^3 129.4 / 125.7; tri6 512^2 110.9 / 109.8; hex8 FP64 56^3 135.1 / 133.1).  With RAMP the extra block, the last, is block -1.
-template <bool RAMP> __device__ __forceinline__ int64_t node_block() {
-  return (int64_t)gridDim.x - (RAMP ? 2 : 1) - blockIdx.x;
+// The block of nodes of a thread block of the node updates.  With NU_DOWN from
+// the last one down, as the element kernel has just written the slots of the
+// last nodes (they are in L2), and leaves the next step's elements the
+// displacements of the first ones there.  With RAMP the extra block, the last,
+// has none (its index is -1, or past the nodes).
+template <bool RAMP> __device__ __forceinline__ int64_t node_block(int flags) {
+  return flags & NU_DOWN ? (int64_t)gridDim.x - (RAMP ? 2 : 1) - blockIdx.x : blockIdx.x;
 }
 
 // launched with up to 1024 threads per block (the autotuner's candidates):
@@ -2376,7 +2377,7 @@ __global__ void __launch_bounds__(1024) k_node_update(int64_t N, const int32_t *
                               unsigned int *__restrict__ status, const PrescArgs pr) {
   pdl_begin(flags & NU_TRIGGER);
   if (RAMP && blockIdx.x == gridDim.x - 1) return prescribe_block(pr, u_next, true);
-  const int64_t i = node_block<RAMP>() * blockDim.x + threadIdx.x;
+  const int64_t i = node_block<RAMP>(flags) * blockDim.x + threadIdx.x;
   if (i >= N || !node_range_ok(ptr, N, i, status)) return;
   node_body<D, RT, KAHAN, WIDE, RAMP>(i, ptr, re, fext, mass, blocked, fint, a, v, u, u_next, dt,
                                 node_inst, inst_dt, flags, status);
@@ -2396,7 +2397,7 @@ __global__ void __launch_bounds__(1024)
                         const double *__restrict__ u, double *__restrict__ u_next, double dt,
                         const int32_t *__restrict__ node_inst, const double *__restrict__ inst_dt,
                         int flags, unsigned int *__restrict__ status, const PrescArgs pr) {
-  const int64_t i = node_block<RAMP>() * blockDim.x + threadIdx.x;
+  const int64_t i = node_block<RAMP>(flags) * blockDim.x + threadIdx.x;
   const bool in = (!RAMP || i >= 0) && i < N;
   int32_t p0 = 0, p1 = 0;
   NodeState<D> st;
@@ -2495,7 +2496,7 @@ __global__ void __launch_bounds__(BLOCK)
   constexpr int CAPW = kStagedBytes / (int)sizeof(V);
   constexpr int CAP = CAPW / WPS;               // slots per chunk
   __shared__ V sm[CAPW];
-  const int64_t i0 = node_block<RAMP>() * BLOCK;
+  const int64_t i0 = node_block<RAMP>(flags) * BLOCK;
   const int64_t i = i0 + threadIdx.x;
   const int64_t iend = i0 + BLOCK < N ? i0 + BLOCK : N;
   const int32_t pb = ptr[i0], pe = ptr[iend];

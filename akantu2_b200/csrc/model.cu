@@ -682,11 +682,29 @@ int predict(akb_model *m) {
 // u_pred into the other buffer (which held the displacement of the previous
 // step); the internal force is only gathered when asked for (ensure_fint).
 // Standalone (correct == false): the internal force only.
+// whether what a step reads and writes is well beyond L2 (1.25 x 126 MB): the
+// node update then goes from the last nodes down (us per step, up / down: hex8
+// mixed 78 x 41 x 76, 104 MB, 51.0 / 51.7, 96 x 70 x 58, 151 MB, 60.0 / 60.5, 80^3,
+// 199 MB, 77.8 / 76.7, 96^3 129.4 / 125.7, 128^3 285.8 / 282.5; FP64 56^3 135.1 /
+// 133.1; plastic triangles 512^2 110.9 / 109.8)
+bool step_beyond_l2(const akb_model *m) {
+  const bool mixed = m->precision == AKB_PRECISION_MIXED;
+  const bool hex = m->et == AKB_HEXAHEDRON_8, tri = m->et == AKB_TRIANGLE_6;
+  const double value = mixed ? 4. : 8.;
+  const double slot = mixed ? (tri ? 8. : 16.) : 8. * m->dim;
+  double table = tri || (hex && !mixed && !m->fast64) ? m->nq * (m->nn * m->dim + 1.) * value
+                                                      : 10. * value;
+  for (auto &gr : m->groups)
+    if (gr.law == LAW_PLASTIC) table += m->nq * (tri ? 2. * 60. : 2. * 130.) * gr.e_count / m->E;
+  return m->E * (m->nn * (8. + slot) + table) + 150. * m->N > 1.25 * 126e6;
+}
+
 int launch_nodes(akb_model *m, bool correct) {
   DevGeom g = m->geom();
   cudaError_t e;
   int flags = correct ? (NU_CORRECT | NU_PREDICT) : NU_FINT;
   if (correct && m->fext_zero) flags |= NU_FEXT_ZERO;
+  if (step_beyond_l2(m)) flags |= NU_DOWN;
   if (correct && m->trigger > 0 && (m->trigger & 2)) flags |= NU_TRIGGER;
   const double *u = m->u_pred();
   double *u_next = m->u();
@@ -2688,7 +2706,8 @@ int akb_model_autotune(akb_model *m, int repeats) {
     m->trigger = -1;
     rc = find_trigger(m);
     const int flags = NU_CORRECT | NU_PREDICT | (m->fext_zero ? NU_FEXT_ZERO : 0) |
-                      (m->trigger > 0 && (m->trigger & 2) ? NU_TRIGGER : 0);
+                      (m->trigger > 0 && (m->trigger & 2) ? NU_TRIGGER : 0) |
+                      (step_beyond_l2(m) ? NU_DOWN : 0);
     float ms[2] = {0.f, 0.f};
     for (int pdl = 0; pdl < 2 && rc == AKB_OK; ++pdl) {
       g.pdl = pdl;
