@@ -2427,7 +2427,9 @@ __global__ void __launch_bounds__(1024)
 // a node of a stopped instance keeps its state; the displacement buffer that
 // becomes the model's displacement after this step (u, the prediction's
 // buffer) takes the value of the other one (u_next), which holds the
-// instance's last displacement, so that both buffers hold it from then on
+// instance's last displacement, so that both buffers hold it from then on.
+// The last step of an instance stores its internal force: a later gather of
+// the slots leaves stopped instances out
 template <int D, class RT, bool KAHAN>
 __global__ void __launch_bounds__(1024) k_node_update_retire(int64_t N, const int32_t *__restrict__ ptr,
                                      const RT *__restrict__ re, const double *__restrict__ fext,
@@ -2444,13 +2446,15 @@ __global__ void __launch_bounds__(1024) k_node_update_retire(int64_t N, const in
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N || !node_range_ok(ptr, N, i, status)) return;
   // a batch of one instance has no node -> instance table
-  if (*step >= inst_end[node_inst ? node_inst[i] : 0]) {
+  const int64_t left = inst_end[node_inst ? node_inst[i] : 0] - *step;
+  if (left <= 0) {
     if (flags & NU_PREDICT) {
 #pragma unroll
       for (int c = 0; c < D; ++c) u[i * D + c] = u_next[i * D + c];
     }
     return;
   }
+  if (left == 1) flags |= NU_FINT;
   node_body<D, RT, KAHAN, false>(i, ptr, re, fext, mass, blocked, fint, a, v, u, u_next, dt,
                                  node_inst, inst_dt, flags, status);
 }

@@ -352,15 +352,21 @@ __global__ void __launch_bounds__(THREADS, MINB)
     }
   }
   pdl_begin(trigger);
-  // a stopped instance keeps its state (k_node_update_retire)
-  if (pa.inst_end && *pa.step >= pa.inst_end[h.inst]) {
-    copy_async_wait();
-    if (pa.flags & NU_PREDICT)
-      for (int j = threadIdx.x; j < h.n_own * D; j += THREADS) {
-        const int64_t k = (int64_t)own[j / D].node * D + j % D;
-        pa.u[k] = pa.u_next[k];
-      }
-    return;
+  // as in k_node_update_retire: a stopped instance keeps its state, and the
+  // last step of an instance stores its internal force
+  int flags = pa.flags;
+  if (pa.inst_end) {
+    const int64_t left = pa.inst_end[h.inst] - *pa.step;
+    if (left <= 0) {
+      copy_async_wait();
+      if (flags & NU_PREDICT)
+        for (int j = threadIdx.x; j < h.n_own * D; j += THREADS) {
+          const int64_t k = (int64_t)own[j / D].node * D + j % D;
+          pa.u[k] = pa.u_next[k];
+        }
+      return;
+    }
+    if (left == 1) flags |= NU_FINT;
   }
 #pragma unroll
   for (int k = 0; k < U; ++k) {
@@ -482,7 +488,7 @@ __global__ void __launch_bounds__(THREADS, MINB)
       accumulate_slot<D, KAHAN>(rv, acc, comp);
     }
     node_apply_state<D, true>(node, acc, st, pa.fint, pa.a, pa.v, pa.u_next, dt, nullptr, nullptr,
-                        pa.flags, pa.status);
+                        flags, pa.status);
   }
 }
 

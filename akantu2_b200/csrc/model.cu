@@ -1978,6 +1978,8 @@ int akb_batch_set_instance_steps(akb_model *m, const int64_t *steps) {
   AKB_TRY(check_model(m, true));
   if (!m->is_batch) return fail(AKB_EINVAL, "not a batch (akb_batch_create)");
   if (!steps) return fail(AKB_EINVAL, "null argument");
+  // an instance that stops here has its internal force stored by no step
+  AKB_TRY(ensure_fint(m));
   const int ni = m->ninst;
   if (!m->dinst_end) {
     // instance of each internal element, from the user order offsets

@@ -224,3 +224,32 @@ def test_dependent_launches_around_one_wave(n):
         m.solveStep(2)
         models.append(m)
     _same(models)
+
+
+@pytest.mark.parametrize("fused", [True, False])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_internal_force_of_stopped_instances(precision, fused):
+    """an instance that stops at once, in the middle of a sequence or with its
+    last step has the internal force of its own last step, in both forms of the
+    step: that of the same mesh run alone"""
+    meshes = [akb.box_tet4(n) for n in (3, 6, 4)]
+    b = akb.BatchModel(meshes)
+    mat = {k: v for k, v in UNIT_ELASTIC.items() if k != "type"}
+    b.addMaterial("elastic", **mat)
+    b.initFull(precision=precision)
+    b.setFusedStep(fused)
+    dt = 0.8 * b.getStableTimeSteps()
+    b.setTimeSteps(dt)
+    b.setNodal("velocity", sinusoidal_velocity(b.mesh.nodes, 0.03))
+    b.solveStep(20)
+    b.setInstanceSteps([0, 30, 7])
+    b.solveStep(30)
+    b.solveStep(5)
+    for k, steps in enumerate((20, 50, 27)):
+        alone = gpu_model(meshes[k], [UNIT_ELASTIC], precision=precision)
+        alone.setNodal("velocity", sinusoidal_velocity(meshes[k].nodes, 0.03))
+        alone.setTimeStep(float(dt[k]))
+        alone.solveStep(steps)
+        for f in FIELDS:
+            a, c = getattr(b, f)()[b.instance_nodes(k)], getattr(alone, f)()
+            assert np.abs(c).max() > 0 and np.array_equal(a, c), (k, f)
