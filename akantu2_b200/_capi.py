@@ -150,6 +150,7 @@ def lib():
         "akb_estimate_device_bytes": (c_int, [c_int, c_int, i64, i64, c_int, c_int,
                                               ctypes.POINTER(i64)]),
         "akb_bounds_checked": (c_int, []),
+        "akb_debug_limit_device_bytes": (c_int, [i64]),
         "akb_model_debug_write_index": (c_int, [vp, c_int, i64, ctypes.c_int32]),
         "akb_model_set_persistent_wait_test": (c_int, [vp, ctypes.c_uint, c_int, ctypes.c_uint]),
         "akb_exchange_create": (c_int, [vp, c_int, pp]),

@@ -19,6 +19,7 @@
 
 namespace akb {
 static thread_local std::string g_last_error;
+static thread_local int64_t g_device_limit = 0;  // akb_debug_limit_device_bytes (0: none)
 int fail(int code, const std::string &msg) {
   g_last_error = msg;
   return code;
@@ -302,6 +303,8 @@ struct akb_model {
   // fused step (patch.h): one launch per step over patches of nodes, when the
   // model has a plan for it and no kernel of the two-kernel step was chosen
   PatchArgs patch;
+  void *patch_mem = nullptr;  // its arrays
+  size_t patch_bytes = 0;
   bool patch_ready = false, patch_on = false;
   // persistent multi-step kernel: 0 never (default: on B200 the 100-step
   // graphs of the two-kernel step are faster at every measured size), 1 for
@@ -340,10 +343,27 @@ struct akb_model {
   }
   // stream-ordered allocations on the model's stream: neither allocating
   // nor freeing waits for the work of other models on the device
+  cudaError_t device_malloc(void **q, size_t bytes) {
+    if (g_device_limit > 0 && device_bytes + bytes > (size_t)g_device_limit)
+      return cudaErrorMemoryAllocation;
+    const cudaError_t e = cudaMallocAsync(q, bytes, stream);
+    if (e == cudaErrorMemoryAllocation) cudaGetLastError();
+    return e;
+  }
+  // the same for what the model cannot do without: the plan of the fused step
+  // gives its memory back first
+  cudaError_t device_malloc_needed(void **q, size_t bytes) {
+    cudaError_t e = device_malloc(q, bytes);
+    if (e == cudaErrorMemoryAllocation && patch_bytes > 0) {
+      release_patches();
+      e = device_malloc(q, bytes);
+    }
+    return e;
+  }
   template <class P> int alloc(P **p, size_t bytes) {
     void *q = nullptr;
     if (bytes == 0) bytes = 16;
-    cudaError_t e = cudaMallocAsync(&q, bytes, stream);
+    cudaError_t e = device_malloc_needed(&q, bytes);
     if (e != cudaSuccess)
       return fail(e == cudaErrorMemoryAllocation ? AKB_ENOMEM : AKB_ECUDA,
                   std::string("cudaMallocAsync: ") + cudaGetErrorString(e));
@@ -353,6 +373,18 @@ struct akb_model {
     return AKB_OK;
   }
   size_t device_bytes = 0;
+  // the plan of the fused step; the two kernels step from now on (between
+  // steps, so the last one has stored the internal force)
+  void release_patches() {
+    cudaStreamSynchronize(stream);
+    drop_graphs();
+    cudaFreeAsync(patch_mem, stream);
+    cudaStreamSynchronize(stream);
+    device_bytes -= patch_bytes;
+    patch_mem = nullptr;
+    patch_bytes = 0;
+    patch_ready = patch_on = false;
+  }
   // asynchronous nodal I/O: copy streams, device staging (two upload
   // buffers, AKB_ASYNC_READS_IN_FLIGHT read buffers) and the events that
   // order them against the step stream
@@ -369,6 +401,7 @@ struct akb_model {
     if (aio.in) cudaStreamSynchronize(aio.in);
     if (aio.out) cudaStreamSynchronize(aio.out);
     drop_graphs();
+    if (patch_mem) cudaFreeAsync(patch_mem, stream);
     for (void *p : allocs) cudaFreeAsync(p, stream);
     for (int k = 0; k < AsyncIO::kIn; ++k)
       for (cudaEvent_t e : {aio.in_ready[k], aio.in_used[k]})
@@ -1161,26 +1194,34 @@ PatchTables patch_tables(int et, int law, int precision, int nq) {
   return t;
 }
 
-// bytes of a plan's arrays at their capacity, in one allocation
-size_t patch_capacity_bytes(const PatchCaps &c, int64_t N, int nn, const PatchTables &t) {
-  size_t bytes = 0;
-  auto take = [&](int64_t n, size_t size) { bytes += ((size_t)n * size + 255) / 256 * 256; };
-  take(c.patches, sizeof(PatchHead));
-  take(c.nodes, sizeof(int32_t));
-  take(N, sizeof(PatchOwn));
-  take(c.elems, sizeof(int32_t));
-  take(c.elems, 2 * sizeof(uint16_t) * (nn <= 4 ? 4 : 8) + t.rows * t.value);
-  return bytes;
+// Where a plan's arrays lie in their allocation: the lists of its patches,
+// nodes, owned nodes and elements, then the chunks
+struct PatchRoom {
+  size_t nodes, own, elems, tab, bytes;
+};
+PatchRoom patch_room(const PatchCaps &c, int64_t N, int nn, const PatchTables &t) {
+  size_t at = 0;
+  auto take = [&](int64_t n, size_t size) {
+    at += ((size_t)n * size + 255) / 256 * 256;
+    return at;
+  };
+  PatchRoom r;
+  r.nodes = take(c.patches, sizeof(PatchHead));
+  r.own = take(c.nodes, sizeof(int32_t));
+  r.elems = take(N, sizeof(PatchOwn));
+  r.tab = take(c.elems, sizeof(int32_t));
+  r.bytes = take(c.elems, 2 * sizeof(uint16_t) * (nn <= 4 ? 4 : 8) + t.rows * t.value);
+  return r;
 }
 
-// device bytes of a plan (the same for any mesh of these sizes)
+// device bytes of a plan at most (the same for any mesh of these sizes)
 int64_t patch_bytes(int et, int rule, int law, int precision, int64_t N, int64_t E, int ninst) {
   const PatchTables t = patch_tables(et, law, precision, et == AKB_TRIANGLE_6 && rule ? 6 : 3);
   if (t.rows == 0 || N == 0 || E == 0) return 0;
   const int own = patch_nodes(et, rule, law, precision, N, E, ninst);
   if (own == 0) return 0;
   const PatchCaps c = patch_caps(dim_of(et), N, E, ninst, own);
-  return (int64_t)patch_capacity_bytes(c, N, nodes_per_element(et), t);
+  return (int64_t)patch_room(c, N, nodes_per_element(et), t).bytes;
 }
 
 // Builds the plan on a thread of its own while initFull goes on with the
@@ -1230,21 +1271,24 @@ void start_patches(akb_model *m, const std::vector<int32_t> &conn_soa,
   pm.pos = pos.data();
   pm.inst_off = m->inst_node_off.data();
   pm.ninst = m->ninst;
-  if (gr.nmat > 1) {
-    task.mat.resize(m->E);
-    for (int64_t ie = 0; ie < m->E; ++ie) task.mat[ie] = m->mat_user[m->perm[ie]];
-    pm.mat = task.mat.data();
-  }
   task.caps = patch_caps(m->dim, m->N, m->E, m->ninst, pm.max_own);
-  task.wanted = true;
   try {
+    if (gr.nmat > 1) {
+      task.mat.resize(m->E);
+      for (int64_t ie = 0; ie < m->E; ++ie) task.mat[ie] = m->mat_user[m->perm[ie]];
+      pm.mat = task.mat.data();
+    }
+    task.wanted = true;
     task.worker = std::thread([&task] { task.build(); });
+  } catch (const std::bad_alloc &) {
+    task.wanted = false;
   } catch (const std::exception &) {
-    task.build();
+    task.build();  // no thread to be had
   }
 }
 
-// the finished plan's arrays on the device
+// The finished plan's arrays on the device.  The model can do without them:
+// with too little device memory the two kernels step.
 int finish_patches(akb_model *m, PatchTask &task) {
   task.wait();
   const bool hex = m->et == AKB_HEXAHEDRON_8, mixed = m->precision == AKB_PRECISION_MIXED;
@@ -1256,62 +1300,67 @@ int finish_patches(akb_model *m, PatchTask &task) {
   const int points = m->et == AKB_TRIANGLE_6 ? m->nq : 1;  // slot arrays
   pa.smem = patch_smem(m->dim, plan.max_local, plan.max_slots * points, t.value);
   if (pa.smem + kPatchStageSmem > kPatchMaxSmem) return AKB_OK;
-  const size_t bytes =
-      patch_capacity_bytes(task.caps, m->N, m->nn, t);  // the capacity, whatever the mesh needs
-  char *base = nullptr;
-  AKB_TRY(m->alloc(&base, bytes));
+  PatchCaps need;
+  need.patches = (int64_t)plan.head.size();
+  need.nodes = (int64_t)plan.nodes.size();
+  need.elems = (int64_t)plan.elems.size();
+  const PatchRoom room = patch_room(need, m->N, m->nn, t);
+  // a small plan takes its capacity, what akb_estimate_device_bytes says to the
+  // byte; a large one what it needs (two thirds of it)
+  const size_t bytes = std::min(patch_room(task.caps, m->N, m->nn, t).bytes,
+                                std::max(room.bytes, (size_t)8 << 20));
   cudaStream_t s = m->stream;
-  // the lists in one upload, the chunks behind them; the local indices the
-  // chunks are made of are on the device for the time being
-  const int64_t n = (int64_t)plan.elems.size();
-  size_t at = 0;
-  auto take = [&](size_t size) {
-    const size_t here = at;
-    at += (size + 255) / 256 * 256;
-    return here;
-  };
-  const size_t o_head = take(plan.head.size() * sizeof(PatchHead));
-  const size_t o_nodes = take(plan.nodes.size() * sizeof(int32_t));
-  const size_t o_own = take(plan.own.size() * sizeof(PatchOwn));
-  const size_t o_elems = take(plan.elems.size() * sizeof(int32_t));
-  const size_t o_tab = at;
+  // the local indices the chunks are made of are on the device for the time being
   const size_t lb = plan.conn.size() * sizeof(uint16_t);
-  std::vector<char> lists(o_tab), local(2 * lb);
-  std::memcpy(lists.data() + o_head, plan.head.data(), plan.head.size() * sizeof(PatchHead));
-  std::memcpy(lists.data() + o_nodes, plan.nodes.data(), plan.nodes.size() * sizeof(int32_t));
-  std::memcpy(lists.data() + o_own, plan.own.data(), plan.own.size() * sizeof(PatchOwn));
-  std::memcpy(lists.data() + o_elems, plan.elems.data(), plan.elems.size() * sizeof(int32_t));
-  std::memcpy(local.data(), plan.conn.data(), lb);
-  std::memcpy(local.data() + lb, plan.slot.data(), lb);
-  AKB_CUDA(cudaMemcpyAsync(base, lists.data(), lists.size(), cudaMemcpyHostToDevice, s));
-  pa.npatch = (int64_t)plan.head.size();
+  void *mem = nullptr, *local = nullptr;
+  cudaError_t e = m->device_malloc(&mem, bytes);
+  if (e == cudaSuccess) e = m->device_malloc(&local, 2 * lb);
+  if (e != cudaSuccess) {
+    if (mem) cudaFreeAsync(mem, s);
+    if (e == cudaErrorMemoryAllocation) return AKB_OK;
+    return fail(AKB_ECUDA, std::string("fused step: ") + cudaGetErrorString(e));
+  }
+  char *base = (char *)mem, *dlocal = (char *)local;
+  auto upload = [&](char *to, const void *from, size_t bytes) {
+    if (e == cudaSuccess) e = cudaMemcpyAsync(to, from, bytes, cudaMemcpyHostToDevice, s);
+  };
+  upload(base, plan.head.data(), plan.head.size() * sizeof(PatchHead));
+  upload(base + room.nodes, plan.nodes.data(), plan.nodes.size() * sizeof(int32_t));
+  upload(base + room.own, plan.own.data(), plan.own.size() * sizeof(PatchOwn));
+  upload(base + room.elems, plan.elems.data(), plan.elems.size() * sizeof(int32_t));
+  upload(dlocal, plan.conn.data(), lb);
+  upload(dlocal + lb, plan.slot.data(), lb);
+  pa.npatch = need.patches;
   pa.max_own = task.mesh.max_own;
   pa.multi = 0;
   for (const PatchHead &h : plan.head) pa.multi |= gr.nmat > 1 && h.mat < 0 && h.n_elem > 0;
-  pa.head = (const PatchHead *)(base + o_head);
-  pa.nodes = (const int32_t *)(base + o_nodes);
-  pa.own = (const PatchOwn *)(base + o_own);
-  pa.elems = (const int32_t *)(base + o_elems);
-  pa.tab = base + o_tab;
+  pa.head = (const PatchHead *)base;
+  pa.nodes = (const int32_t *)(base + room.nodes);
+  pa.own = (const PatchOwn *)(base + room.own);
+  pa.elems = (const int32_t *)(base + room.elems);
+  pa.tab = base + room.tab;
   pa.e_count = m->E;
   pa.nq = m->nq;
   // beyond L2 (126 MB): the tables of the next wave of patches are prefetched
   // (us per step, without / with: batch of 64 cubes, mixed, 148 / 137, FP64 242 /
   // 223; 1.3 M tetrahedra, FP64, 73.7 / 72.8; mixed, whose 104 MB stay in L2,
   // 45.9 / 47.6)
-  pa.ahead = (size_t)n * (2 * sizeof(uint16_t) * plan.NNP + t.rows * t.value) > (size_t)126 << 20;
-  char *dlocal = nullptr;
-  AKB_CUDA(cudaMallocAsync((void **)&dlocal, std::max<size_t>(local.size(), 16), s));
-  cudaError_t e = cudaMemcpyAsync(dlocal, local.data(), local.size(), cudaMemcpyHostToDevice, s);
+  pa.ahead = room.bytes - room.tab > (size_t)126 << 20;
   const void *ta = hex ? (const void *)m->dgeo : mixed ? (const void *)m->fB : m->dB;
   const void *tb = hex ? nullptr : mixed ? (const void *)m->fwJ : m->dwJ;
   if (e == cudaSuccess)
-    e = launch_patch_chunks(plan.NNP, n, pa.elems, (const uint16_t *)dlocal,
+    e = launch_patch_chunks(plan.NNP, need.elems, pa.elems, (const uint16_t *)dlocal,
                             (const uint16_t *)(dlocal + lb), m->E, hex ? t.rows : t.rows - m->nq,
-                            ta, hex ? 0 : m->nq, tb, t.value, base + o_tab, s);
+                            ta, hex ? 0 : m->nq, tb, t.value, base + room.tab, s);
   cudaFreeAsync(dlocal, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);  // the host copies are freed
-  if (e != cudaSuccess) return fail(AKB_ECUDA, std::string("fused step: ") + cudaGetErrorString(e));
+  if (e != cudaSuccess) {
+    cudaFreeAsync(mem, s);
+    return fail(AKB_ECUDA, std::string("fused step: ") + cudaGetErrorString(e));
+  }
+  m->patch_mem = mem;
+  m->patch_bytes = bytes;
+  m->device_bytes += bytes;
   m->patch_ready = m->patch_on = true;
   return AKB_OK;
 }
@@ -2535,7 +2584,7 @@ int akb_model_autotune(akb_model *m, int repeats) {
   const int64_t dd = (int64_t)m->dim * m->dim, ns = sym_comps(m->dim);
   double *tmp = nullptr;
   const size_t tmp_doubles = (size_t)(state_n * (2 * ns + dd + 1) + 3 * nd + 1);
-  AKB_CUDA(cudaMallocAsync((void **)&tmp, sizeof(double) * tmp_doubles, s));
+  AKB_CUDA(m->device_malloc_needed((void **)&tmp, sizeof(double) * tmp_doubles));
   double *t_sig = tmp, *t_gu = t_sig + state_n * ns, *t_eps = t_gu + state_n * dd;
   double *t_iso = t_eps + state_n * ns, *t_a = t_iso + state_n, *t_v = t_a + nd;
   double *t_u = t_v + nd;
@@ -2564,7 +2613,7 @@ int akb_model_autotune(akb_model *m, int repeats) {
   for (auto &gr : m->groups)
     if (gr.c33) c33_n = std::max(c33_n, gr.e_count * m->nq);
   double *t_c33 = nullptr;
-  if (c33_n > 0) AKB_CUDA(cudaMallocAsync((void **)&t_c33, sizeof(double) * c33_n, s));
+  if (c33_n > 0) AKB_CUDA(m->device_malloc_needed((void **)&t_c33, sizeof(double) * c33_n));
   auto scratch_args = [&](const Group &gr) {
     GroupArgs ps = group_args(m, gr, false);
     if (gr.c33) ps.c33 = t_c33;
@@ -3400,6 +3449,12 @@ int akb_bounds_checked(void) {
 #endif
 }
 
+int akb_debug_limit_device_bytes(int64_t bytes) {
+  if (bytes < 0) return fail(AKB_EINVAL, "negative size");
+  g_device_limit = bytes;
+  return AKB_OK;
+}
+
 int akb_model_debug_write_index(akb_model *m, int which, int64_t position, int32_t value) {
 #ifndef AKB_BOUNDS_CHECK
   (void)m, (void)which, (void)position, (void)value;
@@ -3522,6 +3577,12 @@ struct akb_exchange {
     DeviceGuard g(dev);
     void *q = nullptr;
     cudaError_t e = cudaMalloc(&q, bytes ? bytes : 16);
+    if (e == cudaErrorMemoryAllocation) {  // the parts' plans give theirs back
+      cudaGetLastError();
+      for (auto *m : parts)
+        if (m->device == dev && m->patch_bytes > 0) m->release_patches();
+      e = cudaMalloc(&q, bytes ? bytes : 16);
+    }
     if (e != cudaSuccess)
       return fail(e == cudaErrorMemoryAllocation ? AKB_ENOMEM : AKB_ECUDA,
                   std::string("cudaMalloc: ") + cudaGetErrorString(e));

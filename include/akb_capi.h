@@ -560,6 +560,9 @@ int akb_bounds_checked(void);
  * checks: which 0 connectivity [n][E] (internal order), 1 slot positions
  * [n][E], 2 CSR offsets [N + 1] */
 int akb_model_debug_write_index(akb_model *model, int which, int64_t position, int32_t value);
+/* for tests: device bytes a model can have, as on a smaller device, in calls of
+ * this thread (0: no limit); what exceeds it fails with AKB_ENOMEM */
+int akb_debug_limit_device_bytes(int64_t bytes);
 
 /* ---- serving: many solves resident on one GPU ---------------------------- */
 /* No reference counterpart (the reference runs one model per process).  A

@@ -253,3 +253,56 @@ def test_internal_force_of_stopped_instances(precision, fused):
         for f in FIELDS:
             a, c = getattr(b, f)()[b.instance_nodes(k)], getattr(alone, f)()
             assert np.abs(c).max() > 0 and np.array_equal(a, c), (k, f)
+
+
+@pytest.fixture
+def device_limit():
+    """limits the device bytes of this thread's models, as a smaller device"""
+    from akantu2_b200 import _capi
+
+    def limit(nbytes):
+        _capi.check(_capi.lib().akb_debug_limit_device_bytes(int(nbytes)))
+
+    yield limit
+    limit(0)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_without_memory_for_the_plan_the_two_kernels_step(device_limit, precision):
+    """a device with room for the model but not for the fused step's plan"""
+    mesh = akb.box_tet4(6)
+    full = gpu_model(mesh, [UNIT_ELASTIC], precision=precision)
+    assert full.getFusedStep()
+    device_limit(1)
+    with pytest.raises(akb.AkbError) as e:
+        gpu_model(mesh, [UNIT_ELASTIC], precision=precision)
+    assert e.value.name == "AKB_ENOMEM"
+    device_limit(full.getDeviceBytes() - 1)
+    m = gpu_model(mesh, [UNIT_ELASTIC], precision=precision)
+    assert not m.getFusedStep() and m.getDeviceBytes() < full.getDeviceBytes()
+    device_limit(0)
+    dt = 0.8 * full.getStableTimeStep()
+    for x in (full, m):
+        x.setNodal("velocity", sinusoidal_velocity(mesh.nodes, 0.03))
+        x.setTimeStep(dt)
+        x.solveStep(130)
+    _same([full, m])
+
+
+def test_the_plan_gives_its_memory_back(device_limit):
+    """what a model asks for later comes before its plan: the same steps go on
+    as two kernels"""
+    mesh = akb.box_tet4(6)
+    models = _pair(mesh, [UNIT_ELASTIC], "fp64")
+    for m in models:
+        m.solveStep(130)
+    device_limit(models[0].getDeviceBytes())
+    models[0].setIncrementTracking(True)
+    device_limit(0)
+    assert not models[0].getFusedStep()
+    models[1].setIncrementTracking(True)
+    for m in models:
+        m.solveStep(130)
+    _same(models)
+    a, b = (m.getPreviousDisplacement() for m in models)
+    assert np.array_equal(a, b)
