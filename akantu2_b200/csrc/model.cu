@@ -2496,41 +2496,45 @@ int akb_model_set_prescribed_velocity_ramp(akb_model *m, const int64_t *dofs, in
   cudaStream_t s = m->stream;
   AKB_CUDA(cudaStreamSynchronize(s));
   m->drop_graphs();
-  m->presc_count = 0;
   if (count == 0 && m->presc_dofs.empty()) return AKB_OK;
+  // everything that can fail comes before the marks of the dofs: a marked dof
+  // is written by the ramp alone.  Buffers are kept for the model's lifetime.
+  int64_t *ddofs = nullptr;
+  double *du0 = nullptr;
+  std::vector<double> u(nd), u0(count);  // starting displacement of the dofs
+  if (count > 0) {
+    AKB_CUDA(cudaMemcpyAsync(u.data(), m->u(), sizeof(double) * nd, cudaMemcpyDeviceToHost, s));
+    AKB_CUDA(cudaStreamSynchronize(s));
+    for (int64_t k = 0; k < count; ++k) u0[k] = u[dofs[k]];
+    if (!m->dpresc_acc) AKB_TRY(m->alloc(&m->dpresc_acc, sizeof(double)));
+    if (!m->dpresc_step) AKB_TRY(m->alloc(&m->dpresc_step, sizeof(int64_t)));
+    AKB_TRY(m->alloc(&ddofs, sizeof(int64_t) * count));
+    AKB_TRY(m->alloc(&du0, sizeof(double) * count));
+    AKB_CUDA(cudaMemcpyAsync(ddofs, dofs, sizeof(int64_t) * count, cudaMemcpyHostToDevice, s));
+    AKB_CUDA(cudaMemcpyAsync(du0, u0.data(), sizeof(double) * count, cudaMemcpyHostToDevice, s));
+  }
   // the dofs are blocked from now on, and marked as prescribed
   std::vector<uint8_t> mask(m->N);
   AKB_CUDA(cudaMemcpyAsync(mask.data(), m->dblocked, m->N, cudaMemcpyDeviceToHost, s));
   AKB_CUDA(cudaStreamSynchronize(s));
   for (uint8_t &x : mask) x &= (uint8_t)((1u << kPrescribedBit) - 1);
-  m->presc_dofs.assign(dofs, dofs + count);
-  for (int64_t k : m->presc_dofs)
+  std::vector<int64_t> marked(dofs, dofs + count);
+  for (int64_t k : marked)
     mask[k / m->dim] |= (uint8_t)((1u | 1u << kPrescribedBit) << (k % m->dim));
   AKB_CUDA(cudaMemcpyAsync(m->dblocked, mask.data(), m->N, cudaMemcpyHostToDevice, s));
-  AKB_CUDA(cudaStreamSynchronize(s));
-  if (count == 0) return AKB_OK;
-  // starting displacement of the dofs
-  std::vector<double> u(nd), u0(count);
-  AKB_CUDA(cudaMemcpyAsync(u.data(), m->u(), sizeof(double) * nd, cudaMemcpyDeviceToHost, s));
-  AKB_CUDA(cudaStreamSynchronize(s));
-  for (int64_t k = 0; k < count; ++k) u0[k] = u[dofs[k]];
-  // buffers are kept for the model's lifetime; a longer list reallocates
-  AKB_TRY(m->alloc(&m->dpresc_dofs, sizeof(int64_t) * count));
-  AKB_TRY(m->alloc(&m->dpresc_u0, sizeof(double) * count));
-  if (!m->dpresc_acc) {
-    AKB_TRY(m->alloc(&m->dpresc_acc, sizeof(double)));
-    AKB_TRY(m->alloc(&m->dpresc_step, sizeof(int64_t)));
-  }
-  AKB_CUDA(cudaMemcpyAsync(m->dpresc_dofs, dofs, sizeof(int64_t) * count, cudaMemcpyHostToDevice, s));
-  AKB_CUDA(cudaMemcpyAsync(m->dpresc_u0, u0.data(), sizeof(double) * count, cudaMemcpyHostToDevice, s));
-  AKB_CUDA(cudaMemsetAsync(m->dpresc_acc, 0, sizeof(double), s));
-  AKB_CUDA(cudaMemsetAsync(m->dpresc_step, 0, sizeof(int64_t), s));
-  AKB_CUDA(cudaStreamSynchronize(s));
+  m->presc_dofs.swap(marked);
   m->presc_count = count;
-  m->presc_vmax = v_max;
-  m->presc_ramp = ramp_steps;
-  m->presc_ahead = false;
-  m->predicted = false;
+  if (count > 0) {
+    m->dpresc_dofs = ddofs;
+    m->dpresc_u0 = du0;
+    m->presc_vmax = v_max;
+    m->presc_ramp = ramp_steps;
+    m->presc_ahead = false;
+    m->predicted = false;
+    AKB_CUDA(cudaMemsetAsync(m->dpresc_acc, 0, sizeof(double), s));
+    AKB_CUDA(cudaMemsetAsync(m->dpresc_step, 0, sizeof(int64_t), s));
+  }
+  AKB_CUDA(cudaStreamSynchronize(s));
   return AKB_OK;
 }
 

@@ -306,3 +306,30 @@ def test_the_plan_gives_its_memory_back(device_limit):
     _same(models)
     a, b = (m.getPreviousDisplacement() for m in models)
     assert np.array_equal(a, b)
+
+
+def test_a_ramp_that_cannot_be_set_leaves_the_model_as_it_was(device_limit):
+    """without memory for its buffers the call fails; the steps that follow are
+    those of the model without it, or with the ramp it had"""
+    mesh = akb.box_tet4(6)
+    top = np.isclose(mesh.nodes[:, 2], 1.0)
+    for earlier in (False, True):
+        models = []
+        for failing in (True, False):
+            m = gpu_model(mesh, [UNIT_ELASTIC], precision="fp64")
+            m.setNodal("velocity", sinusoidal_velocity(mesh.nodes, 0.03))
+            m.setNodal("blocked_dofs", blocked_face(mesh.nodes))
+            m.setTimeStep(0.8 * m.getStableTimeStep())
+            if earlier:
+                m.setPrescribedVelocityRamp(top, 1, 1e-2, 10)
+            m.solveStep(5)
+            if failing:
+                device_limit(1)
+                with pytest.raises(akb.AkbError):
+                    m.setPrescribedVelocityRamp(top, 0, 5e-2, 20)
+                device_limit(0)
+            m.solveStep(130)
+            models.append(m)
+        for f in FIELDS + ("getBlockedDOFs",):
+            a, b = (getattr(m, f)() for m in models)
+            assert np.array_equal(a, b), (earlier, f)
