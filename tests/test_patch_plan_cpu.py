@@ -57,3 +57,40 @@ def test_regular_grids_are_cut_between_their_planes():
     8^2 x 9 ... elements that touch it"""
     patches, elements, nodes, slots = _check(akb.box_hex8(15), 512)
     assert patches == 8 and elements == 16 ** 3 and nodes == 9 ** 3 and slots == 8 * 512
+
+
+@pytest.mark.parametrize("cells,lengths", [((60, 60, 2), (1, 1, 1)), ((80, 12, 5), (1, 1, 1)),
+                                           ((9, 9, 9), (1, 30, 4))])
+@pytest.mark.parametrize("max_own", [27, 125, 216])
+def test_stretched_cells_are_cut_like_cubic_ones(cells, lengths, max_own):
+    """patches hold as many cells along each axis whatever their lengths: the same
+    number of patches and of elements evaluated, a twentieth apart"""
+    cubic = _check(akb.box_tet4(*cells, lengths=[c / 10 for c in cells]), max_own)
+    stretched = _check(akb.box_tet4(*cells, lengths=lengths), max_own)
+    for a, b in zip(stretched[:2], cubic[:2]):
+        assert abs(a - b) <= b / 20
+
+
+def test_stretched_instances_of_a_batch():
+    """each instance of a batch by its own cells"""
+    plate = akb.box_tet4(30, 30, 2)
+    cube = akb.box_tet4(7)
+    alone = _check(akb.box_tet4(30, 30, 2, lengths=(3.0, 3.0, 0.2)), 125)[1] + _check(cube, 125)[1]
+    both = akb.Mesh(3, np.concatenate([plate.nodes, cube.nodes]),
+                    np.concatenate([plate.connectivity, cube.connectivity + plate.getNbNodes()]),
+                    "_tetrahedron_4")
+    got = _check(both, 125, [plate.getNbNodes(), cube.getNbNodes()])[1]
+    assert abs(got - alone) <= alone / 20
+
+
+@pytest.mark.parametrize("n,max_own", [(5, 27), (9, 125), (9, 216)])
+def test_plan_of_an_unstructured_mesh(n, max_own):
+    """a Delaunay mesh of scattered points: uneven valences, no planes"""
+    from scipy.spatial import Delaunay
+    points = np.random.default_rng(n).uniform(0, 1, (n ** 3, 3))
+    tets = Delaunay(points).simplices
+    volume = np.linalg.det(points[tets[:, 1:]] - points[tets[:, :1]])
+    tets[volume < 0] = tets[volume < 0][:, [0, 2, 1, 3]]
+    mesh = akb.Mesh(3, points, tets.astype(np.int32), "_tetrahedron_4")
+    patches, elements, nodes, slots = _check(mesh, max_own)
+    assert patches >= n ** 3 / max_own and elements >= len(tets) and slots > 0
