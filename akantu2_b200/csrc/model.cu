@@ -1108,9 +1108,49 @@ int reduce_to_host(akb_model *m, const double *x, int64_t n, bool op_min, double
 
 // ---- plan of the fused step ------------------------------------------------
 
+// Whether a plan of so many patches and evaluated elements (those on a border
+// counted in each patch), whose largest patch needs smem bytes, steps faster
+// than the two kernels.
+//
+// Tetrahedra: the time of either form in us from constants fitted to 200
+// measured meshes (cubes, plates, bars, Delaunay meshes, batches; mean error 7
+// per cent).  An SM steps through its patches resident ones at a time, each round
+// with a latency, each element with a time that grows when fewer blocks than
+// the kernel is built for are resident; the two kernels have a time per element
+// and, beyond 100 MB, per byte.  The plan must win by a twentieth: the few
+// meshes the fit has on the wrong side differ by less.  Two kernels / fused:
+// 1000 cubes of 1^3, mixed, 5.3 / 7.8, 4000 6.1 / 25.6, 2000 of 3^3 17.4 / 20.8, 300
+// of 4^3 9.5 / 5.9; Delaunay, mixed, 54 k 10.8 / 6.6, 429 k, one block per SM, 22.0
+// / 24.7, 1.4 M, two, 71.8 / 73.7; 1000 x 8 x 8 cells neohookean 18.6 / 18.6.
+//
+// Hexahedra: the elements of an SM within half as many again as the largest
+// box of the rule below has.  Triangles: up to four patches per SM, two of 6
+// points (mixed 400 x 20 x 2, 606 patches, 10.3, two kernels 9.7; FP64 1000 x 5 x 2,
+// 502 patches, 8.9 / 10.6).
+bool patches_pay(int et, int rule, int law, bool mixed, int64_t E, int64_t patches,
+                 int64_t evaluated, size_t smem) {
+  const double sms = (double)kPatchSms;
+  const double rounds = std::ceil((double)patches / sms);  // patches of an SM
+  const double work = rounds * (double)evaluated / (double)patches;  // and their elements
+  if (et == AKB_TRIANGLE_6) return rounds <= (rule ? 2. : 4.);
+  if (et == AKB_HEXAHEDRON_8) return work <= 250.;
+  const double built = mixed ? 3. : 2.;
+  const double resident = std::min(built, std::max(1., std::floor(233472. / (double)(smem + 1024))));
+  const double rate = std::min(built, rounds) / std::min(resident, rounds);
+  const bool neo = law == LAW_NEOHOOKEAN;
+  const double element = mixed ? (neo ? 3.1e-3 : 2.6e-3) : (neo ? 12.5e-3 : 3.15e-3);
+  const double fused = (mixed ? 3.0 : 2.7) * std::ceil(rounds / resident) + element * work * rate;
+  const double beyond = std::max(0., (mixed ? 190. : 270.) * (double)E - 100e6);
+  const double two = mixed ? 6.1 + 33.3e-6 * (double)E + 0.116e-6 * beyond
+                           : (neo ? 8.2 : 7.0) + (neo ? 65e-6 : 60.7e-6) * (double)E +
+                                 0.0575e-6 * beyond;
+  return fused <= 0.95 * two;
+}
+
 // Owned nodes of a patch at most, s per edge; 0 where the two-kernel step is
-// the faster one.  Regular boxes are assumed: the rule also sizes the plan's
-// memory before there is a mesh.
+// the faster one for any plan (the plan itself is looked at once it is built).
+// Regular boxes are assumed: the rule also sizes the plan's memory before there
+// is a mesh.
 //
 // Tetrahedra and hexahedra: a patch evaluates about ((s + 1) / s)^3 times its
 // share of the elements, so large meshes take the largest patch that leaves
@@ -1150,7 +1190,7 @@ int patch_nodes(int et, int rule, int law, int precision, int64_t N, int64_t E, 
       const double slabs = std::ceil(planes / s - 1e-6), side = std::ceil(planes / slabs - 1e-6);
       // resident blocks per SM, fewer with the slots of 6 points
       const double patches = ninst * slabs * slabs;
-      if (patches > sms * (rule ? 2. : mixed ? 4. : 3.)) break;
+      if (patches > sms * (rule ? 2. : mixed ? 4. : 3.)) break;  // as in patches_pay
       const double cells = std::floor((side + 1.) / 2.) + 1.;  // that its node planes touch
       const double rounds = std::ceil(std::ceil(2. * cells * cells / 32.) * (rule ? 6. : 3.) / 6.);
       if (least == 0. || rounds < least || (rounds == least && patches <= sms)) {
@@ -1174,7 +1214,11 @@ int patch_nodes(int et, int rule, int law, int precision, int64_t N, int64_t E, 
       best = s;
     }
   }
-  return best * best * best;
+  // no patch reaches across two instances of a batch
+  const int own = best * best * best;
+  if (tet && !patches_pay(et, rule, law, mixed, E, std::max<int64_t>(ninst, N / own), E, 0))
+    return 0;
+  return own;
 }
 
 // rows of the per-element tables the fused kernel reads and the size of one
@@ -1300,8 +1344,12 @@ int finish_patches(akb_model *m, PatchTask &task) {
   const int points = m->et == AKB_TRIANGLE_6 ? m->nq : 1;  // slot arrays
   pa.smem = patch_smem(m->dim, plan.max_local, plan.max_slots * points, t.value);
   if (pa.smem + kPatchStageSmem > kPatchMaxSmem) return AKB_OK;
+  int64_t evaluated = 0;
+  for (const PatchHead &h : plan.head) evaluated += h.n_elem;
   PatchCaps need;
   need.patches = (int64_t)plan.head.size();
+  if (!patches_pay(m->et, m->rule, gr.law, mixed, m->E, need.patches, evaluated, pa.smem))
+    return AKB_OK;
   need.nodes = (int64_t)plan.nodes.size();
   need.elems = (int64_t)plan.elems.size();
   const PatchRoom room = patch_room(need, m->N, m->nn, t);

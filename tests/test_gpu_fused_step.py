@@ -333,3 +333,21 @@ def test_a_ramp_that_cannot_be_set_leaves_the_model_as_it_was(device_limit):
         for f in FIELDS + ("getBlockedDOFs",):
             a, b = (getattr(m, f)() for m in models)
             assert np.array_equal(a, b), (earlier, f)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("cells,count,fused", [(1, 100, True), (1, 2000, False), (2, 2000, False),
+                                               (4, 300, True)])
+def test_batches_of_tiny_instances_step_as_two_kernels(precision, cells, count, fused):
+    """an instance is a patch at least: many of a few elements are rounds of
+    nearly empty blocks"""
+    b = akb.BatchModel([akb.box_tet4(cells)] * count)
+    b.addMaterial("elastic", rho=1.0, E=1.0, nu=0.3)
+    b.initFull(precision=precision)
+    assert b.getFusedStep() == fused
+
+
+@pytest.mark.parametrize("cells,fused", [((100, 100), True), ((400, 20), False)])
+def test_triangles_whose_patches_are_not_resident_step_as_two_kernels(cells, fused):
+    m = gpu_model(akb.square_tri6(*cells), [UNIT_PLASTIC], precision="mixed")
+    assert m.getFusedStep() == fused
