@@ -1268,33 +1268,41 @@ int64_t patch_bytes(int et, int rule, int law, int precision, int64_t N, int64_t
   return (int64_t)patch_room(c, N, nodes_per_element(et), t).bytes;
 }
 
-// Builds the plan on a thread of its own while initFull goes on with the
-// device (it only reads the host arrays it is given, which outlive it).
+// Builds the plan on a thread of its own while initFull goes on (it only reads
+// the host arrays it is given, which outlive it): the cut into patches beside
+// initFull's own lists, the rest beside its work on the device.
 struct PatchTask {
   PatchMesh mesh;
   PatchCaps caps;
+  PatchCut cut;
   PatchPlan plan;
   std::vector<int32_t> mat;
-  bool wanted = false, ok = false;
-  std::thread worker;
+  bool wanted = false, ok = false;  // without host memory the two kernels step
+  std::thread first, second;
   ~PatchTask() { wait(); }
   void wait() {
-    if (worker.joinable()) worker.join();
+    if (second.joinable()) second.join();
+    if (first.joinable()) first.join();
   }
-  void build() {
+  template <class F> void go(std::thread &t, const F &f) {
+    auto run = [this, f] {
+      try {
+        ok = f();
+      } catch (const std::exception &) {
+        ok = false;
+      }
+    };
     try {
-      ok = build_patches(mesh, caps, plan);
+      t = std::thread(run);
     } catch (const std::exception &) {
-      ok = false;  // out of host memory or threads: the two-kernel step runs
+      run();  // no thread to be had
     }
   }
 };
 
 // starts the plan where the model may have one: a single law group of an
 // element type and law with a fused kernel, of a size it is the faster at
-void start_patches(akb_model *m, const std::vector<int32_t> &conn_soa,
-                   const std::vector<int32_t> &ptr, const std::vector<int32_t> &pos,
-                   PatchTask &task) {
+void start_patches(akb_model *m, PatchTask &task) {
 #ifdef AKB_BOUNDS_CHECK
   return;
 #endif
@@ -1310,25 +1318,40 @@ void start_patches(akb_model *m, const std::vector<int32_t> &conn_soa,
   pm.N = m->N;
   pm.E = m->E;
   pm.X = m->X.data();
-  pm.conn = conn_soa.data();
-  pm.ptr = ptr.data();
-  pm.pos = pos.data();
+  pm.elements = m->conn.data();
   pm.inst_off = m->inst_node_off.data();
   pm.ninst = m->ninst;
   task.caps = patch_caps(m->dim, m->N, m->E, m->ninst, pm.max_own);
-  try {
-    if (gr.nmat > 1) {
+  task.wanted = true;
+  task.go(task.first, [&task] {
+    cut_patches(task.mesh, task.cut);
+    return true;
+  });
+}
+
+// the rest of the plan, from the connectivity and the slots
+void continue_patches(akb_model *m, const std::vector<int32_t> &conn_soa,
+                      const std::vector<int32_t> &ptr, const std::vector<int32_t> &pos,
+                      PatchTask &task) {
+  if (!task.wanted) return;
+  PatchMesh &pm = task.mesh;
+  pm.conn = conn_soa.data();
+  pm.ptr = ptr.data();
+  pm.pos = pos.data();
+  if (m->groups[0].nmat > 1) {
+    try {
       task.mat.resize(m->E);
-      for (int64_t ie = 0; ie < m->E; ++ie) task.mat[ie] = m->mat_user[m->perm[ie]];
-      pm.mat = task.mat.data();
+    } catch (const std::exception &) {
+      task.wanted = false;
+      return;
     }
-    task.wanted = true;
-    task.worker = std::thread([&task] { task.build(); });
-  } catch (const std::bad_alloc &) {
-    task.wanted = false;
-  } catch (const std::exception &) {
-    task.build();  // no thread to be had
+    for (int64_t ie = 0; ie < m->E; ++ie) task.mat[ie] = m->mat_user[m->perm[ie]];
+    pm.mat = task.mat.data();
   }
+  task.go(task.second, [&task] {
+    if (task.first.joinable()) task.first.join();
+    return task.ok && build_patches(task.mesh, task.cut, task.caps, task.plan);
+  });
 }
 
 // The finished plan's arrays on the device.  The model can do without them:
@@ -1741,9 +1764,12 @@ int akb_model_init_full(akb_model *m, int method, int precision) {
     m->pdl = law == LAW_ELASTIC ||
              (law == LAW_NEOHOOKEAN && (E <= 148 * 32 || E > 148 * 4 * 32));
   }
+  std::vector<int32_t> conn_soa, ptr, ent, pos;  // (outlive the plan's threads)
+  PatchTask patches;
+  start_patches(m, patches);
   std::vector<int64_t> iperm(E);  // user element -> internal element
   for (int64_t ie = 0; ie < E; ++ie) iperm[m->perm[ie]] = ie;
-  std::vector<int32_t> conn_soa((size_t)nn * E);
+  conn_soa.resize((size_t)nn * E);
   for (int64_t ie = 0; ie < E; ++ie)
     for (int a = 0; a < nn; ++a) conn_soa[(size_t)a * E + ie] = m->conn[m->perm[ie] * nn + a];
   // node -> slot CSR.  A node's slots follow the reference's scatter order of
@@ -1754,8 +1780,9 @@ int akb_model_init_full(akb_model *m, int method, int precision) {
   // gather reads its forces contiguously.  ent: the slots of each node in
   // the order of the lumped-mass assembly, which runs over all elements of
   // the type in user order (solid_mechanics_model_mass.cc:115-128).
-  std::vector<int32_t> ptr(N + 1, 0), ent((size_t)E * nn), pos((size_t)E * nn);
-  PatchTask patches;
+  ptr.resize(N + 1);
+  ent.resize((size_t)E * nn);
+  pos.resize((size_t)E * nn);
   for (int64_t ie = 0; ie < E; ++ie)
     for (int a = 0; a < nn; ++a) ptr[conn_soa[(size_t)a * E + ie] + 1]++;
   for (int64_t i = 0; i < N; ++i) ptr[i + 1] += ptr[i];
@@ -1766,7 +1793,7 @@ int akb_model_init_full(akb_model *m, int method, int precision) {
       for (int64_t ie = mt.e_begin; ie < mt.e_begin + mt.e_count; ++ie)
         for (int a = 0; a < nn; ++a) pos[(size_t)a * E + ie] = fill[conn_soa[(size_t)a * E + ie]]++;
     }
-    start_patches(m, conn_soa, ptr, pos, patches);
+    continue_patches(m, conn_soa, ptr, pos, patches);
     std::copy(ptr.begin(), ptr.end() - 1, fill.begin());
     for (int64_t e = 0; e < E; ++e) {
       const int64_t ie = iperm[e];
@@ -3459,6 +3486,7 @@ int akb_patch_plan_check(int et, const double *nodes, int64_t N, const int32_t *
   pm.N = N;
   pm.E = E;
   pm.X = nodes;
+  pm.elements = conn;
   pm.inst_off = node_offsets;
   pm.ninst = nb_instances;
   pm.max_own = max_own;
@@ -3480,7 +3508,9 @@ int akb_patch_plan_check(int et, const double *nodes, int64_t N, const int32_t *
     caps.patches = N;
     caps.nodes = caps.elems = std::numeric_limits<int32_t>::max();
     PatchPlan plan;
-    if (!build_patches(pm, caps, plan)) return fail(AKB_EUNSUPPORTED, "no plan for this mesh");
+    PatchCut cut;
+    cut_patches(pm, cut);
+    if (!build_patches(pm, cut, caps, plan)) return fail(AKB_EUNSUPPORTED, "no plan for this mesh");
     if (!check_patches(pm, plan)) return fail(AKB_ESTATE, "the plan is wrong");
     stats[0] = (int64_t)plan.head.size();
     stats[1] = 0;

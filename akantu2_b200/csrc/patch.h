@@ -8,6 +8,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <memory>
 #include <vector>
 
 #include "presc.h"
@@ -36,18 +37,49 @@ struct PatchOwn {
   uint16_t local, valence;
 };
 
-// what the builder reads, all in host memory (internal element order)
+// What the builder reads, all in host memory.  cut_patches reads the first
+// part only, build_patches all of it but elements.
 struct PatchMesh {
   int D = 3, NN = 4;
   int64_t N = 0, E = 0;
-  const double *X = nullptr;         // [N][D]
+  const double *X = nullptr;          // [N][D]
+  const int32_t *elements = nullptr;  // [E][NN], in any order
+  const int64_t *inst_off = nullptr;  // node offsets of the instances [ninst + 1]
+  int ninst = 1;
+  int max_own = 512;                  // owned nodes of a patch at most
+  // in the internal element order
   const int32_t *conn = nullptr;     // [NN][E]
   const int32_t *ptr = nullptr;      // node -> slot CSR offsets [N + 1]
   const int32_t *pos = nullptr;      // [NN][E] CSR position of each slot
-  const int64_t *inst_off = nullptr; // node offsets of the instances [ninst + 1]
-  int ninst = 1;
   const int32_t *mat = nullptr;      // material of each element [E], or null
-  int max_own = 512;                 // owned nodes of a patch at most
+};
+
+// the patches' owned nodes: patch p has those of nodes [b, e), ascending
+struct PatchRange {
+  int64_t b, e;
+  int inst;
+};
+struct PatchCut {
+  std::vector<PatchRange> patch;
+  std::vector<int32_t> nodes;  // [N]
+  std::vector<int32_t> owner;  // [N] patch of each node
+};
+void cut_patches(const PatchMesh &m, PatchCut &cut);
+
+// an array that is not written when it is made (its pages are then touched
+// first by the threads that fill it)
+template <class T> struct PlanArray {
+  std::unique_ptr<T[]> p;
+  size_t n = 0;
+  void resize(size_t count) {
+    p.reset(new T[count]);
+    n = count;
+  }
+  size_t size() const { return n; }
+  T *data() { return p.get(); }
+  const T *data() const { return p.get(); }
+  T &operator[](size_t k) { return p[k]; }
+  const T &operator[](size_t k) const { return p[k]; }
 };
 
 // Every node is owned by one patch.  Patch element k has its nodes' local
@@ -59,10 +91,10 @@ struct PatchMesh {
 struct PatchPlan {
   int NNP = 4;
   std::vector<PatchHead> head;
-  std::vector<int32_t> nodes;
-  std::vector<PatchOwn> own;  // N entries
-  std::vector<int32_t> elems;
-  std::vector<uint16_t> conn, slot;
+  PlanArray<int32_t> nodes;
+  PlanArray<PatchOwn> own;  // N entries
+  PlanArray<int32_t> elems;
+  PlanArray<uint16_t> conn, slot;
   int max_local = 0;  // nodes of a patch at most
   int max_slots = 0;  // slots of a patch at most (largest valence x owned nodes)
 };
@@ -75,7 +107,8 @@ struct PatchCaps {
 PatchCaps patch_caps(int D, int64_t N, int64_t E, int ninst, int max_own);
 
 // false: the mesh does not fit (capacities, 16-bit local indices)
-bool build_patches(const PatchMesh &m, const PatchCaps &caps, PatchPlan &plan);
+bool build_patches(const PatchMesh &m, const PatchCut &cut, const PatchCaps &caps,
+                   PatchPlan &plan);
 
 // every index of the plan is in range and names what it should: each node
 // owned once, each slot of an owned node written by one element, in order

@@ -7,47 +7,105 @@
 #include <array>
 #include <atomic>
 #include <cmath>
+#include <condition_variable>
 #include <exception>
+#include <functional>
+#include <mutex>
 #include <thread>
+#include <utility>
 
 namespace akb {
 namespace {
 
-struct Range {
-  int64_t b, e;
-  int inst;
-};
+using Range = PatchRange;
 
+// Threads for the plan of a mesh: its initialisation goes on meanwhile, and
+// others may be at theirs.
 int host_threads(int64_t work) {
-  const int64_t t = std::min<int64_t>(std::max(1u, std::thread::hardware_concurrency()), 16);
-  return (int)std::max<int64_t>(1, std::min<int64_t>(t, work / 16000));
+  const int64_t most = std::min<int64_t>(std::max(1u, std::thread::hardware_concurrency()), 8);
+  return (int)std::min<int64_t>(most, 1 + work / 8000);
 }
 
-// f(first, last, t) on contiguous chunks of [0, n), one per thread; a chunk
-// whose thread cannot be started runs here, an exception is rethrown here
-template <class F> void chunked(int64_t n, int threads, const F &f) {
-  std::vector<std::exception_ptr> error(threads);
-  auto part = [&](int t) {
-    try {
-      f(n * t / threads, n * (t + 1) / threads, t);
-    } catch (...) {
-      error[t] = std::current_exception();
-    }
-  };
-  std::vector<std::thread> pool;
-  pool.reserve(threads);
-  for (int t = 1; t < threads; ++t) {
-    try {
-      pool.emplace_back(part, t);
-    } catch (...) {
-      part(t);
+// The plan's threads, started once: its phases are too short to start threads
+// for each.  Every phase is cut into parts() parts whatever number of threads
+// could be started.
+class Workers {
+  using Part = std::function<void(int)>;
+
+ public:
+  explicit Workers(int parts) : parts_(parts), error_(parts) {
+    pool_.reserve(parts - 1);
+    for (int t = 1; t < parts; ++t) {
+      try {
+        pool_.emplace_back([this] { serve(); });
+      } catch (const std::exception &) {
+        break;  // the parts run on the threads there are
+      }
     }
   }
-  part(0);
-  for (auto &p : pool) p.join();
-  for (auto &x : error)
-    if (x) std::rethrow_exception(x);
-}
+  ~Workers() {
+    {
+      std::lock_guard<std::mutex> lock(mu_);
+      stop_ = true;
+    }
+    wake_.notify_all();
+    for (auto &p : pool_) p.join();
+  }
+  int parts() const { return parts_; }
+  // f(first, last, part) on contiguous pieces of [0, n); an exception of one is
+  // rethrown here
+  template <class F> void chunked(int64_t n, const F &f) {
+    run([&](int t) { f(n * t / parts_, n * (t + 1) / parts_, t); });
+  }
+
+ private:
+  void run(const Part &part) {
+    {
+      std::lock_guard<std::mutex> lock(mu_);
+      part_ = &part;
+      next_ = 0;
+      left_ = parts_;
+    }
+    if (!pool_.empty()) wake_.notify_all();
+    std::unique_lock<std::mutex> lock(mu_);
+    take_parts(lock);
+    done_.wait(lock, [this] { return left_ == 0; });
+    part_ = nullptr;
+    for (auto &x : error_)
+      if (x) std::rethrow_exception(std::exchange(x, nullptr));
+  }
+  void take_parts(std::unique_lock<std::mutex> &lock) {
+    while (part_ && next_ < parts_) {
+      const int t = next_++;
+      const Part &part = *part_;
+      lock.unlock();
+      std::exception_ptr error;
+      try {
+        part(t);
+      } catch (...) {
+        error = std::current_exception();
+      }
+      lock.lock();
+      error_[t] = error;
+      if (--left_ == 0) done_.notify_one();
+    }
+  }
+  void serve() {
+    std::unique_lock<std::mutex> lock(mu_);
+    while (!stop_) {
+      wake_.wait(lock, [this] { return stop_ || (part_ && next_ < parts_); });
+      take_parts(lock);
+    }
+  }
+  const int parts_;
+  std::vector<std::exception_ptr> error_;
+  std::vector<std::thread> pool_;
+  std::mutex mu_;
+  std::condition_variable wake_, done_;
+  const Part *part_ = nullptr;
+  int next_ = 0, left_ = 0;
+  bool stop_ = false;
+};
 
 // Node planes of a box of n nodes with extents ext, were it a regular grid:
 // the spacing h solves prod(ext_a / h + 1) = n.
@@ -82,11 +140,11 @@ std::vector<std::array<double, 3>> cell_scales(const PatchMesh &m) {
     const int64_t e = m.E / samples * k + m.E % samples * k / samples;
     const int64_t inst = m.ninst <= 1 ? 0
                                       : std::upper_bound(m.inst_off, m.inst_off + m.ninst,
-                                                         (int64_t)m.conn[e]) - m.inst_off - 1;
+                                                         (int64_t)m.elements[e * m.NN]) - m.inst_off - 1;
     for (int a = 0; a < m.D; ++a) {
       double lo = 0., hi = 0.;
       for (int c = 0; c < m.NN; ++c) {
-        const double x = m.X[(int64_t)m.conn[(int64_t)c * m.E + e] * m.D + a];
+        const double x = m.X[(int64_t)m.elements[e * m.NN + c] * m.D + a];
         lo = c == 0 ? x : std::min(lo, x);
         hi = c == 0 ? x : std::max(hi, x);
       }
@@ -112,72 +170,163 @@ struct Item {
 struct Box {
   double lo[3], hi[3];
 };
+// nodes [b, e) of the bisection, ascending, and their bounds
+struct Part {
+  Range r;
+  Box box;
+};
 
-// Splits it[b, e) into leaves of at most max_own nodes.  The axis split is the
-// one with the most patch edges in its extent, at the fraction that leaves
-// whole patch edges on both sides, moved to the nearest plane of equal
-// coordinates: regular grids are cut between their planes, into boxes.  box:
-// bounds of the nodes (the halves take the split coordinate as theirs).
-void bisect(const PatchMesh &m, std::vector<Item> &it, int64_t b, int64_t e, const Box &box,
-            int inst, int depth, std::vector<Range> &out) {
-  const int64_t n = e - b;
-  if (n <= m.max_own) {
-    if (n > 0) out.push_back({b, e, inst});
-    return;
-  }
-  double ext[3];
-  for (int a = 0; a < m.D; ++a) ext[a] = box.hi[a] - box.lo[a];
+// Splits a part of more than max_own nodes in two.  The axis split is the one
+// with the most patch edges in its extent, at the fraction that leaves whole
+// patch edges on both sides, moved to the nearest plane of equal coordinates:
+// regular grids are cut between their planes, into boxes.  The half that the cut
+// does not touch takes the split coordinate as its bound.  The coordinate of that
+// rank is found from a histogram and the nodes of one of its bins, and the nodes
+// are moved once, in order (through tmp): 5 passes of a few ns per node, where a
+// selection by swaps took 27.
+void split(const PatchMesh &m, Item *it, Item *tmp, const Part &p, Part half[2]) {
+  constexpr int kBins = 256;
+  const int64_t b = p.r.b, e = p.r.e, n = e - b;
+  double ext[3] = {0., 0., 0.};
+  for (int a = 0; a < m.D; ++a) ext[a] = p.box.hi[a] - p.box.lo[a];
   const double edge = std::floor(std::pow((double)m.max_own, 1. / m.D) + 1e-9);
   const double h = grid_spacing(ext, m.D, (double)n);
   int axis = 0;
   for (int a = 1; a < m.D; ++a)
     if (ext[a] > ext[axis]) axis = a;
   const int64_t parts =
-      std::max<int64_t>(2, (int64_t)std::ceil((ext[axis] / h + 1.) / edge - 1e-3));
-  int64_t at = b + n * (parts / 2) / parts;
-  at = std::min(std::max(at, b + 1), e - 1);
-  std::nth_element(it.begin() + b, it.begin() + at, it.begin() + e,
-                   [axis](const Item &x, const Item &y) {
-                     return x.x[axis] < y.x[axis] || (x.x[axis] == y.x[axis] && x.node < y.node);
-                   });
+      std::max<int64_t>(2, (int64_t)std::ceil(std::min((ext[axis] / h + 1.) / edge, (double)n) - 1e-3));
+  int64_t at = n * (parts / 2) / parts;
+  at = std::min(std::max<int64_t>(at, 1), n - 1);
+  // bins of equal width
+  const double lo = p.box.lo[axis], per = ext[axis] > 0. ? (kBins - 1) / ext[axis] : 0.;
+  auto bin = [=](const Item &i) {
+    const double k = (i.x[axis] - lo) * per;
+    return k > 0. ? (int)std::min(k, (double)(kBins - 1)) : 0;
+  };
+  int64_t count[kBins] = {0};
+  for (int64_t k = b; k < e; ++k) ++count[bin(it[k])];
+  int at_bin = 0;
+  int64_t below = 0;
+  while (below + count[at_bin] <= at) below += count[at_bin++];
+  std::vector<double> x;
+  x.reserve(count[at_bin]);
+  for (int64_t k = b; k < e; ++k)
+    if (bin(it[k]) == at_bin) x.push_back(it[k].x[axis]);
+  std::nth_element(x.begin(), x.begin() + (at - below), x.end());
   // the plane of equal coordinates around the split point is [p0, p1)
-  const double c = it[at].x[axis];
-  const int64_t p0 = std::partition(it.begin() + b, it.begin() + at,
-                                    [=](const Item &i) { return i.x[axis] < c; }) - it.begin();
-  const int64_t p1 = std::partition(it.begin() + at, it.begin() + e,
-                                    [=](const Item &i) { return i.x[axis] == c; }) - it.begin();
-  if (p0 > b || p1 < e) at = (p0 > b && (at - p0 <= p1 - at || p1 == e)) ? p0 : p1;
-  // the nodes next to the cut bound the halves
-  Box half[2] = {box, box};
-  half[0].hi[axis] = box.lo[axis];
-  for (int64_t k = b; k < at; ++k) half[0].hi[axis] = std::max(half[0].hi[axis], it[k].x[axis]);
-  half[1].lo[axis] = at == p1 ? box.hi[axis] : c;
-  if (at == p1)
-    for (int64_t k = at; k < e; ++k) half[1].lo[axis] = std::min(half[1].lo[axis], it[k].x[axis]);
-  if (depth > 0 && n > 50000) {
-    std::vector<Range> list[2];
-    chunked(2, 2, [&](int64_t, int64_t, int t) {
-      bisect(m, it, t ? at : b, t ? e : at, half[t], inst, depth - 1, list[t]);
-    });
-    for (auto &x : list) out.insert(out.end(), x.begin(), x.end());
-  } else {
-    bisect(m, it, b, at, half[0], inst, 0, out);
-    bisect(m, it, at, e, half[1], inst, 0, out);
+  const double c = x[at - below];
+  int64_t p0 = below, p1 = below;
+  for (const double v : x) {
+    p0 += v < c;
+    p1 += v <= c;
   }
+  const bool cut = p0 > 0 || p1 < n;
+  if (cut) at = (p0 > 0 && (at - p0 <= p1 - at || p1 == n)) ? p0 : p1;
+  const bool with_plane = at == p1;  // the plane belongs to the first half
+  Item *first = it + b, *second = tmp + b;
+  double hi0 = p.box.lo[axis], lo1 = p.box.hi[axis];
+  int64_t taken = 0;
+  for (int64_t k = b; k < e; ++k) {
+    const Item i = it[k];
+    const double v = i.x[axis];
+    const bool left = cut ? (with_plane ? v <= c : v < c) : taken < at;
+    if (left) {
+      hi0 = std::max(hi0, v);
+      *first++ = i;
+      ++taken;
+    } else {
+      lo1 = std::min(lo1, v);
+      *second++ = i;
+    }
+  }
+  std::copy(tmp + b, second, first);
+  half[0] = half[1] = p;
+  half[0].r.e = half[1].r.b = b + taken;
+  half[0].box.hi[axis] = hi0;
+  half[1].box.lo[axis] = with_plane ? lo1 : c;
 }
 
-// the whole of one instance
-void bisect_all(const PatchMesh &m, std::vector<Item> &it, int64_t b, int64_t e, int inst,
-                int depth, std::vector<Range> &out) {
-  if (b == e) return;
-  Box box;
-  for (int a = 0; a < 3; ++a) box.lo[a] = box.hi[a] = it[b].x[a];
-  for (int64_t k = b; k < e; ++k)
-    for (int a = 0; a < m.D; ++a) {
-      box.lo[a] = std::min(box.lo[a], it[k].x[a]);
-      box.hi[a] = std::max(box.hi[a], it[k].x[a]);
+// the leaves of a part, of at most max_own nodes, in order
+void bisect(const PatchMesh &m, Item *it, Item *tmp, const Part &p, std::vector<Range> &out) {
+  if (p.r.e - p.r.b <= m.max_own) {
+    if (p.r.e > p.r.b) out.push_back(p.r);
+    return;
+  }
+  Part half[2];
+  split(m, it, tmp, p, half);
+  bisect(m, it, tmp, half[0], out);
+  bisect(m, it, tmp, half[1], out);
+}
+
+// the nodes' patches, instance by instance: every leaf's nodes in idx, ascending
+std::vector<Range> leaves_of(const PatchMesh &m, Workers &w, int32_t *idx) {
+  const int64_t N = m.N;
+  std::unique_ptr<Item[]> it(new Item[N]), tmp(new Item[N]);
+  const std::vector<std::array<double, 3>> scale = cell_scales(m);
+  std::vector<std::vector<Part>> part(w.parts());
+  std::vector<Part> all;
+  w.chunked(N, [&](int64_t i0, int64_t i1, int) {
+    int64_t inst = std::upper_bound(m.inst_off, m.inst_off + m.ninst, i0) - m.inst_off - 1;
+    for (int64_t i = i0; i < i1; ++i) {
+      while (inst + 1 < m.ninst && i >= m.inst_off[inst + 1]) ++inst;
+      for (int a = 0; a < 3; ++a) {
+        const double x = a < m.D ? m.X[i * m.D + a] * scale[inst][a] : 0.;
+        // (what is no number has an order, and no difference overflows)
+        it[i].x[a] = std::isnan(x) ? 0. : std::min(std::max(x, -1e150), 1e150);
+      }
+      it[i].node = (int32_t)i;
     }
-  bisect(m, it, b, e, box, inst, depth, out);
+  });
+  auto join = [&] {
+    all.clear();
+    for (auto &p : part) {
+      all.insert(all.end(), p.begin(), p.end());
+      p.clear();
+    }
+  };
+  w.chunked(m.ninst, [&](int64_t k0, int64_t k1, int t) {
+    for (int64_t k = k0; k < k1; ++k) {
+      const Range r = {m.inst_off[k], m.inst_off[k + 1], (int)k};
+      if (r.b == r.e) continue;
+      Box box;
+      for (int a = 0; a < 3; ++a) box.lo[a] = box.hi[a] = it[r.b].x[a];
+      for (int64_t i = r.b; i < r.e; ++i)
+        for (int a = 0; a < m.D; ++a) {
+          box.lo[a] = std::min(box.lo[a], it[i].x[a]);
+          box.hi[a] = std::max(box.hi[a], it[i].x[a]);
+        }
+      part[t].push_back({r, box});
+    }
+  });
+  join();
+  // level by level until there is a part for every thread, then part by part
+  for (size_t before = 0; w.parts() > 1 && all.size() != before &&
+                          all.size() < 4 * (size_t)w.parts();) {
+    before = all.size();
+    w.chunked((int64_t)all.size(), [&](int64_t k0, int64_t k1, int t) {
+      for (int64_t k = k0; k < k1; ++k) {
+        if (all[k].r.e - all[k].r.b <= m.max_own) {
+          part[t].push_back(all[k]);
+          continue;
+        }
+        Part half[2];
+        split(m, it.get(), tmp.get(), all[k], half);
+        part[t].insert(part[t].end(), half, half + 2);
+      }
+    });
+    join();
+  }
+  std::vector<std::vector<Range>> list(w.parts());
+  w.chunked((int64_t)all.size(), [&](int64_t k0, int64_t k1, int t) {
+    for (int64_t k = k0; k < k1; ++k) bisect(m, it.get(), tmp.get(), all[k], list[t]);
+  });
+  std::vector<Range> leaves;
+  for (auto &x : list) leaves.insert(leaves.end(), x.begin(), x.end());
+  w.chunked(N, [&](int64_t i0, int64_t i1, int) {
+    for (int64_t i = i0; i < i1; ++i) idx[i] = it[i].node;
+  });
+  return leaves;
 }
 
 }  // namespace
@@ -196,60 +345,38 @@ PatchCaps patch_caps(int D, int64_t N, int64_t E, int ninst, int max_own) {
   return c;
 }
 
-bool build_patches(const PatchMesh &m, const PatchCaps &caps, PatchPlan &plan) {
+void cut_patches(const PatchMesh &m, PatchCut &cut) {
+  Workers w(host_threads(std::max(m.N, m.E)));
+  cut.nodes.resize(m.N);
+  cut.owner.resize(m.N);
+  cut.patch = leaves_of(m, w, cut.nodes.data());
+  w.chunked((int64_t)cut.patch.size(), [&](int64_t p0, int64_t p1, int) {
+    for (int64_t p = p0; p < p1; ++p)
+      for (int64_t k = cut.patch[p].b; k < cut.patch[p].e; ++k)
+        cut.owner[cut.nodes[k]] = (int32_t)p;
+  });
+}
+
+bool build_patches(const PatchMesh &m, const PatchCut &cut, const PatchCaps &caps,
+                   PatchPlan &plan) {
   const int NN = m.NN;
   const int64_t N = m.N, E = m.E;
   plan = PatchPlan();
   plan.NNP = NN <= 4 ? 4 : 8;
   const int NNP = plan.NNP;
-  if (N == 0 || E == 0 || m.max_own < 1) return false;
-  // ---- patches of nodes, instance by instance
-  std::vector<int32_t> idx(N);
-  std::vector<Range> leaves;
-  const int nt = host_threads(N);
-  {
-    std::vector<Item> it(N);
-    const std::vector<std::array<double, 3>> scale = cell_scales(m);
-    chunked(N, nt, [&](int64_t i0, int64_t i1, int) {
-      int64_t inst = 0;
-      for (int64_t i = i0; i < i1; ++i) {
-        while (inst + 1 < m.ninst && i >= m.inst_off[inst + 1]) ++inst;
-        for (int a = 0; a < m.D; ++a) it[i].x[a] = m.X[i * m.D + a] * scale[inst][a];
-        for (int a = m.D; a < 3; ++a) it[i].x[a] = 0.;
-        it[i].node = (int32_t)i;
-      }
-    });
-    if (m.ninst <= 1) {
-      bisect_all(m, it, 0, N, 0, nt > 1 ? 4 : 0, leaves);
-    } else {
-      std::vector<std::vector<Range>> part(nt);
-      chunked(m.ninst, nt, [&](int64_t k0, int64_t k1, int t) {
-        for (int64_t k = k0; k < k1; ++k)
-          bisect_all(m, it, m.inst_off[k], m.inst_off[k + 1], (int)k, 0, part[t]);
-      });
-      for (auto &p : part) leaves.insert(leaves.end(), p.begin(), p.end());
-    }
-    chunked(N, nt, [&](int64_t i0, int64_t i1, int) {
-      for (int64_t i = i0; i < i1; ++i) idx[i] = it[i].node;
-    });
-  }
+  const std::vector<Range> &leaves = cut.patch;
+  const std::vector<int32_t> &idx = cut.nodes, &owner = cut.owner;
   const int64_t P = (int64_t)leaves.size();
-  if (P > caps.patches) return false;
-  std::vector<int32_t> owner(N);
-  chunked(P, nt, [&](int64_t p0, int64_t p1, int) {
-    for (int64_t p = p0; p < p1; ++p) {
-      std::sort(idx.begin() + leaves[p].b, idx.begin() + leaves[p].e);
-      for (int64_t k = leaves[p].b; k < leaves[p].e; ++k) owner[idx[k]] = (int32_t)p;
-    }
-  });
+  if (P == 0 || P > caps.patches) return false;
+  Workers w(host_threads(std::max(N, E)));
   // ---- elements of each patch: those with a node it owns, ascending
-  const int et = host_threads(E);
+  const int et = w.parts();
   struct Pair {
     int32_t patch, element;
   };
   std::vector<std::vector<Pair>> pairs(et);
   std::vector<std::vector<int32_t>> count(et, std::vector<int32_t>(P + 1, 0));
-  chunked(E, et, [&](int64_t e0, int64_t e1, int t) {
+  w.chunked(E, [&](int64_t e0, int64_t e1, int t) {
     std::vector<Pair> &list = pairs[t];
     std::vector<int32_t> &c = count[t];
     list.reserve((size_t)((e1 - e0) * 1.7) + 64);
@@ -288,24 +415,25 @@ bool build_patches(const PatchMesh &m, const PatchCaps &caps, PatchPlan &plan) {
     total += (n + 31) / 32 * 32;
     if (total > caps.elems) return false;
   }
-  plan.elems.assign(total, 0);
-  chunked(et, et, [&](int64_t t0, int64_t t1, int) {
+  plan.elems.resize(total);
+  w.chunked(et, [&](int64_t t0, int64_t t1, int) {
     for (int64_t t = t0; t < t1; ++t)
       for (const Pair &x : pairs[t]) plan.elems[count[t][x.patch]++] = x.element;
   });
   // ---- local indices
-  plan.conn.assign((size_t)total * NNP, 0);
-  plan.slot.assign((size_t)total * NNP, kNoSlot);
+  plan.conn.resize((size_t)total * NNP);
+  plan.slot.resize((size_t)total * NNP);
   std::vector<std::vector<int32_t>> local(P);
   plan.own.resize(N);
   std::atomic<bool> ok{true};
-  chunked(P, et, [&](int64_t p0, int64_t p1, int) {
+  w.chunked(P, [&](int64_t p0, int64_t p1, int) {
     // node -> 1 + its index in the patch, 0 outside; cleared after each patch
     std::vector<int32_t> where(N, 0);
     std::vector<int32_t> corner, mine;
     for (int64_t p = p0; p < p1 && ok; ++p) {
       PatchHead &h = plan.head[p];
-      const int32_t *el = plan.elems.data() + (size_t)h.chunk0 * 32;
+      int32_t *el = plan.elems.data() + (size_t)h.chunk0 * 32;
+      std::fill(el + h.n_elem, el + (h.n_elem + 31) / 32 * 32, 0);
       const int32_t *mine0 = idx.data() + leaves[p].b;
       std::vector<int32_t> &nodes = local[p];
       nodes.reserve(2 * h.n_own + h.n_elem);
@@ -353,6 +481,9 @@ bool build_patches(const PatchMesh &m, const PatchCaps &caps, PatchPlan &plan) {
       }
       uint16_t *lc = plan.conn.data() + (size_t)h.chunk0 * 32 * NNP;
       uint16_t *sc = plan.slot.data() + (size_t)h.chunk0 * 32 * NNP;
+      const size_t padded = (size_t)(h.n_elem + 31) / 32 * 32 * NNP;
+      std::fill(lc, lc + padded, (uint16_t)0);
+      std::fill(sc, sc + padded, kNoSlot);
       for (int a = 0; a < NN; ++a) {
         const int32_t *pos = m.pos + (int64_t)a * E;
         for (int k = 0; k < h.n_elem; ++k) {
@@ -377,8 +508,10 @@ bool build_patches(const PatchMesh &m, const PatchCaps &caps, PatchPlan &plan) {
   }
   if (nodes > caps.nodes) return false;
   plan.nodes.resize(nodes);
-  for (int64_t p = 0; p < P; ++p)
-    std::copy(local[p].begin(), local[p].end(), plan.nodes.begin() + plan.head[p].node0);
+  w.chunked(P, [&](int64_t p0, int64_t p1, int) {
+    for (int64_t p = p0; p < p1; ++p)
+      std::copy(local[p].begin(), local[p].end(), plan.nodes.data() + plan.head[p].node0);
+  });
   return true;
 }
 
