@@ -306,6 +306,7 @@ struct akb_model {
   void *patch_mem = nullptr;  // its arrays
   size_t patch_bytes = 0;
   bool patch_ready = false, patch_on = false;
+  bool plan_left_out = false;  // leave_out_plan
   // persistent multi-step kernel: 0 never (default: on B200 the 100-step
   // graphs of the two-kernel step are faster at every measured size), 1 for
   // small single-group meshes, 2 whenever the model allows it
@@ -1258,16 +1259,6 @@ PatchRoom patch_room(const PatchCaps &c, int64_t N, int nn, const PatchTables &t
   return r;
 }
 
-// device bytes of a plan at most (the same for any mesh of these sizes)
-int64_t patch_bytes(int et, int rule, int law, int precision, int64_t N, int64_t E, int ninst) {
-  const PatchTables t = patch_tables(et, law, precision, et == AKB_TRIANGLE_6 && rule ? 6 : 3);
-  if (t.rows == 0 || N == 0 || E == 0) return 0;
-  const int own = patch_nodes(et, rule, law, precision, N, E, ninst);
-  if (own == 0) return 0;
-  const PatchCaps c = patch_caps(dim_of(et), N, E, ninst, own);
-  return (int64_t)patch_room(c, N, nodes_per_element(et), t).bytes;
-}
-
 // Builds the plan on a thread of its own while initFull goes on (it only reads
 // the host arrays it is given, which outlive it): the cut into patches beside
 // initFull's own lists, the rest beside its work on the device.
@@ -1306,7 +1297,7 @@ void start_patches(akb_model *m, PatchTask &task) {
 #ifdef AKB_BOUNDS_CHECK
   return;
 #endif
-  if (m->groups.size() != 1 || m->N == 0 || m->E == 0) return;
+  if (m->plan_left_out || m->groups.size() != 1 || m->N == 0 || m->E == 0) return;
   const Group &gr = m->groups[0];
   for (auto &mt : m->mats)
     if (mt.c33) return;
@@ -1437,6 +1428,19 @@ int finish_patches(akb_model *m, PatchTask &task) {
 }
 
 }  // namespace
+
+// device bytes of a plan at most (the same for any mesh of these sizes)
+int64_t akb::plan_device_bytes(int et, int rule, int law, int precision, int64_t N, int64_t E,
+                               int ninst) {
+  const PatchTables t = patch_tables(et, law, precision, et == AKB_TRIANGLE_6 && rule ? 6 : 3);
+  if (t.rows == 0 || N == 0 || E == 0) return 0;
+  const int own = patch_nodes(et, rule, law, precision, N, E, ninst);
+  if (own == 0) return 0;
+  const PatchCaps c = patch_caps(dim_of(et), N, E, ninst, own);
+  return (int64_t)patch_room(c, N, nodes_per_element(et), t).bytes;
+}
+
+void akb::leave_out_plan(akb_model *m) { m->plan_left_out = true; }
 
 /* ------------------------------------------------------------------------ */
 /* C ABI                                                                    */
@@ -2525,7 +2529,7 @@ int akb_estimate_device_bytes(int et, int rule, int64_t N, int64_t E, int law, i
   if (law == LAW_NEOHOOKEAN && d == 2) t += r(8 * E * nq);  // plane-stress C33
   // mixed hexahedra: the adjugate table of a mesh of parallelepipeds
   if (precision == AKB_PRECISION_MIXED && et == AKB_HEXAHEDRON_8) t += r(4 * 10 * E);
-  t += patch_bytes(et, rule, law, precision, N, E, 1);
+  t += plan_device_bytes(et, rule, law, precision, N, E, 1);
   *bytes = t;
   return AKB_OK;
 }
@@ -2541,8 +2545,8 @@ int akb_estimate_batch_device_bytes(int et, int rule, int64_t N, int64_t E, int 
   // stop steps; the material table and the step counter
   *bytes += r(4 * N) + 3 * r(4 * E) + 3 * r(8 * ni) + r(8 * (ni + 1)) +
             r((int64_t)sizeof(MatParams) * ni) + r(8);
-  *bytes += patch_bytes(et, rule, law, precision, N, E, nb_instances) -
-            patch_bytes(et, rule, law, precision, N, E, 1);
+  *bytes += plan_device_bytes(et, rule, law, precision, N, E, nb_instances) -
+            plan_device_bytes(et, rule, law, precision, N, E, 1);
   return AKB_OK;
 }
 

@@ -66,7 +66,10 @@ struct Job {
   std::string mat_type, mat_params;
   double dt_factor = 0.8;
   double *u_out = nullptr, *v_out = nullptr;
-  int64_t est_bytes = 0;  // this request's own footprint (reported)
+  // this request's own footprint (reported): without the plan of the fused
+  // step until it is admitted with one
+  int64_t est_bytes = 0;
+  bool plan = false;
   // run state
   Phase phase = QUEUED;
   akb_model *m = nullptr;
@@ -91,6 +94,7 @@ struct Cohort {
   std::vector<Job *> jobs;
   int et = 0, rule = 0, precision = 0, dim = 3, law = 0;
   int64_t N = 0, E = 0, est_bytes = 0;
+  bool plan = false;
   akb_model *m = nullptr;
   void *stream = nullptr;
   cudaEvent_t ev[2] = {nullptr, nullptr};
@@ -148,6 +152,8 @@ struct akb_server {
   void retire_cohort(Cohort *c);
   void complete(Job *j);  // caller holds mu
   int64_t cohort_bytes(const Cohort *c) const;
+  void admit_alone(Job *j);  // caller holds mu
+  bool with_plan(int64_t E, int64_t steps, int64_t bytes) const;  // caller holds mu
   Cohort *take_cohort();  // caller holds mu; the head is batchable
 };
 
@@ -206,12 +212,37 @@ void akb_server::complete(Job *j) {
   cv_work.notify_all();
 }
 
+// without the plan of the fused step
 int64_t akb_server::cohort_bytes(const Cohort *c) const {
   int64_t b = 0;
   if (akb_estimate_batch_device_bytes(c->et, c->rule, c->N, c->E, (int)c->jobs.size(), c->law,
                                       c->precision, &b) != AKB_OK)
     return std::numeric_limits<int64_t>::max() / 4;
-  return b;
+  return b - akb::plan_device_bytes(c->et, c->rule, c->law, c->precision, c->N, c->E,
+                                    (int)c->jobs.size());
+}
+
+// Whether a solve of so many steps that needs so many bytes with the plan of the
+// fused step gets one: the plan lengthens its preparation by what 40 to 600 of
+// its steps save (tetrahedra 3 k 40, 48 k 100 to 140, 162 k and 912 k 500 to 600;
+// plastic triangles 8 k 160, 20 k 350; hexahedra 8 k 180; batches of 115 k 200 to 270,
+// of 3 M 340), and takes no memory that another waits for.
+bool akb_server::with_plan(int64_t E, int64_t steps, int64_t bytes) const {
+  if (steps < (E <= 50000 ? 200 : 600)) return false;
+  int64_t waiting = 0;
+  for (const Job *q : queue) waiting += q->est_bytes;
+  return reserved + bytes + waiting <= cfg.device_bytes;
+}
+
+void akb_server::admit_alone(Job *j) {
+  const int64_t plan = akb::plan_device_bytes(j->et, j->rule, j->law, j->precision, j->N, j->E, 1);
+  j->plan = plan > 0 && with_plan(j->E, j->steps, j->est_bytes + plan);
+  if (j->plan) j->est_bytes += plan;
+  reserved += j->est_bytes;
+  active++;
+  n_building++;
+  j->phase = BUILDING;
+  j->t_admit = now();
 }
 
 // the queue's head and the queued requests that can share its batch, in
@@ -249,6 +280,12 @@ Cohort *akb_server::take_cohort() {
     it = queue.erase(it);
   }
   c->est_bytes = cohort_bytes(c);
+  int64_t steps = 0;
+  for (const Job *j : c->jobs) steps = std::max(steps, j->steps);
+  const int64_t plan = akb::plan_device_bytes(c->et, c->rule, c->law, c->precision, c->N, c->E,
+                                              (int)c->jobs.size());
+  c->plan = plan > 0 && with_plan(c->E, steps, c->est_bytes + plan);
+  if (c->plan) c->est_bytes += plan;
   return c;
 }
 
@@ -263,6 +300,7 @@ void akb_server::build(Job *j) {
   }
   if (rc == AKB_OK) rc = akb_model_add_material(j->m, j->mat_type.c_str(), j->mat_params.c_str());
   if (rc == AKB_OK && j->rule) rc = akb_model_set_quadrature_rule(j->m, j->rule);
+  if (rc == AKB_OK && !j->plan) akb::leave_out_plan(j->m);
   if (rc == AKB_OK) rc = akb_model_init_full(j->m, AKB_EXPLICIT_LUMPED_MASS, j->precision);
   const int64_t nd = j->N * j->dim;
   if (rc == AKB_OK && !j->u0.empty())
@@ -349,6 +387,7 @@ void akb_server::build_cohort(Cohort *c) {
   for (int k = 0; k < ni; ++k) mat_of[k] = k;
   if (rc == AKB_OK) rc = akb_batch_set_instance_materials(c->m, mat_of.data());
   if (rc == AKB_OK && c->rule) rc = akb_model_set_quadrature_rule(c->m, c->rule);
+  if (rc == AKB_OK && !c->plan) akb::leave_out_plan(c->m);
   if (rc == AKB_OK) rc = akb_model_init_full(c->m, AKB_EXPLICIT_LUMPED_MASS, c->precision);
   if (rc == AKB_OK && any_u)
     rc = akb_model_set_nodal(c->m, AKB_DISPLACEMENT, u0.data(), nd * (int64_t)sizeof(double));
@@ -521,11 +560,7 @@ void akb_server::builder_loop() {
           j = c->jobs[0];
           delete c;
           c = nullptr;
-          reserved += j->est_bytes;
-          active++;
-          n_building++;
-          j->phase = BUILDING;
-          j->t_admit = now();
+          admit_alone(j);
         } else {
           reserved += c->est_bytes;
           const double t = now();
@@ -539,11 +574,7 @@ void akb_server::builder_loop() {
       } else {
         j = queue.front();
         queue.pop_front();
-        reserved += j->est_bytes;
-        active++;
-        n_building++;
-        j->phase = BUILDING;
-        j->t_admit = now();
+        admit_alone(j);
       }
     }
     if (fin)
@@ -775,6 +806,7 @@ int akb_server_submit(akb_server *s, const akb_request *r, int64_t *id) {
     delete j;
     return rc;
   }
+  j->est_bytes -= akb::plan_device_bytes(j->et, j->rule, law, j->precision, j->N, j->E, 1);
   if (j->est_bytes > s->cfg.device_bytes) {
     const int64_t need = j->est_bytes;
     delete j;

@@ -472,7 +472,9 @@ int akb_model_stream(const akb_model *model, void **stream);
 int akb_model_device_bytes(const akb_model *model, int64_t *bytes);
 /* upper bound of the device memory akb_model_init_full allocates for a mesh
  * of one material of law `law` (0 elastic, 1 neohookean, 2 plastic); used
- * for admission by memory footprint */
+ * for admission by memory footprint.  With the plan of the fused step at its
+ * capacity: the plan is smaller above 8 MB, and a model is initialised without it
+ * where it does not fit */
 int akb_estimate_device_bytes(int element_type, int quadrature_rule, int64_t nb_nodes,
                               int64_t nb_elements, int law, int precision, int64_t *bytes);
 /* the same for a batch of nb_instances meshes with N nodes and E elements in
@@ -568,7 +570,9 @@ int akb_debug_limit_device_bytes(int64_t bytes);
 /* No reference counterpart (the reference runs one model per process).  A
  * server admits submitted solves in arrival order while their estimated
  * device memory (akb_estimate_device_bytes, akb_estimate_batch_device_bytes)
- * fits in its budget and fewer than max_active are resident.  Solves of at
+ * fits in its budget and fewer than max_active are resident.  The plan of the
+ * fused step counts only where a solve gets one: of 200 steps or more (600 above
+ * 50,000 elements), while every queued solve fits beside it.  Solves of at
  * most batch_max_request_elements elements are admitted in batches: the
  * queue's head with every queued solve of the same element type, quadrature
  * rule, law and precision (limits above) becomes one batch model whose
@@ -632,7 +636,8 @@ typedef struct {
 } akb_server_stats;
 
 int akb_server_create(const akb_server_config *config, akb_server **server);
-/* copies the request's inputs; AKB_ENOMEM if it can never fit the budget */
+/* copies the request's inputs; AKB_ENOMEM if it can never fit the budget (without
+ * the fused step's plan) */
 int akb_server_submit(akb_server *server, const akb_request *request, int64_t *id);
 /* up to `capacity` completions, waiting at most wait_seconds for the first */
 int akb_server_poll(akb_server *server, akb_completion *out, int capacity, int *count,

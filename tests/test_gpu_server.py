@@ -199,3 +199,39 @@ def test_batch_estimate_bounds_the_allocation():
              _capi.TRIANGLE_6), 0, b.mesh.getNbNodes(), b.mesh.getNbElement(), len(meshes),
             law, 0 if prec == "fp64" else 1, ctypes.byref(est)))
         assert used <= est.value <= used + 8192, (meshes[0].element_type, prec, used, est.value)
+
+
+@pytest.mark.parametrize("steps,plan", [(100, False), (200, True)])
+@pytest.mark.parametrize("count", [1, 3])
+def test_the_fused_steps_plan_is_optional(steps, plan, count):
+    """a budget for the solves but not for the plan of the fused step admits
+    them all at once; the plan is built for enough steps where there is room;
+    the same results"""
+    rng = np.random.default_rng(21)
+    req = _request(0, rng)
+    req["mesh"] = akb.box_tet4(8)
+    x = req["mesh"].nodes
+    req.update(velocity=0.01 * np.sin(3 * x), blocked=np.zeros(x.shape, dtype=np.uint8),
+               material={k: v for k, v in UNIT_ELASTIC.items() if k != "name"}, steps=steps,
+               precision="fp64")
+    full = akb.Server.estimate_bytes(req["mesh"], req["material"], "fp64")
+    m = akb.SolidMechanicsModel(req["mesh"])
+    m.addMaterial("elastic", rho=1.0, E=1.0, nu=0.3)
+    m.initFull()
+    assert m.getFusedStep()
+    u, v = _alone(req)
+    reserved = {}
+    for budget in (full - 1, 8 * full):
+        srv = akb.Server(max_active=8, device_bytes=count * budget, batching=False)
+        outs = dict(srv.submit(req["mesh"], req["material"], steps, velocity=req["velocity"],
+                               blocked=req["blocked"], want_velocity=True) for _ in range(count))
+        done = srv.drain(timeout=60)
+        srv.close()
+        assert len(done) == count and all(c["status"] == 0 for c in done)
+        for c in done:
+            assert np.array_equal(outs[c["id"]]["displacement"], u)
+            assert np.array_equal(outs[c["id"]]["velocity"], v)
+        reserved[budget] = {c["device_bytes"] for c in done}
+    small = full // 2  # without the plan
+    assert all(r < small for r in reserved[full - 1]) or count > 1
+    assert all((r == full) == plan for r in reserved[8 * full])
