@@ -2690,6 +2690,26 @@ int akb_model_autotune(akb_model *m, int repeats) {
     if (check(cudaEventElapsedTime(ms, e0, e1), "cudaEventElapsedTime")) *ms /= repeats;
     return rc == AKB_OK;
   };
+  // whole steps are timed as they run, replayed from a graph (unless the model
+  // has none): launched one by
+  // one their launches hide what a dependent launch costs (FP64 neohookean
+  // hexahedra, 20^3, us per step without / with dependent launches: one by one
+  // the latter is shorter, in graphs 12.7 / 14.0)
+  auto time_steps = [&](const std::function<cudaError_t()> &steps, float *ms) {
+    if (m->graph_steps == 0) return time_it(steps, ms);
+    cudaGraph_t graph = nullptr;
+    cudaGraphExec_t exec = nullptr;
+    if (!check(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal), "autotune capture"))
+      return false;
+    const cudaError_t launched = steps();
+    check(cudaStreamEndCapture(s, &graph), "autotune capture");
+    check(launched, "autotune launch");
+    if (rc == AKB_OK) check(cudaGraphInstantiate(&exec, graph, 0), "autotune graph");
+    if (graph) cudaGraphDestroy(graph);
+    const bool ok = rc == AKB_OK && time_it([&] { return cudaGraphLaunch(exec, s); }, ms);
+    if (exec) cudaGraphExecDestroy(exec);
+    return ok;
+  };
   // the stress evaluations of the timed launches update C33 in place: they
   // get a copy
   int64_t c33_n = 0;
@@ -2697,8 +2717,12 @@ int akb_model_autotune(akb_model *m, int repeats) {
     if (gr.c33) c33_n = std::max(c33_n, gr.e_count * m->nq);
   double *t_c33 = nullptr;
   if (c33_n > 0) AKB_CUDA(m->device_malloc_needed((void **)&t_c33, sizeof(double) * c33_n));
+  // timed alone a kernel lets no copy of itself start early; in a whole step it
+  // lets the next kernel, as the step does
+  bool whole_step = false;
   auto scratch_args = [&](const Group &gr) {
     GroupArgs ps = group_args(m, gr, false);
+    ps.trigger = whole_step && m->trigger > 0 && (m->trigger & 1);
     if (gr.c33) ps.c33 = t_c33;
     if (gr.law == LAW_PLASTIC) {
       ps.sig = t_sig;
@@ -2806,7 +2830,8 @@ int akb_model_autotune(akb_model *m, int repeats) {
     }
   }
   if (rc == AKB_OK) {
-    const int flags = NU_CORRECT | NU_PREDICT | (m->fext_zero ? NU_FEXT_ZERO : 0);
+    const int flags = NU_CORRECT | NU_PREDICT | (m->fext_zero ? NU_FEXT_ZERO : 0) |
+                      (step_beyond_l2(m) ? NU_DOWN : 0);
     check(cudaMemcpyAsync(t_a, m->da, sizeof(double) * nd, cudaMemcpyDeviceToDevice, s), "copy");
     check(cudaMemcpyAsync(t_v, m->dv, sizeof(double) * nd, cudaMemcpyDeviceToDevice, s), "copy");
     // direct gather with 128 .. 1024 threads, staged gather with 128 .. 512,
@@ -2839,15 +2864,17 @@ int akb_model_autotune(akb_model *m, int repeats) {
   if (rc == AKB_OK) {
     m->trigger = -1;
     rc = find_trigger(m);
+    whole_step = true;
     const int flags = NU_CORRECT | NU_PREDICT | (m->fext_zero ? NU_FEXT_ZERO : 0) |
                       (m->trigger > 0 && (m->trigger & 2) ? NU_TRIGGER : 0) |
                       (step_beyond_l2(m) ? NU_DOWN : 0);
+    constexpr int kTimedSteps = 20;
     float ms[2] = {0.f, 0.f};
     for (int pdl = 0; pdl < 2 && rc == AKB_OK; ++pdl) {
       g.pdl = pdl;
       auto step = [&]() {
         cudaError_t e = cudaSuccess;
-        for (int r = 0; r < 8 && e == cudaSuccess; ++r) {
+        for (int r = 0; r < kTimedSteps && e == cudaSuccess; ++r) {
           for (auto &gr : m->groups)
             if (e == cudaSuccess) e = elem_launch(gr, gr.tune);
           if (e != cudaSuccess) break;
@@ -2862,7 +2889,7 @@ int akb_model_autotune(akb_model *m, int repeats) {
         }
         return e;
       };
-      time_it(step, &ms[pdl]);
+      time_steps(step, &ms[pdl]);
     }
     if (rc == AKB_OK) m->pdl = ms[1] < ms[0];
     g.pdl = m->pdl ? 1 : 0;
@@ -2879,12 +2906,12 @@ int akb_model_autotune(akb_model *m, int repeats) {
       pa.flags = flags;
       auto step = [&]() {
         cudaError_t e = cudaSuccess;
-        for (int r = 0; r < 8 && e == cudaSuccess; ++r) 
+        for (int r = 0; r < kTimedSteps && e == cudaSuccess; ++r)
           e = launch_patches(m, pa, scratch_args(m->groups[0]), pdl != 0);
         return e;
       };
       float t = 0.f;
-      if (!time_it(step, &t) || t >= best) continue;
+      if (!time_steps(step, &t) || t >= best) continue;
       best = t;
       m->patch_on = true;
       m->pdl = pdl != 0;
@@ -2892,6 +2919,7 @@ int akb_model_autotune(akb_model *m, int repeats) {
   }
   // the slot array again holds the forces of the current state, computed
   // with the chosen shapes
+  whole_step = false;
   for (auto &gr : m->groups)
     if (rc == AKB_OK) check(elem_launch(gr, gr.tune), "autotune launch");
   check(cudaStreamSynchronize(s), "cudaStreamSynchronize");
