@@ -269,6 +269,68 @@ template <int NQ_, class T_> struct PatchTri6 {
   }
 };
 
+// AKB_BOUNDS_CHECK builds check every index of the plan before it is used: the
+// ranges of a patch, the nodes it lists and owns, its elements' local indices
+// and slots.  What has an index out of range sets status bit 2 and is skipped.
+template <class EV>
+__device__ __forceinline__ bool patch_head_ok(const PatchArgs &pa, const GroupArgs &ps,
+                                              const PatchHead &h) {
+#ifdef AKB_BOUNDS_CHECK
+  const int64_t nod = ((int64_t)h.n_local * EV::D + 1) & ~(int64_t)1;
+  if (h.node0 >= 0 && h.n_local >= 0 && (int64_t)h.node0 + h.n_local <= pa.list_nodes &&
+      h.own0 >= 0 && h.n_own >= 0 && (int64_t)h.own0 + h.n_own <= ps.nb_nodes && h.chunk0 >= 0 &&
+      h.n_elem >= 0 && ((int64_t)h.chunk0 + (h.n_elem + 31) / 32) * 32 <= pa.list_elems &&
+      h.n_slot >= 0 && h.inst >= 0 && h.inst < pa.instances && h.mat < pa.materials &&
+      8 * nod + (int64_t)sizeof(typename EV::T) * h.n_slot * EV::kPoints * EV::D <=
+          (int64_t)pa.smem)
+    return true;
+  atomicOr(ps.status, ST_INDEX_RANGE);
+  return false;
+#else
+  (void)pa, (void)ps, (void)h;
+  return true;
+#endif
+}
+__device__ __forceinline__ bool patch_node_ok(const GroupArgs &ps, int64_t node) {
+#ifdef AKB_BOUNDS_CHECK
+  if (node >= 0 && node < ps.nb_nodes) return true;
+  atomicOr(ps.status, ST_INDEX_RANGE);
+  return false;
+#else
+  (void)ps, (void)node;
+  return true;
+#endif
+}
+__device__ __forceinline__ bool patch_own_ok(const GroupArgs &ps, const PatchHead &h,
+                                             const PatchOwn &o) {
+#ifdef AKB_BOUNDS_CHECK
+  if (o.node >= 0 && o.node < ps.nb_nodes && o.local < h.n_local &&
+      (int64_t)o.valence * h.n_own <= h.n_slot)
+    return true;
+  atomicOr(ps.status, ST_INDEX_RANGE);
+  return false;
+#else
+  (void)ps, (void)h, (void)o;
+  return true;
+#endif
+}
+template <int NN, class Chunk>
+__device__ __forceinline__ bool patch_element_ok(const PatchArgs &pa, const GroupArgs &ps,
+                                                 const PatchHead &h, const Chunk &ch,
+                                                 int64_t le) {
+#ifdef AKB_BOUNDS_CHECK
+  bool ok = le >= 0 && le < pa.e_count;
+#pragma unroll
+  for (int a = 0; a < NN; ++a)
+    ok = ok && ch.node(a) < h.n_local && (ch.slot(a) == kNoSlot || ch.slot(a) < h.n_slot);
+  if (!ok) atomicOr(ps.status, ST_INDEX_RANGE);
+  return ok;
+#else
+  (void)pa, (void)ps, (void)h, (void)ch, (void)le;
+  return true;
+#endif
+}
+
 // a chunk into the warp's shared buffer, 16 bytes per lane and pass
 template <int BYTES> __device__ __forceinline__ void stage_chunk(char *dst, const char *src) {
   const int lane = threadIdx.x & 31;
@@ -312,6 +374,7 @@ __global__ void __launch_bounds__(THREADS, MINB)
     return prescribe_block(pa.presc, pa.u_next, true);
   }
   const PatchHead h = pa.head[blockIdx.x];
+  if (!patch_head_ok<EV>(pa, ps, h)) return;
   const int32_t *nodes = pa.nodes + h.node0;
   const PatchOwn *own = pa.own + h.own0;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -347,8 +410,10 @@ __global__ void __launch_bounds__(THREADS, MINB)
   if constexpr (EARLY) {
     if (threadIdx.x < h.n_own) {
       o0 = own[threadIdx.x];
-      st0.m = pa.mass[o0.node];
-      st0.bl = pa.blocked[o0.node];
+      if (patch_own_ok(ps, h, o0)) {
+        st0.m = pa.mass[o0.node];
+        st0.bl = pa.blocked[o0.node];
+      }
     }
   }
   pdl_begin(trigger);
@@ -361,6 +426,7 @@ __global__ void __launch_bounds__(THREADS, MINB)
       copy_async_wait();
       if (flags & NU_PREDICT)
         for (int j = threadIdx.x; j < h.n_own * D; j += THREADS) {
+          if (!patch_own_ok(ps, h, own[j / D])) continue;
           const int64_t k = (int64_t)own[j / D].node * D + j % D;
           pa.u[k] = pa.u_next[k];
         }
@@ -371,12 +437,13 @@ __global__ void __launch_bounds__(THREADS, MINB)
 #pragma unroll
   for (int k = 0; k < U; ++k) {
     const int i = threadIdx.x + k * THREADS;
-    if (i < h.n_local)
+    if (i < h.n_local && patch_node_ok(ps, id[k]))
 #pragma unroll
       for (int c = 0; c < D; ++c) copy_async_8(us + i * D + c, pa.u + (int64_t)id[k] * D + c);
   }
   for (int i = threadIdx.x + U * THREADS; i < h.n_local; i += THREADS) {
     const int64_t n = nodes[i];
+    if (!patch_node_ok(ps, n)) continue;
 #pragma unroll
     for (int c = 0; c < D; ++c) copy_async_8(us + i * D + c, pa.u + n * D + c);
   }
@@ -390,11 +457,12 @@ __global__ void __launch_bounds__(THREADS, MINB)
     }
   };
   if constexpr (EARLY) {
-    if (threadIdx.x < h.n_own) load_state(o0.node, st0);
+    if (threadIdx.x < h.n_own && patch_own_ok(ps, h, o0)) load_state(o0.node, st0);
   } else {
     // the owned nodes' state, which the update reads last, into L2 meanwhile
     for (int i = threadIdx.x; i < h.n_own; i += THREADS) {
       const int64_t node = own[i].node;
+      if (!patch_node_ok(ps, node)) continue;
       prefetch_l2_line(pa.a + node * D);
       prefetch_l2_line(pa.v + node * D);
       prefetch_l2_line(pa.mass + node);
@@ -405,10 +473,11 @@ __global__ void __launch_bounds__(THREADS, MINB)
   constexpr int kWave = (int)kPatchSms * MINB;
   if (AHEAD && threadIdx.x == 32 && blockIdx.x + kWave < pa.npatch) {
     const PatchHead hn = pa.head[blockIdx.x + kWave];
-    auto fetch = [](const void *lo, const void *hi) {
+    const bool next_ok = patch_head_ok<EV>(pa, ps, hn);
+    auto fetch = [next_ok](const void *lo, const void *hi) {
       const uint64_t a = (uint64_t)__cvta_generic_to_global(lo) & ~(uint64_t)15;
       const uint64_t z = ((uint64_t)__cvta_generic_to_global(hi) + 15) & ~(uint64_t)15;
-      if (z > a)
+      if (z > a && next_ok)
         asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a), "r"((unsigned)(z - a))
                      : "memory");
     };
@@ -442,7 +511,7 @@ __global__ void __launch_bounds__(THREADS, MINB)
     int64_t le = 0;
     if (MULTI || pa.need_index) le = pa.elems[(int64_t)(h.chunk0 + c) * 32 + lane];
     const bool active = c * 32 + lane < h.n_elem;
-    if (!EV::kActive || active) {
+    if ((!EV::kActive || active) && patch_element_ok<EV::NN>(pa, ps, h, ch, le)) {
       if constexpr (MULTI) {
         const MatParams mpe = ps.mtab[ps.mslot[le]];
         EV::forces(pa, mpe, ps, us, ch, le, q, sl + q * plane);
@@ -461,8 +530,10 @@ __global__ void __launch_bounds__(THREADS, MINB)
     if (EARLY && i < THREADS) {
       o = o0;
       st = st0;
+      if (!patch_own_ok(ps, h, o)) continue;
     } else {
       o = own[i];
+      if (!patch_own_ok(ps, h, o)) continue;
       st.m = pa.mass[o.node];
       st.bl = pa.blocked[o.node];
       load_state(o.node, st);

@@ -792,9 +792,6 @@ int ensure_fint(akb_model *m) {
 }
 
 bool use_patches(const akb_model *m) {
-#ifdef AKB_BOUNDS_CHECK
-  return false;  // the bounds-checking build runs the checked two-kernel step only
-#endif
   return m->patch_ready && m->patch_on;
 }
 
@@ -1294,9 +1291,6 @@ struct PatchTask {
 // starts the plan where the model may have one: a single law group of an
 // element type and law with a fused kernel, of a size it is the faster at
 void start_patches(akb_model *m, PatchTask &task) {
-#ifdef AKB_BOUNDS_CHECK
-  return;
-#endif
   if (m->plan_left_out || m->groups.size() != 1 || m->N == 0 || m->E == 0) return;
   const Group &gr = m->groups[0];
   for (auto &mt : m->mats)
@@ -1424,6 +1418,13 @@ int finish_patches(akb_model *m, PatchTask &task) {
   m->patch_bytes = bytes;
   m->device_bytes += bytes;
   m->patch_ready = m->patch_on = true;
+#ifdef AKB_BOUNDS_CHECK
+  pa.list_nodes = need.nodes;
+  pa.list_elems = need.elems;
+  pa.instances = m->ninst;
+  pa.materials = (int)m->mats.size();
+  m->patch_on = false;  // the bounds-checking build runs it when asked to
+#endif
   return AKB_OK;
 }
 
@@ -3586,8 +3587,17 @@ int akb_model_debug_write_index(akb_model *m, int which, int64_t position, int32
   } else if (which == 2) {
     arr = m->dptr;
     n = m->N + 1;
+  } else if (which >= 3 && which <= 6 && m->patch_ready) {
+    const PatchArgs &pa = m->patch;
+    const int32_t *lists[4] = {(const int32_t *)pa.head, pa.nodes, (const int32_t *)pa.own,
+                               (const int32_t *)pa.tab};
+    const int64_t sizes[4] = {pa.npatch * (int64_t)(sizeof(PatchHead) / 4), pa.list_nodes,
+                              2 * m->N, 64 * (m->nn <= 4 ? 4 : 8) / 2};
+    arr = const_cast<int32_t *>(lists[which - 3]);
+    n = sizes[which - 3];
   } else {
-    return fail(AKB_EINVAL, "which is 0 (connectivity), 1 (slot positions) or 2 (CSR offsets)");
+    return fail(AKB_EINVAL, "which is 0 (connectivity), 1 (slot positions), 2 (CSR offsets) or, "
+                            "with a fused step, 3 to 6 (its plan)");
   }
   if (position < 0 || position >= n) return fail(AKB_EINVAL, "position out of range");
   AKB_CUDA(cudaMemcpyAsync(arr + position, &value, sizeof(int32_t), cudaMemcpyHostToDevice,

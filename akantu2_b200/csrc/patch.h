@@ -151,6 +151,10 @@ struct PatchArgs {
   int flags = 0;
   unsigned int *status = nullptr;
   PrescArgs presc;  // prescribed motion, written by an extra block
+#ifdef AKB_BOUNDS_CHECK
+  int64_t list_nodes = 0, list_elems = 0;  // entries of nodes and elems
+  int instances = 1, materials = 1;
+#endif
 };
 
 // fills the chunks: conn and slot [entries][NNP], and rows value rows of

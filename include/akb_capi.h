@@ -552,15 +552,19 @@ int akb_batch_get_time_steps(const akb_model *model, double *dt);
 /* ---- bounds-checking build ----------------------------------------------- */
 /* libakb_checked.so is this library built with AKB_BOUNDS_CHECK: its step
  * kernels check every index they read (node ids of the connectivity, slot
- * positions, each node's CSR slot range) before using it; an element or node
- * with an index out of range is skipped and sets bit 2 of the status word
- * (akb_model_get_status).  It stands in for a memory checker.  The persistent
- * kernel and the staged node gather are not used by it.  1 in that build. */
+ * positions, each node's CSR slot range; the fused step's plan) before using
+ * it; an element, node or patch with an index out of range is skipped and sets
+ * bit 2 of the status word (akb_model_get_status).  It stands in for a memory
+ * checker.  The persistent kernel and the staged node gather are not used by it,
+ * the fused step only where akb_model_set_fused_step asks for it.  1 in that
+ * build. */
 int akb_bounds_checked(void);
 /* bounds-checking build only (AKB_EUNSUPPORTED otherwise): overwrites one
  * entry of an index array on the device from the host, for tests of the
  * checks: which 0 connectivity [n][E] (internal order), 1 slot positions
- * [n][E], 2 CSR offsets [N + 1] */
+ * [n][E], 2 CSR offsets [N + 1]; of the fused step's plan, in words of 32 bits, 3
+ * the patches, 4 their node lists, 5 their owned nodes (node, then 16-bit local
+ * index and valence), 6 the first chunk's 16-bit local indices, then slots */
 int akb_model_debug_write_index(akb_model *model, int which, int64_t position, int32_t value);
 /* for tests: device bytes a model can have, as on a smaller device, in calls of
  * this thread (0: no limit); what exceeds it fails with AKB_ENOMEM */

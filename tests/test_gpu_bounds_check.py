@@ -85,3 +85,46 @@ def test_index_writes_need_the_checked_build():
     m.initFull()
     rc = _capi.lib().akb_model_debug_write_index(m._h, 0, 0, 5)
     assert _capi.ERRORS[rc] == "AKB_EUNSUPPORTED"
+
+
+FUSED = r"""
+cases = [(akb.box_tet4(4), EL, "fp64"), (akb.box_tet4(4), NEO, "mixed"),
+         (akb.box_hex8(4), NEO, "mixed"), (akb.square_tri6(5), PL, "mixed")]
+for mesh, mat, prec in cases:
+    N, n = mesh.getNbNodes(), mesh.connectivity.shape[1]
+    # a patch's first node, node count, first owned node, first chunk, element,
+    # slot and instance; a listed node; an owned node, its local index and valence
+    # (16 bits each); two local indices and two slots of the first chunk
+    words = 16 * (4 if n <= 4 else 8)
+    wrong = [(3, k, 1 << 24) for k in (0, 1, 2, 4, 5, 6, 7)] + [(3, 1, -1)]
+    wrong += [(4, 3, N), (4, 0, -5), (5, 2, N + 3), (5, 1, 0xfffe), (5, 3, 0xfffe << 16),
+              (6, 5, 0x00010fff), (6, words + 2, 0x0fff)]
+    for which, position, value in wrong:
+        m = model(mesh, mat, prec)
+        assert not m.getFusedStep()  # asked for in this build
+        m.setFusedStep(True)
+        m.solveStep(4)
+        assert m.getStatus() == 0
+        _capi.check(L.akb_model_debug_write_index(m._h, which, position, value))
+        m.solveStep(3)
+        st = m.getStatus()
+        assert st & 4, (mesh.element_type, prec, which, position, st)
+        del m
+    two, fused = model(mesh, mat, prec), model(mesh, mat, prec)
+    fused.setFusedStep(True)
+    for m in (two, fused):
+        m.solveStep(110)
+        assert m.getStatus() == 0
+    assert np.array_equal(two.getDisplacement(), fused.getDisplacement())
+    assert np.abs(two.getDisplacement()).max() > 0
+print("checked fused step OK")
+"""
+
+
+def test_bounds_checking_build_checks_the_fused_steps_plan():
+    env = dict(os.environ, AKB_BOUNDS_CHECK="1")
+    setup = CHILD[:CHILD.index("cases = [")]
+    r = subprocess.run([sys.executable, "-c", "ROOT = %r\n" % ROOT + setup + FUSED], env=env,
+                       capture_output=True, text=True, timeout=600)
+    assert r.returncode == 0, r.stdout + r.stderr
+    assert "checked fused step OK" in r.stdout
