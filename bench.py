@@ -254,12 +254,28 @@ def read_traffic(config, precision):
         return None
 
 
-def roofline_entry(kern_bytes, elem_ms, peak, peak_kind, traffic):
-    """the element-force kernel against the measured HBM peak: the formula's
-    algorithmic bytes per launch, and (when an ncu capture gave the kernel's
-    DRAM bytes per launch) the measured DRAM traffic per launch time"""
+def launches_per_step(fused):
+    """the element-force kernel and the node update (with the next predictor and
+    the next prescribed motion), or the fused step"""
+    return 1 if fused else 2
+
+
+def phases_per_step(phases, nsteps, fused):
+    """profileSteps' times (predictor, elements, nodes) of nsteps, each per step;
+    the fused step is one launch"""
+    ms = [p / nsteps for p in phases]
+    if fused:
+        return {"predictor": ms[0], "fused_step": ms[1]}
+    return {"predictor": ms[0], "element_forces": ms[1], "node_update": ms[2]}
+
+
+def roofline_entry(kern_bytes, elem_ms, peak, peak_kind, traffic, fused=False):
+    """the element-force kernel, or the fused step, against the measured HBM
+    peak: the formula's algorithmic bytes per launch, and (when an ncu capture
+    gave the kernel's DRAM bytes per launch) the measured DRAM traffic per launch
+    time"""
     secs = elem_ms / 1e3
-    r = {"bound": "hbm", "kernel": "k_element_forces",
+    r = {"bound": "hbm", "kernel": "k_patch_step" if fused else "k_element_forces",
          "achieved": kern_bytes / secs / 1e9, "peak": peak, "unit": "GB/s",
          "frac": kern_bytes / secs / 1e9 / peak, "traffic": traffic,
          "peak_source": f"{peak_kind} hbm_gbs"}
@@ -513,12 +529,10 @@ def run_ours(args, rep=None, emit=True, extra=False):
         results[prec] = {
             "ms_per_step": ms / args.steps,
             "value": aggregate_rate(E * args.steps, world, ms),
-            "phase_ms_per_step": {"predictor": phases[0] / nprof,
-                                  "element_forces": phases[1] / nprof,
-                                  "node_update": phases[2] / nprof},
+            "phase_ms_per_step": phases_per_step(phases, nprof, fused),
             "roofline": roofline_entry(step_b if fused else kern_b, elem_ms, peak, peak_kind,
                                        None if args.qp_rule or fused else
-                                       read_traffic(args.config, prec)),
+                                       read_traffic(args.config, prec), fused),
             "roofline_step": {"bytes_per_element_step": step_b / E,
                               "achieved": step_b / (ms / args.steps / 1e3) / 1e9,
                               "frac": step_b / (ms / args.steps / 1e3) / 1e9 / peak},
@@ -531,10 +545,7 @@ def run_ours(args, rep=None, emit=True, extra=False):
                    f"{ms_resident / args.steps:.5f} ms per step with the model L2-resident "
                    "(100-step graphs)") if fits_l2 else
                   f"inputs larger than L2 ({footprint / 1e6:.0f} MB on the device; no flush)",
-            # per step: the element-force kernel and the node update (with the
-            # next predictor), or the fused step; for the ramp, the
-            # prescribed-motion kernel
-            "gpu_launches": args.steps * ((1 if fused else 2) + (args.config == "tri6")),
+            "gpu_launches": args.steps * launches_per_step(fused),
             # the state after the timed steps must be finite (device status word)
             "state_finite": m.getStatus() == 0 and bool(np.all(np.isfinite(m.getDisplacement()))),
         }
@@ -815,16 +826,14 @@ def run_batch(args, rep=None, emit=True, extra=False):
         results[prec] = {
             "ms_per_step": ms / args.steps,
             "value": aggregate_rate(E * args.steps, world, ms),
-            "phase_ms_per_step": {"predictor": phases[0] / nprof,
-                                  "element_forces": phases[1] / nprof,
-                                  "node_update": phases[2] / nprof},
+            "phase_ms_per_step": phases_per_step(phases, nprof, fused),
             "roofline": roofline_entry(step_b if fused else kern_b, elem_ms, peak, peak_kind,
-                                       None if fused else read_traffic("batch", prec)),
+                                       None if fused else read_traffic("batch", prec), fused),
             "roofline_step": {"bytes_per_element_step": step_b / E,
                               "achieved": step_b / (ms / args.steps / 1e3) / 1e9,
                               "frac": step_b / (ms / args.steps / 1e3) / 1e9 / peak},
             "clocks": clk.summary(),
-            "gpu_launches": args.steps * (1 if fused else 2),
+            "gpu_launches": args.steps * launches_per_step(fused),
             "state_finite": b.getStatus() == 0 and bool(np.all(np.isfinite(b.getDisplacement()))),
         }
         if prec == precisions[0] and not extra:
@@ -1091,10 +1100,9 @@ def run_partitioned(args):
                        "subdomain_elements_rank0": local_elems,
                        "l2": "inputs larger than L2 (no flush)"},
             "clocks": clk.summary(),
-            # per step and subdomain: element forces and node update or the
-            # fused step, the ramp (tri6), one halo pack and one unpack per
-            # neighbor (rank 0's subdomains)
-            "gpu_launches": args.steps * sum((1 if lc.model.getFusedStep() else 2) + (1 if args.config == "tri6" else 0) +
+            # per step and subdomain: the step's launches, one halo pack and one
+            # unpack per neighbor (rank 0's subdomains)
+            "gpu_launches": args.steps * sum(launches_per_step(lc.model.getFusedStep()) +
                                              2 * len(lc.sub.neighbors) for lc in pm.locals),
         }
         print(json.dumps(line), flush=True)
