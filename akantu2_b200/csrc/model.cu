@@ -1760,15 +1760,14 @@ int akb_model_init_full(akb_model *m, int method, int precision) {
   // dependent launches: shorter steps at every size (us per step, plain /
   // dependent: tet4 25 k, FP64, 9.0 / 8.5, 384 k 29.6 / 29.2; hex8 64 k, mixed, 13.1
   // / 12.7; FP64 hexahedra, elastic 6^3 7.6 / 7.4, 24^3 11.9 / 11.3, 44^3 58.1 /
-  // 58.0, neohookean 16^3 11.1 / 10.6, 28^3 21.7 / 21.0) but for FP64 hexahedra of
-  // the other laws with one to four of their blocks per SM (neohookean 20^3 13.2 /
-  // 13.8, 24^3 16.1 / 16.8), and unmeasured for mixtures of laws
+  // 58.0, plastic 6^3 8.9 / 8.1, 20^3 14.0 / 13.4, 48^3 158.6 / 157.4, neohookean
+  // 16^3 11.0 / 10.7, 28^3 21.9 / 21.3) but for FP64 neohookean hexahedra with one to
+  // four of their blocks per SM (20^3 13.1 / 14.1, 24^3 16.4 / 16.9); off, as not
+  // measured, for FP64 hexahedra of several laws
   m->pdl = true;
-  if (m->et == AKB_HEXAHEDRON_8 && precision == AKB_PRECISION_FP64) {
-    const int law = m->groups.size() == 1 ? m->groups[0].law : LAW_PLASTIC;
-    m->pdl = law == LAW_ELASTIC ||
-             (law == LAW_NEOHOOKEAN && (E <= 148 * 32 || E > 148 * 4 * 32));
-  }
+  if (m->et == AKB_HEXAHEDRON_8 && precision == AKB_PRECISION_FP64)
+    m->pdl = m->groups.size() == 1 && (m->groups[0].law != LAW_NEOHOOKEAN ||
+                                       E <= 148 * 32 || E > 148 * 4 * 32);
   std::vector<int32_t> conn_soa, ptr, ent, pos;  // (outlive the plan's threads)
   PatchTask patches;
   start_patches(m, patches);

@@ -351,3 +351,22 @@ def test_batches_of_tiny_instances_step_as_two_kernels(precision, cells, count, 
 def test_triangles_whose_patches_are_not_resident_step_as_two_kernels(cells, fused):
     m = gpu_model(akb.square_tri6(*cells), [UNIT_PLASTIC], precision="mixed")
     assert m.getFusedStep() == fused
+
+
+@pytest.mark.parametrize("mat,n,dependent", [(UNIT_ELASTIC, 9, True), (UNIT_PLASTIC, 9, True),
+                                             (UNIT_PLASTIC, 20, True), (UNIT_NEOHOOKEAN, 9, True),
+                                             (UNIT_NEOHOOKEAN, 20, False)])
+def test_dependent_launches_of_fp64_hexahedra(mat, n, dependent):
+    """on but for the neohookean law at one to four blocks per SM; the setting
+    changes no result"""
+    mesh = akb.box_hex8(n)
+    runs = []
+    for other in (False, True):
+        m = gpu_model(mesh, [mat])
+        assert m.getDependentLaunch() == dependent
+        m.setDependentLaunch(dependent != other)
+        m.setNodal("velocity", sinusoidal_velocity(mesh.nodes, 0.03))
+        m.setTimeStep(0.8 * m.getStableTimeStep())
+        m.solveStep(103)
+        runs.append(m.getDisplacement())
+    assert np.abs(runs[0]).max() > 0 and np.array_equal(*runs)
