@@ -1233,17 +1233,10 @@ __device__ __forceinline__ T hex8_affine_adjugate(const T (*wx)[3], T *Ja) {
   return T(1) / adj3(Jp, Ja);
 }
 
-// QU: quadrature points per unrolled iteration (1, 2, 4 or 8).  AFF: every
-// element of the launch is a parallelepiped (checked once per mesh), so the
-// per-point geometry and its registers are compiled out; the same arithmetic
-// as the general kernel's affine branch.  GEO (with AFF): the adjugate and
-// 1/det of each element are read from geo [10][E], formed once by
-// k_hex8_affine_geometry with the same arithmetic, instead of gathering the
-// element's coordinates every step
 // The element's work once its nodal displacements wu and (without GEO) its
 // coordinates wx, both relative to its first node in lexicographic corner
 // order, or (with GEO) its adjugate Ja and 1/det are known: the elemental
-// force in the same order, A
+// force in the same order, A (template parameters as in element_hex8sf)
 template <int LAW, int QU, bool AFF, bool GEO, class T>
 __device__ __forceinline__ void hex8sf_forces(T (*wx)[3], T (*wu)[3], T *Ja, T rdet_a,
                                               const MatParams &mpe, const GroupArgs &ps,
@@ -1439,6 +1432,13 @@ __device__ __forceinline__ void hex8sf_forces_pairs(double (*wu)[3], const doubl
   iwht8(A);
 }
 
+// QU: quadrature points per unrolled iteration (1, 2, 4 or 8).  AFF: every
+// element of the launch is a parallelepiped (checked once per mesh), so the
+// per-point geometry and its registers are compiled out; the same arithmetic
+// as the general kernel's affine branch.  GEO (with AFF): the adjugate and
+// 1/det of each element are read from geo [10][E], formed once by
+// k_hex8_affine_geometry with the same arithmetic, instead of gathering the
+// element's coordinates every step.
 template <int LAW, int QU, bool AFF = false, bool GEO = false, class T = float>
 __device__ __forceinline__ void element_hex8sf(int64_t le, int64_t e_begin, int64_t e_count,
                                                int64_t E, const int32_t *conn,
@@ -1967,11 +1967,12 @@ __device__ __forceinline__ void element_law_streamed(const double (*us)[32], dou
 // point, lane = element), the same gather, the same sums over q in
 // increasing order, bit for bit; every point's NN x D force components go to
 // shared memory [q][component][lane] as they are formed and are summed in
-// one round.  The elastic law, whose arithmetic is short against the latency
-// of its dN/dx rows, has them copied there first, without registers and
-// before the preceding kernel ends (no step changes them), the forces taking
-// their place: 64^3 box 163.5 us per step against 187.9 read from L2 and 180.3
-// held in registers.  The neohookean law is bound by the FP64 and
+// one round.  The elastic and plastic laws, whose arithmetic is short against
+// the latency of their dN/dx rows, have them copied there first, without
+// registers and before the preceding kernel ends (no step changes them), the
+// forces taking their place: 64^3 box, elastic, 163.5 us per step against 187.9
+// read from L2 and 180.3 held in registers, plastic 281.5 against 288.  The
+// neohookean law is bound by the FP64 and
 // shared-memory pipes (193.7 against 196.5 us staged).  Dynamic shared
 // memory: (NN D + NQ NN D) x 32 doubles (55,296 bytes for hexahedra in 3D,
 // above the 48 KB of static shared memory).
@@ -2045,9 +2046,9 @@ __global__ void __launch_bounds__(32 * NQ)
 //        NU_FINT      store the internal force (else it is gathered again on
 //                     request by a flags == NU_FINT launch)
 //        NU_FEXT_ZERO the external force is identically zero: not read
+//                     (0 + f_ext + f_int == f_int)
 //        NU_TRIGGER   the next kernel may launch at once (pdl_begin)
 //        NU_DOWN      the nodes from the last one down (node_block)
-//                     (0 + f_ext + f_int == f_int)
 // KAHAN selects a compensated FP64 sum (mixed path).
 enum { NU_CORRECT = 1, NU_PREDICT = 2, NU_FINT = 4, NU_FEXT_ZERO = 8, NU_TRIGGER = 16, NU_DOWN = 32 };
 

@@ -15,18 +15,18 @@
 // gather, so the results are those of the two-kernel step.
 //
 // Measured on B200, us per step, two kernels / fused: tetrahedra, mixed, 3 k
-// 7.0 / 3.3, 48 k 7.7 / 4.4, 384 k 17.1 / 14.1, 912 k (neohookean) 45.5 / 31.3,
-// a batch of 64 cubes (4.5 M) 205 / 145; FP64 3 k 7.6 / 2.9, 48 k 9.2 / 5.3,
-// 1.3 M 100 / 75, the batch 319 / 244.  What bounds the large ones (80^3 x 6
-// tetrahedra, mixed, ncu): 46 % of the issue slots, 60 % of the shared-memory
-// pipe and 42 % of the DRAM bandwidth are busy; a block waits in turn for its
-// node list, its displacements and its nodes' state, and three fit an SM.
-// Blocks that loop over patches and list the next one's nodes ahead were
-// slower (5.0 against 3.3 us at 3 k tetrahedra, 166 against 165 for the
-// batch), and so were 128, 160, 320 and 384 threads (147 to 159 us).  Plastic
-// triangles, one thread per point: 128 triangles of 3 points, mixed, 10.9 /
-// 6.2, 2 k of 6 points, FP64, 18.5 / 6.7 (9.3 and 18.7 with one thread per
-// element), 20 k of 3 points, mixed, 13.5 / 11.3.
+// 6.9 / 3.1, 48 k 7.7 / 4.5, 384 k 17.4 / 14.1, 912 k (neohookean) 45.9 / 32.0, a
+// batch of 64 cubes (4.5 M) 201 / 138; FP64 3 k 7.6 / 2.8, 48 k 9.4 / 4.9, 1.3 M
+// 95 / 73, the batch 308 / 224.  Which meshes gain is decided on the finished plan
+// (patches_pay).  What bounds the large ones (80^3 x 6 tetrahedra, mixed, ncu):
+// 46 % of the issue slots, 60 % of the shared-memory pipe and 42 % of the DRAM
+// bandwidth are busy; a block waits in turn for its node list, its displacements
+// and its nodes' state, and three fit an SM.  Blocks that loop over patches and
+// list the next one's nodes ahead were slower (5.0 against 3.3 us at 3 k
+// tetrahedra, 166 against 165 for the batch), and so were 128, 160, 320 and 384
+// threads (147 to 159 us).  Plastic triangles, one thread per point: 128
+// triangles of 3 points, mixed, 7.5 / 3.7, 2 k of 6 points, FP64, 13.5 / 4.5 (9.3
+// and 18.7 with one thread per element), 20 k of 3 points, mixed, 9.9 / 8.5.
 #pragma once
 
 #include "fe_kernels.cuh"

@@ -651,8 +651,7 @@ bool thermal_steady(const akb_model *m) {
   return true;
 }
 
-// elemental forces at the predicted displacement (inside a step) or at the
-// model's displacement (standalone assembly)
+// the launches of element_forces
 int launch_forces(akb_model *m, bool in_step) {
   DevGeom g = m->geom();
   const double *u = in_step ? m->u_pred() : m->u();
@@ -674,6 +673,8 @@ int launch_forces(akb_model *m, bool in_step) {
   return AKB_OK;
 }
 
+// elemental forces at the predicted displacement (inside a step) or at the
+// model's displacement (standalone assembly)
 int element_forces(akb_model *m, bool in_step) {
   AKB_TRY(thermal_eval(m, in_step));
   return launch_forces(m, in_step);
@@ -711,11 +712,6 @@ int predict(akb_model *m) {
   return AKB_OK;
 }
 
-// node update after the element forces.  In a step (correct == true): the
-// corrector, then the predictor of the next step from the new displacement
-// u_pred into the other buffer (which held the displacement of the previous
-// step); the internal force is only gathered when asked for (ensure_fint).
-// Standalone (correct == false): the internal force only.
 // whether what a step reads and writes is well beyond L2 (1.25 x 126 MB): the
 // node update then goes from the last nodes down (us per step, up / down: hex8
 // mixed 78 x 41 x 76, 104 MB, 51.0 / 51.7, 96 x 70 x 58, 151 MB, 60.0 / 60.5, 80^3,
@@ -733,6 +729,7 @@ bool step_beyond_l2(const akb_model *m) {
   return m->E * (m->nn * (8. + slot) + table) + 150. * m->N > 1.25 * 126e6;
 }
 
+// the launch of node_update
 int launch_nodes(akb_model *m, bool correct) {
   DevGeom g = m->geom();
   cudaError_t e;
@@ -757,6 +754,11 @@ int launch_nodes(akb_model *m, bool correct) {
   return AKB_OK;
 }
 
+// node update after the element forces.  In a step (correct == true): the
+// corrector, then the predictor of the next step from the new displacement
+// u_pred into the other buffer (which held the displacement of the previous
+// step); the internal force is only gathered when asked for (ensure_fint).
+// Standalone (correct == false): the internal force only.
 int node_update(akb_model *m, bool correct) {
   AKB_TRY(launch_nodes(m, correct));
   if (correct && !m->dinst_end) m->presc_ahead = m->presc_count > 0 || m->presc_ahead;
@@ -838,9 +840,10 @@ int patch_step(akb_model *m, bool store_fint) {
 }
 
 // one explicit step: [predictor,] element forces, node update (+ next
-// predictor); afterwards the prediction buffer becomes the model's u
-// The fused step leaves no elemental forces behind, so the last of a sequence
-// of its steps (last) stores the internal force.
+// predictor), the last two as one launch in the fused step; afterwards the
+// prediction buffer becomes the model's u.  The fused step leaves no elemental
+// forces behind, so the last of a sequence of its steps (last) stores the
+// internal force.
 int one_step(akb_model *m, bool any_plastic, bool last = true, cudaEvent_t e1 = nullptr,
              cudaEvent_t e2 = nullptr) {
   if (!m->predicted) AKB_TRY(predict(m));

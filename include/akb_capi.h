@@ -235,7 +235,8 @@ int akb_model_set_qp_field(akb_model *model, int field, int material, const doub
  * before each later step k = 1, 2, ..., get
  *   u = u_set + sum_{j=1..k} dt * v_max * min(1, j / ramp_steps)
  * (u_set: their displacement at this call; the sum is accumulated in that
- * order).  count == 0 removes the motion (the dofs stay blocked).  Not
+ * order).  count == 0 removes the motion (the dofs stay blocked).  A call
+ * that fails leaves the model, and a motion it had, as they were.  Not
  * available for batches. */
 int akb_model_set_prescribed_velocity_ramp(akb_model *model, const int64_t *dofs,
                                            int64_t count, double v_max, int64_t ramp_steps);
@@ -421,12 +422,16 @@ int akb_model_get_node_shape(const akb_model *model, int *node_block, int *stage
 /* Fused step: the element forces and the node update of a step as one launch
  * over compact patches of nodes (each block evaluates every element that
  * touches its nodes and keeps the elemental forces in shared memory).  On
- * after initFull where the model has it: one law group of tetrahedra
- * (elastic, neohookean), of mixed-precision hexahedra (elastic, neohookean;
- * at most about 15,000) that are all parallelepipeds, or of plastic
- * triangles (at most about 20,000).  Choosing a launch shape, prefetch, geometry, streamed law
- * or node form of the two-kernel step turns it off; AKB_EUNSUPPORTED when a
- * model without it is asked for it.  The same numbers as the two-kernel step.
+ * after initFull where the model has it and its patches make it the faster
+ * form: one law group of tetrahedra (elastic; neohookean, in FP64 up to 32,000),
+ * of mixed-precision hexahedra (elastic, neohookean; at most about 15,000)
+ * that are all parallelepipeds, or of plastic triangles (square meshes of 3
+ * points up to 41,000 mixed and 31,000 FP64, of 6 points up to 20,000); not for
+ * many tiny instances or very irregular meshes, and not where the device has
+ * no memory for its plan (which a later allocation of the model takes back).
+ * Choosing a launch shape, prefetch, geometry, streamed law or node form of the
+ * two-kernel step turns it off; AKB_EUNSUPPORTED when a model without it is
+ * asked for it.  The same numbers as the two-kernel step.
  * No reference counterpart (a launch setting of this library). */
 int akb_model_set_fused_step(akb_model *model, int on);
 int akb_model_get_fused_step(const akb_model *model, int *on);
@@ -529,8 +534,8 @@ int akb_batch_set_instance_materials(akb_model *model, const int32_t *material_o
 /* Instances that stop after their own step counts (the serving loop's
  * batches): from the current step on, instance k advances exactly steps[k]
  * more steps (steps[k] < 0: its limit stays as it is, initially none) and
- * then keeps its state (u, v, a;
- * its plastic internals are not maintained) while the others go on; the
+ * then keeps its state (u, v, a and the internal force of its last step; its
+ * plastic internals are not maintained) while the others go on; the
  * captured step graphs stay valid (each step's kernels read the device's
  * step counter).  Called again, it sets new counts from the current step. */
 int akb_batch_set_instance_steps(akb_model *model, const int64_t *steps);
