@@ -1109,43 +1109,76 @@ int reduce_to_host(akb_model *m, const double *x, int64_t n, bool op_min, double
 
 // ---- plan of the fused step ------------------------------------------------
 
-// Whether a plan of so many patches and evaluated elements (those on a border
-// counted in each patch), whose largest patch needs smem bytes, steps faster
-// than the two kernels.
+// the elements that a plan's patches evaluate (those on a border in each patch)
+struct PatchLoad {
+  int64_t patches = 0, evaluated = 0;
+  int64_t largest = 0;   // of a patch
+  int64_t heaviest = 0;  // of an SM, its patches one in every kPatchSms
+};
+PatchLoad patch_load(const std::vector<PatchHead> &head) {
+  PatchLoad l;
+  l.patches = (int64_t)head.size();
+  int64_t sm[kPatchSms] = {0};
+  for (int64_t p = 0; p < l.patches; ++p) {
+    l.evaluated += head[p].n_elem;
+    l.largest = std::max<int64_t>(l.largest, head[p].n_elem);
+    l.heaviest = std::max(l.heaviest, sm[p % kPatchSms] += head[p].n_elem);
+  }
+  return l;
+}
+// patches of the same size, as many and as few elements as given
+PatchLoad even_load(int64_t patches, int64_t evaluated) {
+  PatchLoad l;
+  l.patches = patches;
+  l.evaluated = evaluated;
+  l.largest = evaluated / patches;
+  l.heaviest = (patches + kPatchSms - 1) / kPatchSms * l.largest;
+  return l;
+}
+
+// Whether a plan of such patches, the largest of which needs smem bytes, steps
+// faster than the two kernels.
 //
-// Tetrahedra: the time of either form in us from constants fitted to 200
-// measured meshes (cubes, plates, bars, Delaunay meshes, batches; mean error 7
-// per cent).  An SM steps through its patches resident ones at a time, each round
-// with a latency, each element with a time that grows when fewer blocks than
-// the kernel is built for are resident; the two kernels have a time per element
-// and, beyond 100 MB, per byte.  The plan must win by a twentieth: the few
-// meshes the fit has on the wrong side differ by less.  Two kernels / fused:
-// 1000 cubes of 1^3, mixed, 5.3 / 7.8, 4000 6.1 / 25.6, 2000 of 3^3 17.4 / 20.8, 300
-// of 4^3 9.5 / 5.9; Delaunay, mixed, 54 k 10.8 / 6.6, 429 k, one block per SM, 22.0
-// / 24.7, 1.4 M, two, 71.8 / 73.7; 1000 x 8 x 8 cells neohookean 18.6 / 18.6.
+// Tetrahedra: the time of either form in us from constants fitted to 409 measured
+// meshes (boxes, plates, bars, Delaunay meshes, batches; mean error 7 per cent).
+// An SM steps through its patches resident ones at a time: each round has a
+// latency, each element a time that grows when fewer blocks than the kernel is
+// built for are resident.  With all patches resident at once the SM with the most
+// elements is the last (mixed neohookean, 30 x 30 x 30 cells, 216 patches of up to
+// 5^3 nodes, 9.0 us), beyond that half a patch is still under way when the others
+// end.  Places for three per SM are not filled evenly: of 217 to 296 patches some
+// SM has three (mixed, 264 equal patches of 33 cubes of 11^3, 11.4 us, where two
+// per SM would take 8.9; 44 x 36 x 22 cells, neohookean, 224 patches, 14.6, two
+// kernels 11.9).  The two kernels have a time per
+// element and, beyond 100 MB, per byte.  The plan must win by 7 per cent: no mesh
+// of the fit is then slower by more than 1, and what is left to the two kernels
+// loses 8 to 15 on four.  Two kernels / fused: 1000 cubes of 1^3, mixed, 5.3 / 7.8,
+// 4000 6.1 / 25.6, 2000 of 3^3 17.4 / 20.8, 300 of 4^3 9.5 / 5.9; Delaunay, mixed, 54 k
+// 10.8 / 6.6, 429 k, one block per SM, 22.0 / 24.7, 1.4 M, two, 71.8 / 73.7.
 //
 // Hexahedra: the elements of an SM within half as many again as the largest
 // box of the rule below has.  Triangles: up to four patches per SM, two of 6
 // points (mixed 400 x 20 x 2, 606 patches, 10.3, two kernels 9.7; FP64 1000 x 5 x 2,
 // 502 patches, 8.9 / 10.6).
-bool patches_pay(int et, int rule, int law, bool mixed, int64_t E, int64_t patches,
-                 int64_t evaluated, size_t smem) {
-  const double sms = (double)kPatchSms;
-  const double rounds = std::ceil((double)patches / sms);  // patches of an SM
-  const double work = rounds * (double)evaluated / (double)patches;  // and their elements
+bool patches_pay(int et, int rule, int law, bool mixed, int64_t E, const PatchLoad &load,
+                 size_t smem) {
+  const double rounds = std::ceil((double)load.patches / kPatchSms);  // patches of an SM
   if (et == AKB_TRIANGLE_6) return rounds <= (rule ? 2. : 4.);
-  if (et == AKB_HEXAHEDRON_8) return work <= 250.;
+  if (et == AKB_HEXAHEDRON_8) return rounds * load.evaluated <= 250. * load.patches;
   const double built = mixed ? 3. : 2.;
   const double resident = std::min(built, std::max(1., std::floor(233472. / (double)(smem + 1024))));
   const double rate = std::min(built, rounds) / std::min(resident, rounds);
+  const bool uneven = rounds == 2. && resident == 3. && load.patches > 216;
+  const double work = rounds <= resident ? (uneven ? 1.5 : 1.) * (double)load.heaviest
+                                         : (double)load.evaluated / kPatchSms + 0.5 * load.largest;
   const bool neo = law == LAW_NEOHOOKEAN;
-  const double element = mixed ? (neo ? 3.1e-3 : 2.6e-3) : (neo ? 12.5e-3 : 3.15e-3);
-  const double fused = (mixed ? 3.0 : 2.7) * std::ceil(rounds / resident) + element * work * rate;
+  const double element = mixed ? (neo ? 2.65e-3 : 2.3e-3) : (neo ? 7.2e-3 : 2.9e-3);
+  const double fused = (mixed ? 3.0 : 2.6) * std::ceil(rounds / resident) + element * work * rate;
   const double beyond = std::max(0., (mixed ? 190. : 270.) * (double)E - 100e6);
   const double two = mixed ? 6.1 + 33.3e-6 * (double)E + 0.116e-6 * beyond
                            : (neo ? 8.2 : 7.0) + (neo ? 65e-6 : 60.7e-6) * (double)E +
                                  0.0575e-6 * beyond;
-  return fused <= 0.95 * two;
+  return fused <= 0.93 * two;
 }
 
 // Owned nodes of a patch at most, s per edge; 0 where the two-kernel step is
@@ -1217,7 +1250,8 @@ int patch_nodes(int et, int rule, int law, int precision, int64_t N, int64_t E, 
   }
   // no patch reaches across two instances of a batch
   const int own = best * best * best;
-  if (tet && !patches_pay(et, rule, law, mixed, E, std::max<int64_t>(ninst, N / own), E, 0))
+  if (tet && !patches_pay(et, rule, law, mixed, E,
+                          even_load(std::max<int64_t>(std::max(ninst, 1), N / own), E), 0))
     return 0;
   return own;
 }
@@ -1355,11 +1389,9 @@ int finish_patches(akb_model *m, PatchTask &task) {
   const int points = m->et == AKB_TRIANGLE_6 ? m->nq : 1;  // slot arrays
   pa.smem = patch_smem(m->dim, plan.max_local, plan.max_slots * points, t.value);
   if (pa.smem + kPatchStageSmem > kPatchMaxSmem) return AKB_OK;
-  int64_t evaluated = 0;
-  for (const PatchHead &h : plan.head) evaluated += h.n_elem;
   PatchCaps need;
   need.patches = (int64_t)plan.head.size();
-  if (!patches_pay(m->et, m->rule, gr.law, mixed, m->E, need.patches, evaluated, pa.smem))
+  if (!patches_pay(m->et, m->rule, gr.law, mixed, m->E, patch_load(plan.head), pa.smem))
     return AKB_OK;
   need.nodes = (int64_t)plan.nodes.size();
   need.elems = (int64_t)plan.elems.size();
@@ -1764,13 +1796,18 @@ int akb_model_init_full(akb_model *m, int method, int precision) {
   // dependent: tet4 25 k, FP64, 9.0 / 8.5, 384 k 29.6 / 29.2; hex8 64 k, mixed, 13.1
   // / 12.7; FP64 hexahedra, elastic 6^3 7.6 / 7.4, 24^3 11.9 / 11.3, 44^3 58.1 /
   // 58.0, plastic 6^3 8.9 / 8.1, 20^3 14.0 / 13.4, 48^3 158.6 / 157.4, neohookean
-  // 16^3 11.0 / 10.7, 28^3 21.9 / 21.3) but for FP64 neohookean hexahedra with one to
-  // four of their blocks per SM (20^3 13.1 / 14.1, 24^3 16.4 / 16.9); off, as not
-  // measured, for FP64 hexahedra of several laws
+  // 16^3 11.0 / 10.7, 28^3 21.8 / 21.2, 32^3 27.5 / 26.9, 48^3 87.9 / 87.3) but for FP64
+  // neohookean hexahedra, four of whose blocks are resident per SM, with one to
+  // four (20^3 13.1 / 14.1, 24^3 16.4 / 16.9) or in the third round, with eight to
+  // twelve (34^3 33.7 / 34.4, 47 x 37 x 26 38.3 / 41.2, 38^3 49.0 / 49.4, 40^3 55.4 /
+  // 55.1); off, as not measured, for FP64 hexahedra of several laws
   m->pdl = true;
-  if (m->et == AKB_HEXAHEDRON_8 && precision == AKB_PRECISION_FP64)
-    m->pdl = m->groups.size() == 1 && (m->groups[0].law != LAW_NEOHOOKEAN ||
-                                       E <= 148 * 32 || E > 148 * 4 * 32);
+  if (m->et == AKB_HEXAHEDRON_8 && precision == AKB_PRECISION_FP64) {
+    const double per_sm = (double)E / (32. * 148.);
+    m->pdl = m->groups.size() == 1 &&
+             (m->groups[0].law != LAW_NEOHOOKEAN ||
+              !((per_sm > 1. && per_sm <= 4.) || (per_sm > 8. && per_sm <= 12.)));
+  }
   std::vector<int32_t> conn_soa, ptr, ent, pos;  // (outlive the plan's threads)
   PatchTask patches;
   start_patches(m, patches);

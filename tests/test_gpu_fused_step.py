@@ -355,10 +355,12 @@ def test_triangles_whose_patches_are_not_resident_step_as_two_kernels(cells, fus
 
 @pytest.mark.parametrize("mat,n,dependent", [(UNIT_ELASTIC, 9, True), (UNIT_PLASTIC, 9, True),
                                              (UNIT_PLASTIC, 20, True), (UNIT_NEOHOOKEAN, 9, True),
-                                             (UNIT_NEOHOOKEAN, 20, False)])
+                                             (UNIT_NEOHOOKEAN, 20, False),
+                                             (UNIT_NEOHOOKEAN, 28, True),
+                                             (UNIT_NEOHOOKEAN, 35, False)])
 def test_dependent_launches_of_fp64_hexahedra(mat, n, dependent):
-    """on but for the neohookean law at one to four blocks per SM; the setting
-    changes no result"""
+    """on but for the neohookean law at one to four and eight to twelve blocks per
+    SM; the setting changes no result"""
     mesh = akb.box_hex8(n)
     runs = []
     for other in (False, True):
