@@ -37,7 +37,11 @@ constexpr int kMaxNN = 8;
 // instructions do nothing.
 __device__ __forceinline__ void pdl_begin(bool trigger = true) {
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  if (trigger) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  // (predicated: a branch here changes the code that follows, 0.1 us of FP64
+  // hexahedra)
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %0, 0;\n\t"
+               "@p griddepcontrol.launch_dependents;\n\t}" ::"r"((int)trigger)
+               : "memory");
 }
 
 // L2 prefetch (cp.async.bulk.prefetch.L2: nothing reaches the SM) of the
@@ -125,7 +129,6 @@ struct GroupArgs {
   double *c33;               // [q][ne] plane-stress neohookean out-of-plane stretch
                              // (updated in place by every stress evaluation), or null
   int update_energy;         // 1 inside solveStep (afterSolveStep), 0 otherwise
-  int trigger;               // the next kernel may launch at once (pdl_begin)
   // eigen gradient of the displacement [q][d*d][ne] (double), subtracted from
   // the gradient before the law (material.cc:147), or null when zero
   const double *eig;
@@ -135,6 +138,10 @@ struct GroupArgs {
   const int32_t *einst;
   const int64_t *inst_end;
   const int64_t *step;
+  // the next kernel may launch at once (pdl_begin); beside what every element
+  // reads first, as a parameter's line of the constant bank that is read for
+  // this alone makes the kernel 0.1 us longer
+  int trigger;
   // index checks of the bounds-checking build (AKB_BOUNDS_CHECK): node count,
   // slot count and the model's status word
   int64_t nb_nodes, nb_slots;
@@ -1975,9 +1982,11 @@ __device__ __forceinline__ void element_law_streamed(const double (*us)[32], dou
 // neohookean law is bound by the FP64 and
 // shared-memory pipes (193.7 against 196.5 us staged).  Dynamic shared
 // memory: (NN D + NQ NN D) x 32 doubles (55,296 bytes for hexahedra in 3D,
-// above the 48 KB of static shared memory).
+// above the 48 KB of static shared memory).  Registers for two blocks per SM of
+// the plastic law (130 without the cap leave one: 30^3 45.2 us per step against
+// 33.8, 64^3 281 against 253) and for the four that shared memory allows else.
 template <int D, int NN, int NQ, int LAW>
-__global__ void __launch_bounds__(32 * NQ)
+__global__ void __launch_bounds__(32 * NQ, LAW == LAW_PLASTIC ? 2 : 4)
     k_element_forces_pqs(int64_t e_begin, int64_t e_count, int64_t E,
                          const int32_t *__restrict__ conn, const int32_t *__restrict__ pos,
                          const double *__restrict__ B, const double *__restrict__ wJ,
@@ -2360,14 +2369,16 @@ __device__ __forceinline__ void node_body(int64_t i, const int32_t *ptr,
 // last nodes (they are in L2), and leaves the next step's elements the
 // displacements of the first ones there.  With RAMP the extra block, the last,
 // has none (its index is -1, or past the nodes).
-template <bool RAMP> __device__ __forceinline__ int64_t node_block(int flags) {
-  return flags & NU_DOWN ? (int64_t)gridDim.x - (RAMP ? 2 : 1) - blockIdx.x : blockIdx.x;
+template <bool RAMP> __device__ __forceinline__ int64_t node_block(int head) {
+  return head & NU_DOWN ? (int64_t)gridDim.x - (RAMP ? 2 : 1) - blockIdx.x : blockIdx.x;
 }
 
 // launched with up to 1024 threads per block (the autotuner's candidates):
-// at most 64 registers
-template <int D, class RT, bool KAHAN, bool WIDE = false, bool RAMP = false>
-__global__ void __launch_bounds__(1024) k_node_update(int64_t N, const int32_t *__restrict__ ptr,
+// at most 64 registers.  HEAD: NU_TRIGGER and NU_DOWN of the flags where they are
+// known (0 and NU_TRIGGER, the meshes of a few us per step), or -1: read from head
+// (FP64 tetrahedra 25 k, 11.90 us per step with both read, 11.76 known)
+template <int D, class RT, bool KAHAN, bool WIDE = false, bool RAMP = false, int HEAD = -1>
+__global__ void __launch_bounds__(1024) k_node_update(int64_t N, int head, const int32_t *__restrict__ ptr,
                               const RT *__restrict__ re, const double *__restrict__ fext,
                               const double *__restrict__ mass,
                               const uint8_t *__restrict__ blocked, double *__restrict__ fint,
@@ -2376,9 +2387,10 @@ __global__ void __launch_bounds__(1024) k_node_update(int64_t N, const int32_t *
                               double dt, const int32_t *__restrict__ node_inst,
                               const double *__restrict__ inst_dt, int flags,
                               unsigned int *__restrict__ status, const PrescArgs pr) {
-  pdl_begin(flags & NU_TRIGGER);
+  if constexpr (HEAD >= 0) head = HEAD;
+  pdl_begin(head & NU_TRIGGER);
   if (RAMP && blockIdx.x == gridDim.x - 1) return prescribe_block(pr, u_next, true);
-  const int64_t i = node_block<RAMP>(flags) * blockDim.x + threadIdx.x;
+  const int64_t i = node_block<RAMP>(head) * blockDim.x + threadIdx.x;
   if (i >= N || !node_range_ok(ptr, N, i, status)) return;
   node_body<D, RT, KAHAN, WIDE, RAMP>(i, ptr, re, fext, mass, blocked, fint, a, v, u, u_next, dt,
                                 node_inst, inst_dt, flags, status);
@@ -2391,14 +2403,14 @@ __global__ void __launch_bounds__(1024) k_node_update(int64_t N, const int32_t *
 // they are in flight together with it rather than after it
 template <int D, class RT, bool KAHAN, bool WIDE = false, bool RAMP = false>
 __global__ void __launch_bounds__(1024)
-    k_node_update_early(int64_t N, const int32_t *__restrict__ ptr, const RT *__restrict__ re,
+    k_node_update_early(int64_t N, int head, const int32_t *__restrict__ ptr, const RT *__restrict__ re,
                         const double *__restrict__ fext, const double *__restrict__ mass,
                         const uint8_t *__restrict__ blocked, double *__restrict__ fint,
                         double *__restrict__ a, double *__restrict__ v,
                         const double *__restrict__ u, double *__restrict__ u_next, double dt,
                         const int32_t *__restrict__ node_inst, const double *__restrict__ inst_dt,
                         int flags, unsigned int *__restrict__ status, const PrescArgs pr) {
-  const int64_t i = node_block<RAMP>(flags) * blockDim.x + threadIdx.x;
+  const int64_t i = node_block<RAMP>(head) * blockDim.x + threadIdx.x;
   const bool in = (!RAMP || i >= 0) && i < N;
   int32_t p0 = 0, p1 = 0;
   NodeState<D> st;
@@ -2410,7 +2422,7 @@ __global__ void __launch_bounds__(1024)
     st.m = mass[i];
     st.bl = blocked[i];
   }
-  pdl_begin(flags & NU_TRIGGER);
+  pdl_begin(head & NU_TRIGGER);
   if (RAMP && blockIdx.x == gridDim.x - 1) return prescribe_block(pr, u_next, true);
   if (!in || !node_range_ok(ptr, N, i, status)) return;
   if (flags & NU_CORRECT) load_node_state<D>(st, i, fext, a, v, u, flags);
@@ -2432,7 +2444,7 @@ __global__ void __launch_bounds__(1024)
 // The last step of an instance stores its internal force: a later gather of
 // the slots leaves stopped instances out
 template <int D, class RT, bool KAHAN>
-__global__ void __launch_bounds__(1024) k_node_update_retire(int64_t N, const int32_t *__restrict__ ptr,
+__global__ void __launch_bounds__(1024) k_node_update_retire(int64_t N, int head, const int32_t *__restrict__ ptr,
                                      const RT *__restrict__ re, const double *__restrict__ fext,
                                      const double *__restrict__ mass,
                                      const uint8_t *__restrict__ blocked,
@@ -2443,7 +2455,7 @@ __global__ void __launch_bounds__(1024) k_node_update_retire(int64_t N, const in
                                      const int64_t *__restrict__ inst_end,
                                      const int64_t *__restrict__ step, int flags,
                                      unsigned int *__restrict__ status) {
-  pdl_begin(flags & NU_TRIGGER);
+  pdl_begin(head & NU_TRIGGER);
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N || !node_range_ok(ptr, N, i, status)) return;
   // a batch of one instance has no node -> instance table
@@ -2486,7 +2498,7 @@ __device__ __forceinline__ int swizzle(int w) { return w ^ ((w >> 3) & 7); }
 
 template <int D, class RT, bool KAHAN, int BLOCK, bool RAMP = false>
 __global__ void __launch_bounds__(BLOCK)
-    k_node_update_staged(int64_t N, const int32_t *__restrict__ ptr, const RT *__restrict__ re,
+    k_node_update_staged(int64_t N, int head, const int32_t *__restrict__ ptr, const RT *__restrict__ re,
                          const double *__restrict__ fext, const double *__restrict__ mass,
                          const uint8_t *__restrict__ blocked, double *__restrict__ fint,
                          double *__restrict__ a, double *__restrict__ v,
@@ -2494,14 +2506,14 @@ __global__ void __launch_bounds__(BLOCK)
                          const int32_t *__restrict__ node_inst,
                          const double *__restrict__ inst_dt, int flags,
                          unsigned int *__restrict__ status, const PrescArgs pr) {
-  pdl_begin(flags & NU_TRIGGER);
+  pdl_begin(head & NU_TRIGGER);
   if (RAMP && blockIdx.x == gridDim.x - 1) return prescribe_block(pr, u_next, true);
   using V = typename SlotVec<D, RT>::type;
   constexpr int WPS = SlotVec<D, RT>::per_slot;  // vectors per slot
   constexpr int CAPW = kStagedBytes / (int)sizeof(V);
   constexpr int CAP = CAPW / WPS;               // slots per chunk
   __shared__ V sm[CAPW];
-  const int64_t i0 = node_block<RAMP>(flags) * BLOCK;
+  const int64_t i0 = node_block<RAMP>(head) * BLOCK;
   const int64_t i = i0 + threadIdx.x;
   const int64_t iend = i0 + BLOCK < N ? i0 + BLOCK : N;
   const int32_t pb = ptr[i0], pe = ptr[iend];

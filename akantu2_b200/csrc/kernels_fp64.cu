@@ -120,9 +120,10 @@ cudaError_t launch_node_update_fp64(const DevGeom &g, const double *re, const do
                                     double *a, double *v, const double *u, double *u_next,
                                     double dt, int flags, unsigned int *status, int node_block,
                                     int form, cudaStream_t s) {
+  const int head = flags & (NU_TRIGGER | NU_DOWN);
   if (g.N > 0 && g.inst_end) {
     auto kern = g.D == 3 ? k_node_update_retire<3, double, false> : k_node_update_retire<2, double, false>;
-    return launch_step(g.pdl, kern, grid_for(g.N, node_block), node_block, s, g.N, g.ptr, re,
+    return launch_step(g.pdl, kern, grid_for(g.N, node_block), node_block, s, g.N, head, g.ptr, re,
                        fext, mass, blocked, fint, a, v, const_cast<double *>(u), u_next, dt,
                        g.node_inst, g.inst_dt, g.inst_end, (const int64_t *)g.step, flags, status);
   }
@@ -132,7 +133,7 @@ cudaError_t launch_node_update_fp64(const DevGeom &g, const double *re, const do
   if (form == 1) form = 0;  // the bounds-checking build checks each node's own slot range
 #endif
   auto go = [&](auto kern, int block) {
-    return launch_step(g.pdl, kern, grid_for(g.N, block) + extra, block, s, g.N, g.ptr, re, fext,
+    return launch_step(g.pdl, kern, grid_for(g.N, block) + extra, block, s, g.N, head, g.ptr, re, fext,
                        mass, blocked, fint, a, v, u, u_next, dt, g.node_inst, g.inst_dt, flags,
                        status, g.presc);
   };
@@ -147,12 +148,13 @@ cudaError_t launch_node_update_fp64(const DevGeom &g, const double *re, const do
   }
   // slots read 32 bytes at a time when the array's alignment allows it
   const bool wide = ((uintptr_t)re & 31) == 0;
-  auto pick = [&](auto ramp) {
+  auto pick = [&](auto ramp, auto known) {
     constexpr bool R = decltype(ramp)::value;
-    auto kern = g.D == 3 ? (wide ? k_node_update<3, double, false, true, R>
-                                 : k_node_update<3, double, false, false, R>)
-                         : (wide ? k_node_update<2, double, false, true, R>
-                                 : k_node_update<2, double, false, false, R>);
+    constexpr int H = decltype(known)::value;
+    auto kern = g.D == 3 ? (wide ? k_node_update<3, double, false, true, R, H>
+                                 : k_node_update<3, double, false, false, R, H>)
+                         : (wide ? k_node_update<2, double, false, true, R, H>
+                                 : k_node_update<2, double, false, false, R, H>);
     if (form == 2)
       kern = g.D == 3 ? (wide ? k_node_update_early<3, double, false, true, R>
                               : k_node_update_early<3, double, false, false, R>)
@@ -160,7 +162,12 @@ cudaError_t launch_node_update_fp64(const DevGeom &g, const double *re, const do
                               : k_node_update_early<2, double, false, false, R>);
     return go(kern, node_block);
   };
-  return extra ? pick(std::true_type()) : pick(std::false_type());
+  auto pick_head = [&](auto ramp) {
+    if (head == 0) return pick(ramp, std::integral_constant<int, 0>());
+    if (head == NU_TRIGGER) return pick(ramp, std::integral_constant<int, NU_TRIGGER>());
+    return pick(ramp, std::integral_constant<int, -1>());
+  };
+  return extra ? pick_head(std::true_type()) : pick_head(std::false_type());
 }
 
 // prescribed motion: before step k (k = 1, 2, ... since the motion was set)

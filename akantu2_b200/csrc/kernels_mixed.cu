@@ -178,9 +178,10 @@ cudaError_t launch_node_update_mixed(const DevGeom &g, const float *re, const do
                                      double *u_next, double dt, int flags,
                                      unsigned int *status, int node_block, int form,
                                      cudaStream_t s) {
+  const int head = flags & (NU_TRIGGER | NU_DOWN);
   if (g.N > 0 && g.inst_end) {
     auto kern = g.D == 3 ? k_node_update_retire<3, float, true> : k_node_update_retire<2, float, true>;
-    return launch_step(g.pdl, kern, grid_for(g.N, node_block), node_block, s, g.N, g.ptr, re,
+    return launch_step(g.pdl, kern, grid_for(g.N, node_block), node_block, s, g.N, head, g.ptr, re,
                        fext, mass, blocked, fint, a, v, const_cast<double *>(u), u_next, dt,
                        g.node_inst, g.inst_dt, g.inst_end, (const int64_t *)g.step, flags, status);
   }
@@ -190,7 +191,7 @@ cudaError_t launch_node_update_mixed(const DevGeom &g, const float *re, const do
   if (form == 1) form = 0;  // the bounds-checking build checks each node's own slot range
 #endif
   auto go = [&](auto kern, int block) {
-    return launch_step(g.pdl, kern, grid_for(g.N, block) + extra, block, s, g.N, g.ptr, re, fext,
+    return launch_step(g.pdl, kern, grid_for(g.N, block) + extra, block, s, g.N, head, g.ptr, re, fext,
                        mass, blocked, fint, a, v, u, u_next, dt, g.node_inst, g.inst_dt, flags,
                        status, g.presc);
   };
@@ -205,12 +206,13 @@ cudaError_t launch_node_update_mixed(const DevGeom &g, const float *re, const do
   }
   // slots read 32 bytes at a time when the array's alignment allows it
   const bool wide = ((uintptr_t)re & 31) == 0;
-  auto pick = [&](auto ramp) {
+  auto pick = [&](auto ramp, auto known) {
     constexpr bool R = decltype(ramp)::value;
-    auto kern = g.D == 3 ? (wide ? k_node_update<3, float, true, true, R>
-                                 : k_node_update<3, float, true, false, R>)
-                         : (wide ? k_node_update<2, float, true, true, R>
-                                 : k_node_update<2, float, true, false, R>);
+    constexpr int H = decltype(known)::value;
+    auto kern = g.D == 3 ? (wide ? k_node_update<3, float, true, true, R, H>
+                                 : k_node_update<3, float, true, false, R, H>)
+                         : (wide ? k_node_update<2, float, true, true, R, H>
+                                 : k_node_update<2, float, true, false, R, H>);
     if (form == 2)
       kern = g.D == 3 ? (wide ? k_node_update_early<3, float, true, true, R>
                               : k_node_update_early<3, float, true, false, R>)
@@ -218,7 +220,12 @@ cudaError_t launch_node_update_mixed(const DevGeom &g, const float *re, const do
                               : k_node_update_early<2, float, true, false, R>);
     return go(kern, node_block);
   };
-  return extra ? pick(std::true_type()) : pick(std::false_type());
+  auto pick_head = [&](auto ramp) {
+    if (head == 0) return pick(ramp, std::integral_constant<int, 0>());
+    if (head == NU_TRIGGER) return pick(ramp, std::integral_constant<int, NU_TRIGGER>());
+    return pick(ramp, std::integral_constant<int, -1>());
+  };
+  return extra ? pick_head(std::true_type()) : pick_head(std::false_type());
 }
 
 cudaError_t launch_hex8_affine_geometry(const DevGeom &g, float *geo, cudaStream_t s) {
