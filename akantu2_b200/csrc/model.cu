@@ -768,9 +768,12 @@ int node_update(akb_model *m, bool correct) {
 }
 
 // Both where the two kernels' blocks are resident all together (pdl_begin).  A
-// node update of up to 8 blocks per SM also before element kernels of more,
-// whose many waves start under it (us per step, without / with: FP64
-// tetrahedra, 236 k 21.2 / 20.8, 384 k 29.2 / 28.5).
+// node update of up to 8 blocks per SM also before element kernels of more, and
+// before those of tetrahedra (whose node updates have a fifth of their blocks): the
+// waves of elements start under it (FP64 neohookean tetrahedra, us per step, none /
+// node update / both: 105 k 12.9 / 12.8 / 22.8, 135 k 15.5 / 14.9 / 15.0, 162 k 17.9 /
+// 16.2 / 17.1; mixed neohookean hexahedra 55 k 11.5 / 12.2 / 16.4; plastic FP64
+// triangles 54 k 17.1 / 19.6 / 23.3).
 int find_trigger(akb_model *m) {
   if (m->trigger >= 0) return AKB_OK;
   LaunchProbe probe;
@@ -781,7 +784,9 @@ int find_trigger(akb_model *m) {
   launch_probe = nullptr;
   const unsigned many = 8 * kPatchSms;
   if (rc == AKB_OK)
-    m->trigger = probe.waves <= 1. ? 3 : elem_blocks > many && probe.blocks <= many ? 2 : 0;
+    m->trigger = probe.waves <= 1. ? 3
+                 : (elem_blocks > many || m->et == AKB_TETRAHEDRON_4) && probe.blocks <= many ? 2
+                                                                                             : 0;
   return rc;
 }
 
@@ -1146,10 +1151,10 @@ PatchLoad even_load(int64_t patches, int64_t evaluated) {
 // built for are resident.  With all patches resident at once the SM with the most
 // elements is the last (mixed neohookean, 30 x 30 x 30 cells, 216 patches of up to
 // 5^3 nodes, 9.0 us), beyond that half a patch is still under way when the others
-// end.  Places for three per SM are not filled evenly: of 217 to 296 patches some
-// SM has three (mixed, 264 equal patches of 33 cubes of 11^3, 11.4 us, where two
-// per SM would take 8.9; 44 x 36 x 22 cells, neohookean, 224 patches, 14.6, two
-// kernels 11.9).  The two kernels have a time per
+// end.  Places for three per SM are not filled evenly: of 217 to 340 patches some
+// SM has three large ones (mixed, 264 equal patches of 33 cubes of 11^3, 11.4 us,
+// where two per SM would take 8.9; neohookean, 44 x 36 x 22 cells, 224 patches, 14.6,
+// two kernels 11.9, 54 x 34 x 28, 300 patches, 15.7 and 14.8).  The two kernels have a time per
 // element and, beyond 100 MB, per byte.  The plan must win by 7 per cent: no mesh
 // of the fit is then slower by more than 1, and what is left to the two kernels
 // loses 8 to 15 on four.  Two kernels / fused: 1000 cubes of 1^3, mixed, 5.3 / 7.8,
@@ -1168,9 +1173,10 @@ bool patches_pay(int et, int rule, int law, bool mixed, int64_t E, const PatchLo
   const double built = mixed ? 3. : 2.;
   const double resident = std::min(built, std::max(1., std::floor(233472. / (double)(smem + 1024))));
   const double rate = std::min(built, rounds) / std::min(resident, rounds);
-  const bool uneven = rounds == 2. && resident == 3. && load.patches > 216;
-  const double work = rounds <= resident ? (uneven ? 1.5 : 1.) * (double)load.heaviest
-                                         : (double)load.evaluated / kPatchSms + 0.5 * load.largest;
+  const bool uneven = resident == 3. && load.patches > 216 && load.patches <= 340;
+  const double work = uneven              ? 3. * (double)load.largest
+                      : rounds <= resident ? (double)load.heaviest
+                                           : (double)load.evaluated / kPatchSms + 0.5 * load.largest;
   const bool neo = law == LAW_NEOHOOKEAN;
   const double element = mixed ? (neo ? 2.65e-3 : 2.3e-3) : (neo ? 7.2e-3 : 2.9e-3);
   const double fused = (mixed ? 3.0 : 2.6) * std::ceil(rounds / resident) + element * work * rate;
