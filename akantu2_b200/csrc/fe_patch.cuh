@@ -18,7 +18,7 @@
 // 6.9 / 3.1, 48 k 7.7 / 4.5, 384 k 17.4 / 14.1, 912 k (neohookean) 45.9 / 32.0, a
 // batch of 64 cubes (4.5 M) 201 / 138; FP64 3 k 7.6 / 2.8, 48 k 9.4 / 4.9, 1.3 M
 // 95 / 73, the batch 308 / 224.  Which meshes gain is decided on the finished plan
-// (patches_pay).  What bounds the large ones (80^3 x 6 tetrahedra, mixed, ncu):
+// (patches_over_kernels).  What bounds the large ones (80^3 x 6 tetrahedra, mixed, ncu):
 // 46 % of the issue slots, 60 % of the shared-memory pipe and 42 % of the DRAM
 // bandwidth are busy; a block waits in turn for its node list, its displacements
 // and its nodes' state, and three fit an SM.  Blocks that loop over patches and

@@ -305,7 +305,7 @@ struct akb_model {
   PatchArgs patch;
   void *patch_mem = nullptr;  // its arrays
   size_t patch_bytes = 0;
-  bool patch_ready = false, patch_on = false;
+  bool patch_ready = false, patch_on = false, patch_unsure = false;
   bool plan_left_out = false;  // leave_out_plan
   // persistent multi-step kernel: 0 never (default: on B200 the 100-step
   // graphs of the two-kernel step are faster at every measured size), 1 for
@@ -820,9 +820,8 @@ cudaError_t launch_patches(akb_model *m, PatchArgs pa, const GroupArgs &ps, bool
              : launch_patch_step_fp64(m->et, gr.law, pa, mp, ps, pdl, m->stream);
 }
 
-// element forces and node update as one launch
-int patch_step(akb_model *m, bool store_fint) {
-  AKB_TRY(thermal_eval(m, true));
+// the state the fused step reads and writes
+PatchArgs patch_args(akb_model *m, bool store_fint) {
   PatchArgs pa = m->patch;
   pa.u = m->u_pred();
   pa.u_next = m->u();
@@ -834,6 +833,13 @@ int patch_step(akb_model *m, bool store_fint) {
   pa.status = m->dstatus;
   pa.flags = NU_CORRECT | NU_PREDICT | (m->fext_zero ? NU_FEXT_ZERO : 0) |
              (store_fint ? NU_FINT : 0);
+  return pa;
+}
+
+// element forces and node update as one launch
+int patch_step(akb_model *m, bool store_fint) {
+  AKB_TRY(thermal_eval(m, true));
+  PatchArgs pa = patch_args(m, store_fint);
   const bool with_ramp = !m->dinst_end;  // as in node_update
   if (with_ramp) pa.presc = presc_args(m);
   const cudaError_t e = launch_patches(m, pa, group_args(m, m->groups[0], true), m->pdl);
@@ -1141,42 +1147,39 @@ PatchLoad even_load(int64_t patches, int64_t evaluated) {
   return l;
 }
 
-// Whether a plan of such patches, the largest of which needs smem bytes, steps
-// faster than the two kernels.
+// The time of a step with such patches, the largest of which needs smem bytes,
+// over that of the two kernels: below kPatchSure the fused step is taken, above
+// kPatchNever not, between them both are timed (settle_patches).
 //
 // Tetrahedra: the time of either form in us from constants fitted to 409 measured
-// meshes (boxes, plates, bars, Delaunay meshes, batches; mean error 7 per cent).
-// An SM steps through its patches resident ones at a time: each round has a
-// latency, each element a time that grows when fewer blocks than the kernel is
-// built for are resident.  With all patches resident at once the SM with the most
-// elements is the last (mixed neohookean, 30 x 30 x 30 cells, 216 patches of up to
-// 5^3 nodes, 9.0 us), beyond that half a patch is still under way when the others
-// end.  Places for three per SM are not filled evenly: of 217 to 340 patches some
-// SM has three large ones (mixed, 264 equal patches of 33 cubes of 11^3, 11.4 us,
-// where two per SM would take 8.9; neohookean, 44 x 36 x 22 cells, 224 patches, 14.6,
-// two kernels 11.9, 54 x 34 x 28, 300 patches, 15.7 and 14.8).  The two kernels have a time per
-// element and, beyond 100 MB, per byte.  The plan must win by 7 per cent: no mesh
-// of the fit is then slower by more than 1, and what is left to the two kernels
-// loses 8 to 15 on four.  Two kernels / fused: 1000 cubes of 1^3, mixed, 5.3 / 7.8,
-// 4000 6.1 / 25.6, 2000 of 3^3 17.4 / 20.8, 300 of 4^3 9.5 / 5.9; Delaunay, mixed, 54 k
-// 10.8 / 6.6, 429 k, one block per SM, 22.0 / 24.7, 1.4 M, two, 71.8 / 73.7.
+// meshes (boxes, plates, bars, Delaunay meshes, batches; mean error 7 per cent, the
+// largest 30).  An SM steps through its patches resident ones at a time: each round
+// has a latency, each element a time that grows when fewer blocks than the kernel
+// is built for are resident.  With all patches resident at once the SM with the
+// most elements is the last, beyond that half a patch is still under way when the
+// others end.  The two kernels have a time per element and, beyond 100 MB, per
+// byte.  Two kernels / fused: 1000 cubes of 1^3, mixed, 5.3 / 7.8, 4000 6.1 / 25.6,
+// 2000 of 3^3 17.4 / 20.8, 300 of 4^3 9.5 / 5.9; Delaunay, mixed, 54 k 10.8 / 6.6, 429
+// k, one block per SM, 22.0 / 24.7, 1.4 M, two, 71.8 / 73.7.  What the fit does not
+// see is how the hardware fills places for three blocks per SM: neohookean boxes of
+// 30^3 cells, 216 patches, 11.0 / 9.0, 44 x 36 x 22, 224, 11.9 / 14.6, six cubes of 10^3
+// to 15^3 8.4 / 6.0.
 //
-// Hexahedra: the elements of an SM within half as many again as the largest
-// box of the rule below has.  Triangles: up to four patches per SM, two of 6
-// points (mixed 400 x 20 x 2, 606 patches, 10.3, two kernels 9.7; FP64 1000 x 5 x 2,
-// 502 patches, 8.9 / 10.6).
-bool patches_pay(int et, int rule, int law, bool mixed, int64_t E, const PatchLoad &load,
-                 size_t smem) {
+// Hexahedra: up to 260 elements of an SM (23 x 25 x 24 cells, 245 of them, elastic
+// 6.4, two kernels 7.0, neohookean 8.2 / 8.5).  Triangles: up to four patches per SM,
+// two of 6 points (mixed 400 x 20 x 2, 606 patches, 10.3, two kernels 9.7; FP64 1000 x
+// 5 x 2, 502 patches, 8.9 / 10.6).
+constexpr double kPatchSure = 0.7, kPatchNever = 1.15;
+double patches_over_kernels(int et, int rule, int law, bool mixed, int64_t E,
+                            const PatchLoad &load, size_t smem) {
   const double rounds = std::ceil((double)load.patches / kPatchSms);  // patches of an SM
-  if (et == AKB_TRIANGLE_6) return rounds <= (rule ? 2. : 4.);
-  if (et == AKB_HEXAHEDRON_8) return rounds * load.evaluated <= 250. * load.patches;
+  if (et == AKB_TRIANGLE_6) return rounds <= (rule ? 2. : 4.) ? 0. : 2.;
+  if (et == AKB_HEXAHEDRON_8) return load.heaviest <= 260 ? 0. : 2.;
   const double built = mixed ? 3. : 2.;
   const double resident = std::min(built, std::max(1., std::floor(233472. / (double)(smem + 1024))));
   const double rate = std::min(built, rounds) / std::min(resident, rounds);
-  const bool uneven = resident == 3. && load.patches > 216 && load.patches <= 340;
-  const double work = uneven              ? 3. * (double)load.largest
-                      : rounds <= resident ? (double)load.heaviest
-                                           : (double)load.evaluated / kPatchSms + 0.5 * load.largest;
+  const double work = rounds <= resident ? (double)load.heaviest
+                                         : (double)load.evaluated / kPatchSms + 0.5 * load.largest;
   const bool neo = law == LAW_NEOHOOKEAN;
   const double element = mixed ? (neo ? 2.65e-3 : 2.3e-3) : (neo ? 7.2e-3 : 2.9e-3);
   const double fused = (mixed ? 3.0 : 2.6) * std::ceil(rounds / resident) + element * work * rate;
@@ -1184,7 +1187,7 @@ bool patches_pay(int et, int rule, int law, bool mixed, int64_t E, const PatchLo
   const double two = mixed ? 6.1 + 33.3e-6 * (double)E + 0.116e-6 * beyond
                            : (neo ? 8.2 : 7.0) + (neo ? 65e-6 : 60.7e-6) * (double)E +
                                  0.0575e-6 * beyond;
-  return fused <= 0.93 * two;
+  return fused / two;
 }
 
 // Owned nodes of a patch at most, s per edge; 0 where the two-kernel step is
@@ -1230,7 +1233,7 @@ int patch_nodes(int et, int rule, int law, int precision, int64_t N, int64_t E, 
       const double slabs = std::ceil(planes / s - 1e-6), side = std::ceil(planes / slabs - 1e-6);
       // resident blocks per SM, fewer with the slots of 6 points
       const double patches = ninst * slabs * slabs;
-      if (patches > sms * (rule ? 2. : mixed ? 4. : 3.)) break;  // as in patches_pay
+      if (patches > sms * (rule ? 2. : mixed ? 4. : 3.)) break; 
       const double cells = std::floor((side + 1.) / 2.) + 1.;  // that its node planes touch
       const double rounds = std::ceil(std::ceil(2. * cells * cells / 32.) * (rule ? 6. : 3.) / 6.);
       if (least == 0. || rounds < least || (rounds == least && patches <= sms)) {
@@ -1256,8 +1259,9 @@ int patch_nodes(int et, int rule, int law, int precision, int64_t N, int64_t E, 
   }
   // no patch reaches across two instances of a batch
   const int own = best * best * best;
-  if (tet && !patches_pay(et, rule, law, mixed, E,
-                          even_load(std::max<int64_t>(std::max(ninst, 1), N / own), E), 0))
+  if (tet && patches_over_kernels(et, rule, law, mixed, E,
+                                  even_load(std::max<int64_t>(std::max(ninst, 1), N / own), E),
+                                  0) > kPatchNever)
     return 0;
   return own;
 }
@@ -1397,8 +1401,10 @@ int finish_patches(akb_model *m, PatchTask &task) {
   if (pa.smem + kPatchStageSmem > kPatchMaxSmem) return AKB_OK;
   PatchCaps need;
   need.patches = (int64_t)plan.head.size();
-  if (!patches_pay(m->et, m->rule, gr.law, mixed, m->E, patch_load(plan.head), pa.smem))
-    return AKB_OK;
+  const double over =
+      patches_over_kernels(m->et, m->rule, gr.law, mixed, m->E, patch_load(plan.head), pa.smem);
+  if (over > kPatchNever) return AKB_OK;
+  m->patch_unsure = over > kPatchSure;
   need.nodes = (int64_t)plan.nodes.size();
   need.elems = (int64_t)plan.elems.size();
   const PatchRoom room = patch_room(need, m->N, m->nn, t);
@@ -1466,6 +1472,44 @@ int finish_patches(akb_model *m, PatchTask &task) {
   pa.materials = (int)m->mats.size();
   m->patch_on = false;  // the bounds-checking build runs it when asked to
 #endif
+  return AKB_OK;
+}
+
+// At the end of initFull: the faster form of the step from eight steps of each on
+// the state at rest, which is put back; without the plan where it is the slower.
+// 0.3 ms at 100,000 tetrahedra, whose initFull takes 4.
+int settle_patches(akb_model *m) {
+  if (!m->patch_ready || !m->patch_unsure) return AKB_OK;
+  AKB_TRY(find_trigger(m));
+  cudaStream_t s = m->stream;
+  cudaEvent_t ev[2] = {nullptr, nullptr};
+  cudaError_t e = cudaEventCreate(&ev[0]);
+  if (e == cudaSuccess) e = cudaEventCreate(&ev[1]);
+  float ms[2] = {0.f, 0.f};
+  int rc = AKB_OK;
+  for (int fused = 0; fused < 2 && e == cudaSuccess && rc == AKB_OK; ++fused) {
+    for (int k = 0; k < 10 && e == cudaSuccess && rc == AKB_OK; ++k) {
+      if (k == 2) e = cudaEventRecord(ev[0], s);
+      if (fused) {
+        if (e == cudaSuccess)
+          e = launch_patches(m, patch_args(m, false), group_args(m, m->groups[0], true), m->pdl);
+      } else {
+        rc = launch_forces(m, true);
+        if (rc == AKB_OK) rc = launch_nodes(m, true);
+      }
+    }
+    if (e == cudaSuccess) e = cudaEventRecord(ev[1], s);
+    if (e == cudaSuccess) e = cudaEventSynchronize(ev[1]);
+    if (e == cudaSuccess) e = cudaEventElapsedTime(&ms[fused], ev[0], ev[1]);
+  }
+  for (cudaEvent_t x : ev)
+    if (x) cudaEventDestroy(x);
+  AKB_TRY(rc);
+  for (double *p : {m->dU[0], m->dU[1], m->dv, m->da})
+    if (e == cudaSuccess) e = cudaMemsetAsync(p, 0, sizeof(double) * nodal_doubles(m), s);
+  if (e == cudaSuccess) e = cudaMemsetAsync(m->dstatus, 0, sizeof(unsigned int), s);
+  if (e != cudaSuccess) return fail(AKB_ECUDA, std::string("fused step: ") + cudaGetErrorString(e));
+  if (ms[0] < ms[1]) m->release_patches();
   return AKB_OK;
 }
 
@@ -2030,6 +2074,7 @@ int akb_model_init_full(akb_model *m, int method, int precision) {
                              cudaMemcpyHostToDevice, s));
     AKB_CUDA(cudaStreamSynchronize(s));
   }
+  AKB_TRY(settle_patches(m));
   AKB_CUDA(cudaStreamSynchronize(s));
   m->initialized = true;
   return AKB_OK;
