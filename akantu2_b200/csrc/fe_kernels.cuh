@@ -37,8 +37,13 @@ constexpr int kMaxNN = 8;
 // instructions do nothing.
 __device__ __forceinline__ void pdl_begin(bool trigger = true) {
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  // (predicated: a branch here changes the code that follows, 0.1 us of FP64
-  // hexahedra)
+  if (trigger) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+// the same without a branch, for the FP64 hexahedra: a branch here changes the code
+// that follows it (neohookean 19 x 17 x 15 12.8 us per step, 12.7 without; plastic FP64
+// triangles 281 x 165 x 2 of 6 points 48.5, 50.7 without)
+__device__ __forceinline__ void pdl_begin_predicated(bool trigger) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %0, 0;\n\t"
                "@p griddepcontrol.launch_dependents;\n\t}" ::"r"((int)trigger)
                : "memory");
@@ -2008,7 +2013,7 @@ __global__ void __launch_bounds__(32 * NQ, LAW == LAW_PLASTIC ? 2 : 4)
       for (int c = 0; c < ND; ++c) copy_async_8(&red[q][c][lane], Bq + (int64_t)c * E);
     }
   }
-  pdl_begin(ps.trigger);
+  pdl_begin_predicated(ps.trigger);
   const bool active = le < e_count && element_active(ps, le) &&
                       element_indices_ok<NN>(ps, conn, pos, E, e_begin + le);
   if (active) {

@@ -372,3 +372,25 @@ def test_dependent_launches_of_fp64_hexahedra(mat, n, dependent):
         m.solveStep(103)
         runs.append(m.getDisplacement())
     assert np.abs(runs[0]).max() > 0 and np.array_equal(*runs)
+
+
+@pytest.mark.parametrize("cells", [(36, 32, 21), (44, 36, 22)])
+def test_timing_the_forms_leaves_the_model_at_rest(cells):
+    """sizes at which initFull times both forms of the step: the model is at
+    rest afterwards, forces of an eigen gradient included, and steps as one that
+    was told to use two kernels"""
+    mesh = akb.box_tet4(*cells, lengths=[c / 40 for c in cells])
+    mat = dict(UNIT_ELASTIC, eigen_grad_u=[[1e-3, 0, 0], [0, 2e-3, 0], [5e-4, 0, 0]])
+    models = []
+    for two in (False, True):
+        m = gpu_model(mesh, [mat], precision="mixed")
+        for f in FIELDS:
+            x = getattr(m, f)()
+            assert not x.any() and not np.signbit(x).any(), f
+        assert m.getStatus() == 0
+        if two:
+            m.setNodeShape(*m.getNodeShape())  # leaves the fused step
+        m.setTimeStep(0.8 * m.getStableTimeStep())
+        m.solveStep(3)
+        models.append(m)
+    _same(models)
